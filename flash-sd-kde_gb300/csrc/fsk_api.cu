@@ -161,6 +161,7 @@ int fsk_kde16(const float* queries, int64_t m, const float* data, int64_t n, dou
   CenterBufs cb = take_center(c, n);
   const bool laplace = (flags & FSK_LAPLACE) != 0;
   double* part = nullptr;
+  tc::TcPartials tcp{};
   int splits = 1;
   if (p.ieee) {
     splits = p.atomic ? 1 : p.simt_splits;
@@ -172,15 +173,19 @@ int fsk_kde16(const float* queries, int64_t m, const float* data, int64_t n, dou
   } else {
     launch_mean16(data, n, cb.scratch, cb.mu, cb.mu64, s);
     st = tc::launch_kde16_tc(queries, m, data, n, cb.mu, bandwidth, laplace, (flags & FSK_PREC_FP16_SINGLE) != 0,
-                             (flags & FSK_EXP_OFFLOAD) != 0, p.tcp, c, &part, p.atomic, s);
+                             (flags & FSK_EXP_OFFLOAD) != 0, p.tcp, c, &tcp, p.atomic ? &part : nullptr, s);
     if (st) return st;
-    splits = p.atomic ? 1 : (int)p.tcp.part_rows;
   }
+  // segment partials of the tensor-core kernel, or FP64 rows (CUDA cores, atomic accumulator)
+  const bool segments = !p.ieee && !p.atomic;
   if (p.log_exact) {
     LogExactBufs lb;
     take_logexact(c, m, &lb);
     if (!c.fits()) return FSK_ERR_WORKSPACE_TOO_SMALL;
-    launch_reduce_logexact(queries, m, data, n, bandwidth, laplace, part, splits, out_scale, lb, out, s);
+    if (segments) launch_reduce_tc_logexact(queries, m, data, n, bandwidth, laplace, tcp, out_scale, lb, out, s);
+    else launch_reduce_logexact(queries, m, data, n, bandwidth, laplace, part, splits, out_scale, lb, out, s);
+  } else if (segments) {
+    launch_reduce_tc_rows(tcp, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, s);
   } else {
     launch_reduce_rows(part, splits, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, s);
   }
@@ -202,7 +207,7 @@ static size_t empscore_bytes(int64_t n, int variant, int flags) {
     c.take<double>((size_t)n * FSK_D);
     b = c.used;
   } else if (!(flags & FSK_PREC_IEEE)) {
-    b = align_up(b, 256) + tc::tc_score16_ws_bytes(tc::plan_score16(n), n);
+    b = align_up(b, 256) + tc::tc_score16_ws_bytes(tc::plan_score16(n));
   } else {
     const int splits = simt_score16_splits(n);
     c.take<double>((size_t)splits * n);
@@ -239,21 +244,19 @@ int fsk_empscore16(const float* data, int64_t n, double bandwidth, int variant, 
     launch_zero(apdf, n, s);
     launch_zero(aw, n * FSK_D, s);
     launch_score16_sym_simt(data, n, cb.mu, bandwidth, apdf, aw, s);
-    launch_reduce_score(apdf, aw, 1, 1, n, cb.mu64, nullptr, pdf_sum, weighted_sum, ws_row, ws_col, rscratch, s);
+    launch_reduce_score(apdf, aw, 1, n, cb.mu64, pdf_sum, weighted_sum, ws_row, ws_col, rscratch, s);
   } else if (!(flags & FSK_PREC_IEEE)) {
     const tc::TcPlan pl = tc::plan_score16(n);
-    double *ppdf = nullptr, *pw = nullptr;
-    st = tc::launch_score16_tc(data, n, cb.mu, bandwidth, pl, c, &ppdf, &pw, s);
+    tc::ScPartials parts{};
+    st = tc::launch_score16_tc(data, n, cb.mu, bandwidth, pl, c, &parts, s);
     if (st) return st;
-    launch_reduce_score(ppdf, pw, (int)(2 * pl.splits), (int)pl.splits, n, cb.mu64, data, pdf_sum,
-                        weighted_sum, ws_row, ws_col, rscratch, s);
+    launch_reduce_score_tc(parts, n, cb.mu, data, pdf_sum, weighted_sum, ws_row, ws_col, s);
   } else {
     const int splits = simt_score16_splits(n);
     double* ppdf = c.take<double>((size_t)splits * n);
     double* pw = c.take<double>((size_t)splits * n * FSK_D);
     launch_score16_simt(data, n, cb.mu, bandwidth, splits, ppdf, pw, s);
-    launch_reduce_score(ppdf, pw, splits, splits, n, cb.mu64, nullptr, pdf_sum, weighted_sum, ws_row, ws_col,
-                        rscratch, s);
+    launch_reduce_score(ppdf, pw, splits, n, cb.mu64, pdf_sum, weighted_sum, ws_row, ws_col, rscratch, s);
   }
   return cuda_status(cudaGetLastError());
 }

@@ -133,6 +133,22 @@ struct Comp {
   }
 };
 
+// ---- double-float values (unevaluated FP32 pairs, ~48 bits) --------------------
+// The O(n) kernels around the pairwise sums use them instead of FP64, whose
+// unit runs 2 lanes per clock per SM on this chip against 128 for FP32.
+__device__ __forceinline__ float2 two_sum(float a, float b) {   // a + b = x + y exactly
+  const float s = a + b, z = s - a;
+  return make_float2(s, (a - (s - z)) + (b - z));
+}
+__device__ __forceinline__ float2 two_prod(float a, float b) {  // a * b = x + y exactly
+  const float p = a * b;
+  return make_float2(p, fmaf(a, b, -p));
+}
+__device__ __forceinline__ float2 df_add(float2 a, float2 b) {
+  const float2 s = two_sum(a.x, b.x);
+  return two_sum(s.x, s.y + (a.y + b.y));
+}
+
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

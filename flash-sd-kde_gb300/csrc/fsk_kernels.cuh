@@ -3,6 +3,11 @@
 #include "fsk_common.cuh"
 
 namespace fsk {
+namespace tc {
+struct TcPartials;
+struct ScPartials;
+}  // namespace tc
+
 
 // ---- device error words (see fsk_common.cuh) --------------------------------
 unsigned int kde16_take_device_error();    // fsk_tc_kde16.cu
@@ -43,15 +48,20 @@ void launch_mean16(const float* x, int64_t n, double* scratch, float* mu, double
 // out[i] = g(scale * sum_s partials[s*m + i]), g = identity or log(. + eps).
 void launch_reduce_rows(const double* partials, int splits, int64_t m, double scale, double eps,
                         bool log_out, float* out, cudaStream_t s);
+// The same over the tensor-core KDE's segment partials.
+void launch_reduce_tc_rows(const tc::TcPartials& p, int64_t m, double scale, double eps, bool log_out, float* out,
+                           cudaStream_t s);
 // pdf[i] = sum_s ppdf[s][i]; w[i][k] = sum_s pw[s][i][k] + mu64[k] * pdf[i]
 // (pass splits = 1 with atomic accumulators).  w written at w[i*ws_row + k*ws_col].
-// pdf partials [pdf_splits][n], weighted partials [w_splits][n][16] (centred);
-// self_x: the data when the partials leave out the self pair, else nullptr.
+// FP64 partials ppdf [splits][n], pw [splits][n][16] (centred).
 // scratch: reduce_score_scratch_doubles(n) doubles.
 size_t reduce_score_scratch_doubles(int64_t n);
-void launch_reduce_score(const double* ppdf, const double* pw, int pdf_splits, int w_splits, int64_t n,
-                         const double* mu64, const float* self_x, float* pdf, float* w, int64_t ws_row,
-                         int64_t ws_col, double* scratch, cudaStream_t s);
+void launch_reduce_score(const double* ppdf, const double* pw, int splits, int64_t n, const double* mu64, float* pdf,
+                         float* w, int64_t ws_row, int64_t ws_col, double* scratch, cudaStream_t s);
+// The same from the tensor-core score's segment partials, which leave out the
+// self pair (added here exactly).
+void launch_reduce_score_tc(const tc::ScPartials& p, int64_t n, const float* mu, const float* x, float* pdf, float* w,
+                            int64_t ws_row, int64_t ws_col, cudaStream_t s);
 void launch_debias16(const float* x, int64_t n, const float* pdf, const float* w, int64_t ws_row,
                      int64_t ws_col, double h, double eps, float* debiased, float* score,
                      cudaStream_t s);
@@ -75,6 +85,9 @@ void take_logexact(WsCarver& c, int64_t m, LogExactBufs* b);
 void launch_reduce_logexact(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace,
                             const double* partials, int splits, double scale, const LogExactBufs& b, float* out,
                             cudaStream_t s);
+void launch_reduce_tc_logexact(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace,
+                               const tc::TcPartials& partials, double scale, const LogExactBufs& b, float* out,
+                               cudaStream_t s);
 
 // ---- fsk_nd.cu ------------------------------------------------------------------
 // any 1 <= d <= FSK_ND_MAX features, rows with stride d (CUDA cores)

@@ -18,6 +18,7 @@
 // each query's value comes from a fixed partition of the data.
 #include "fsk_common.cuh"
 #include "fsk_kernels.cuh"
+#include "fsk_tc.cuh"
 
 namespace fsk {
 
@@ -27,6 +28,28 @@ constexpr int LS_WARPS = LS_THREADS / 32;
 constexpr int LS_QG = 64;         // queries per work item (2 per lane)
 constexpr int LS_TN = 32;         // data points per warp tile
 
+// out = log(scale * sum), or the query onto the list when its sum underflows
+__device__ __forceinline__ void finish_or_list(int64_t i, int64_t m, double s, double scale, double tiny,
+                                               float* __restrict__ out, uint32_t* __restrict__ count,
+                                               uint32_t* __restrict__ list) {
+  if (s >= tiny) {
+    out[i] = (float)log(s * scale);
+  } else {
+    const uint32_t slot = atomicAdd(count, 1u);
+    if (in_bounds(slot, m, 56)) list[slot] = (uint32_t)i;
+  }
+}
+
+template <int RL>
+__global__ void __launch_bounds__(tc::TC_RED_THREADS) reduce_tc_rows_logexact_kernel(
+    tc::TcPartials p, int64_t m, double scale, double tiny, float* __restrict__ out, uint32_t* __restrict__ count,
+    uint32_t* __restrict__ list) {
+  constexpr int ROWS = tc::TC_RED_THREADS / RL;
+  const int64_t i = (int64_t)blockIdx.x * ROWS + threadIdx.x % ROWS;
+  double s;
+  if (tc::reduce_tc_row<RL>(p, i, m, s)) finish_or_list(i, m, s, scale, tiny, out, count, list);
+}
+
 // queries flagged by the reduction: out = log(scale * sum) for the others
 __global__ void reduce_rows_logexact_kernel(const double* __restrict__ partials, int splits, int64_t m,
                                             double scale, double tiny, float* __restrict__ out,
@@ -35,12 +58,7 @@ __global__ void reduce_rows_logexact_kernel(const double* __restrict__ partials,
   if (i >= m) return;
   double s = 0.0;
   for (int k = 0; k < splits; ++k) s += partials[(int64_t)k * m + i];
-  if (s >= tiny) {
-    out[i] = (float)log(s * scale);
-  } else {
-    const uint32_t slot = atomicAdd(count, 1u);
-    if (in_bounds(slot, m, 56)) list[slot] = (uint32_t)i;
-  }
+  finish_or_list(i, m, s, scale, tiny, out, count, list);
 }
 
 // data parts per query group: enough work items to fill the grid
@@ -206,15 +224,9 @@ void take_logexact(WsCarver& c, int64_t m, LogExactBufs* b) {
   if (b) *b = t;
 }
 
-void launch_reduce_logexact(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace,
-                            const double* partials, int splits, double scale, const LogExactBufs& b, float* out,
-                            cudaStream_t s) {
-  cudaMemsetAsync(b.count, 0, sizeof(uint32_t), s);
-  const int T = 256;
-  const double tiny = ldexp((double)n, -100);
-  reduce_rows_logexact_kernel<<<(unsigned)((m + T - 1) / T), T, 0, s>>>(partials, splits, m, scale, tiny, out,
-                                                                      b.count, b.list);
-  count_launch();
+// Recomputes the listed queries.
+static void launch_listed(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace, double scale,
+                          const LogExactBufs& b, float* out, cudaStream_t s) {
   const double c2d = FSK_LOG2E / (2.0 * h * h);
   const double c1d = 1.0 / (2.0 * h * h);
   const int grid = 4 * sm_count();
@@ -231,6 +243,33 @@ void launch_reduce_logexact(const float* q, int64_t m, const float* x, int64_t n
   logspace_combine_kernel<<<2 * sm_count(), 256, 0, s>>>(b.count, b.list, b.pd, b.ps, m, grid, c2d, c1d, log(scale),
                                                           out);
   count_launch();
+}
+
+void launch_reduce_logexact(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace,
+                            const double* partials, int splits, double scale, const LogExactBufs& b, float* out,
+                            cudaStream_t s) {
+  cudaMemsetAsync(b.count, 0, sizeof(uint32_t), s);
+  const int T = 256;
+  reduce_rows_logexact_kernel<<<(unsigned)((m + T - 1) / T), T, 0, s>>>(partials, splits, m, scale,
+                                                                      ldexp((double)n, -100), out, b.count, b.list);
+  count_launch();
+  launch_listed(q, m, x, n, h, laplace, scale, b, out, s);
+}
+
+void launch_reduce_tc_logexact(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace,
+                               const tc::TcPartials& p, double scale, const LogExactBufs& b, float* out,
+                               cudaStream_t s) {
+  cudaMemsetAsync(b.count, 0, sizeof(uint32_t), s);
+  const double tiny = ldexp((double)n, -100);
+  constexpr int T = tc::TC_RED_THREADS, RL = 8;
+  if (tc::tc_short_rows(p))
+    reduce_tc_rows_logexact_kernel<1><<<(unsigned)((m + T - 1) / T), T, 0, s>>>(p, m, scale, tiny, out, b.count,
+                                                                              b.list);
+  else
+    reduce_tc_rows_logexact_kernel<RL><<<(unsigned)((m + T / RL - 1) / (T / RL)), T, 0, s>>>(p, m, scale, tiny, out,
+                                                                                            b.count, b.list);
+  count_launch();
+  launch_listed(q, m, x, n, h, laplace, scale, b, out, s);
 }
 
 unsigned int logspace_take_device_error() { return take_unit_device_error(); }

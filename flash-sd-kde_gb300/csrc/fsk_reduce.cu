@@ -5,6 +5,7 @@
 // sums splits in FP32); normalisation follows flash_sd_kde/kde.py:93-94,
 // :119-122; the debias shift follows flash_sd_kde/kde.py:319-322.
 #include "fsk_kernels.cuh"
+#include "fsk_tc.cuh"
 
 namespace fsk {
 
@@ -70,12 +71,35 @@ void launch_mean16(const float* x, int64_t n, double* scratch, float* mu, double
   count_launch();
 }
 
-__global__ void reduce_rows_kernel(const double* __restrict__ partials, int splits, int64_t m,
-                                   double scale, double eps, int log_out, float* __restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
+// Cross-split sums with the FP64 normalisation (and log).  RL threads share a
+// row (split k goes to thread k % RL) so that a query's few hundred partials
+// are not one chain of dependent loads: 49 us for 2048 rows x 300 partials by
+// one thread per row, 8-thread rows take the reduction to launch cost.  The
+// threads' sums are added in thread order, so the result is deterministic.
+constexpr int RED_THREADS = tc::TC_RED_THREADS;
+constexpr int RED_LANES = 8;
+
+template <int RL>
+__global__ void __launch_bounds__(RED_THREADS) reduce_rows_kernel(const double* __restrict__ partials, int splits,
+                                                                  int64_t m, double scale, double eps, int log_out,
+                                                                  float* __restrict__ out) {
+  constexpr int ROWS = RED_THREADS / RL;
+  const int r = threadIdx.x % ROWS, l = threadIdx.x / ROWS;
+  const int64_t i = (int64_t)blockIdx.x * ROWS + r;
   double s = 0.0;
-  for (int k = 0; k < splits; ++k) s += partials[(int64_t)k * m + i];
+  if (i < m) {
+#pragma unroll 4
+    for (int k = l; k < splits; k += RL) s += partials[(int64_t)k * m + i];
+  }
+  if (RL > 1) {
+    __shared__ double sh[RL][ROWS];
+    sh[l][r] = s;
+    __syncthreads();
+    if (l > 0 || i >= m) return;
+#pragma unroll
+    for (int j = 1; j < RL; ++j) s += sh[j][r];
+  }
+  if (i >= m) return;
   double v = s * scale;
   if (log_out) v = log(v + eps);
   out[i] = (float)v;
@@ -83,54 +107,131 @@ __global__ void reduce_rows_kernel(const double* __restrict__ partials, int spli
 
 void launch_reduce_rows(const double* partials, int splits, int64_t m, double scale, double eps,
                         bool log_out, float* out, cudaStream_t s) {
-  const int T = 256;
-  reduce_rows_kernel<<<(unsigned)((m + T - 1) / T), T, 0, s>>>(partials, splits, m, scale, eps,
-                                                              log_out ? 1 : 0, out);
+  // one thread per row while the chain is short
+  if (splits <= 4)
+    reduce_rows_kernel<1><<<(unsigned)((m + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
+        partials, splits, m, scale, eps, log_out ? 1 : 0, out);
+  else
+    reduce_rows_kernel<RED_LANES><<<(unsigned)((m + RED_THREADS / RED_LANES - 1) / (RED_THREADS / RED_LANES)),
+                                    RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out);
   count_launch();
 }
 
-// pdf = sum of pdf partials (thread per row; the FP64 sum of the partials,
-// without the self pair, is kept for the weighted pass), then weighted =
-// sum of centred partials + mu * pdf (thread per element, coalesced over the
-// [split][row][16] partials).  self_x != nullptr: the partials leave the self
-// pair out; it is added here exactly (phi_ii = 1, weight x_i).
+template <int RL>
+__global__ void __launch_bounds__(RED_THREADS) reduce_tc_rows_kernel(tc::TcPartials p, int64_t m, double scale,
+                                                                     double eps, int log_out,
+                                                                     float* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * (RED_THREADS / RL) + threadIdx.x % (RED_THREADS / RL);
+  double sum;
+  if (!tc::reduce_tc_row<RL>(p, i, m, sum)) return;
+  double v = sum * scale;
+  if (log_out) v = log(v + eps);
+  out[i] = (float)v;
+}
+
+void launch_reduce_tc_rows(const tc::TcPartials& p, int64_t m, double scale, double eps, bool log_out, float* out,
+                           cudaStream_t s) {
+  if (tc::tc_short_rows(p))
+    reduce_tc_rows_kernel<1><<<(unsigned)((m + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
+        p, m, scale, eps, log_out ? 1 : 0, out);
+  else
+    reduce_tc_rows_kernel<RED_LANES><<<(unsigned)((m + RED_THREADS / RED_LANES - 1) / (RED_THREADS / RED_LANES)),
+                                       RED_THREADS, 0, s>>>(p, m, scale, eps, log_out ? 1 : 0, out);
+  count_launch();
+}
+
+// Tensor-core score partials -> pdf_sum and weighted_sum, 16 threads per row
+// (thread k: feature k of every segment's centred weighted sum, and the pdf
+// pairs k, k + 16, ... of the row, added across the 16 threads by shuffles).
+// The self pair, which the partials leave out, is added exactly (phi = 1,
+// weight x_i), then mu * pdf undoes the centring.  Everything is carried as
+// double-float and rounded to FP32 once; in FP64 the pass was bound by the
+// FP64 unit (26 us at n = 65536 for 38 MB of traffic).
+__global__ void __launch_bounds__(RED_THREADS) reduce_score_tc_kernel(tc::ScPartials p, int64_t n,
+                                                                      const float* __restrict__ mu,
+                                                                      const float* __restrict__ x,
+                                                                      float* __restrict__ pdf, float* __restrict__ w,
+                                                                      int64_t ws_row, int64_t ws_col) {
+  constexpr int QB = 256;   // rows per query block
+  const int64_t e = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
+  const int64_t i = e / FSK_D;
+  const int k = (int)(threadIdx.x % FSK_D);
+  if (i >= n) return;   // a row's 16 threads leave together
+  const unsigned group = 0xFFFFu << (threadIdx.x & 16);
+  const int64_t qb = i / QB;
+  const int r = (int)(i % QB);
+  int segs;
+  const int64_t seg0 = p.line.segments_of(qb, segs);
+  float2 ps = make_float2(0.f, 0.f);
+  for (int j = k; j < 2 * segs; j += FSK_D) ps = df_add(ps, p.ppdf[(2 * seg0 + j) * QB + r]);
+#pragma unroll
+  for (int o = 1; o < FSK_D; o <<= 1)
+    ps = df_add(ps, make_float2(__shfl_xor_sync(group, ps.x, o), __shfl_xor_sync(group, ps.y, o)));
+  float2 ws = make_float2(0.f, 0.f);
+  const float2* wp = p.pw + (seg0 * QB + r) * FSK_D + k;
+#pragma unroll 4
+  for (int j = 0; j < segs; ++j) ws = df_add(ws, wp[(int64_t)j * QB * FSK_D]);
+  constexpr float phi_unscale = 1.0f / 32768.0f;   // 2^-PHI_LOG2_SCALE
+  static_assert(tc::PHI_LOG2_SCALE == 15.0f, "weight scale");
+  const float w_unscale = ldexpf(1.f, -p.scales->pad[2]);
+  ps.x *= phi_unscale;
+  ps.y *= phi_unscale;
+  ws.x = ws.x * phi_unscale * w_unscale;
+  ws.y = ws.y * phi_unscale * w_unscale;
+  // W + mu * p + x_i
+  const float m = mu[k];
+  float2 mp = two_prod(m, ps.x);
+  mp.y = fmaf(m, ps.y, mp.y);
+  const float2 wt = df_add(df_add(ws, mp), make_float2(x[e], 0.f));
+  const int64_t o = i * ws_row + k * ws_col;
+  if (in_bounds(o, n * FSK_D, 53)) w[o] = wt.x;
+  if (k == 0) pdf[i] = df_add(ps, make_float2(1.0f, 0.f)).x;
+}
+
+void launch_reduce_score_tc(const tc::ScPartials& p, int64_t n, const float* mu, const float* x, float* pdf, float* w,
+                            int64_t ws_row, int64_t ws_col, cudaStream_t s) {
+  reduce_score_tc_kernel<<<(unsigned)((n * FSK_D + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
+      p, n, mu, x, pdf, w, ws_row, ws_col);
+  count_launch();
+}
+
+// CUDA-core score partials (FP64): pdf = sum of pdf partials (thread per row;
+// the FP64 sum is kept for the weighted pass), then weighted = sum of centred
+// partials + mu * pdf (thread per element, coalesced over the
+// [split][row][16] partials).
 __global__ void reduce_score_pdf_kernel(const double* __restrict__ ppdf, int pdf_splits, int64_t n,
-                                        int add_self, float* __restrict__ pdf, double* __restrict__ p_other) {
+                                        float* __restrict__ pdf, double* __restrict__ p_sum) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double p = 0.0;
   for (int s = 0; s < pdf_splits; ++s) p += ppdf[(int64_t)s * n + i];
-  p_other[i] = p;
-  pdf[i] = (float)(add_self ? p + 1.0 : p);
+  p_sum[i] = p;
+  pdf[i] = (float)p;
 }
 
 __global__ void reduce_score_w_kernel(const double* __restrict__ pw, int w_splits, int64_t n,
-                                      const double* __restrict__ mu64, const double* __restrict__ p_other,
-                                      const float* __restrict__ self_x, float* __restrict__ w, int64_t ws_row,
-                                      int64_t ws_col) {
+                                      const double* __restrict__ mu64, const double* __restrict__ p_sum,
+                                      float* __restrict__ w, int64_t ws_row, int64_t ws_col) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n * FSK_D) return;
   const int64_t i = e / FSK_D;
   const int k = (int)(e % FSK_D);
   double a = 0.0;
   for (int s = 0; s < w_splits; ++s) a += pw[(int64_t)s * n * FSK_D + e];
-  const double po = p_other[i];
-  const double v = self_x ? a + mu64[k] * po + (double)self_x[e] : a + mu64[k] * po;
+  const double v = a + mu64[k] * p_sum[i];
   const int64_t o = i * ws_row + k * ws_col;
   if (in_bounds(o, n * FSK_D, 53)) w[o] = (float)v;
 }
 
 size_t reduce_score_scratch_doubles(int64_t n) { return (size_t)n; }
 
-void launch_reduce_score(const double* ppdf, const double* pw, int pdf_splits, int w_splits, int64_t n,
-                         const double* mu64, const float* self_x, float* pdf, float* w, int64_t ws_row,
-                         int64_t ws_col, double* scratch, cudaStream_t s) {
+void launch_reduce_score(const double* ppdf, const double* pw, int splits, int64_t n, const double* mu64, float* pdf,
+                         float* w, int64_t ws_row, int64_t ws_col, double* scratch, cudaStream_t s) {
   const int T = 256;
-  reduce_score_pdf_kernel<<<(unsigned)((n + T - 1) / T), T, 0, s>>>(ppdf, pdf_splits, n, self_x != nullptr, pdf,
-                                                                   scratch);
+  reduce_score_pdf_kernel<<<(unsigned)((n + T - 1) / T), T, 0, s>>>(ppdf, splits, n, pdf, scratch);
   count_launch();
-  reduce_score_w_kernel<<<(unsigned)((n * FSK_D + T - 1) / T), T, 0, s>>>(pw, w_splits, n, mu64, scratch, self_x,
-                                                                         w, ws_row, ws_col);
+  reduce_score_w_kernel<<<(unsigned)((n * FSK_D + T - 1) / T), T, 0, s>>>(pw, splits, n, mu64, scratch, w, ws_row,
+                                                                         ws_col);
   count_launch();
 }
 

@@ -59,6 +59,7 @@ constexpr int SMEM_BYTES = K_QX_OFFSET + EPI_WARPS * 32 * FSK_D * 4;
 // cross product), so a term below an eighth of the sum moves it by well
 // under 1e-6.
 constexpr float NEAR_FRACTION = 1.0f / 8.0f;
+constexpr float PHI_LOG2_SCALE = 15.0f;   // score weights are phi * 2^15
 constexpr float FP16_TARGET = 8192.0f;  // largest operand magnitude aimed for
 
 static_assert(TMEM_COLS == 512, "TMEM budget");
@@ -76,30 +77,99 @@ struct TcScales {
   int pad[3];      // ea, eb, ew: x'' = (x - mu) 2^ew is the weighted-sum operand
 };
 
+// ---- work split -------------------------------------------------------------------
+// Query blocks x data tiles over `grid` CTAs, in segments: a segment is a run
+// of data tiles of one query block, one accumulation and one row of partial
+// sums.  CTA b first takes the `whole` query blocks b, b + grid, ... from
+// their first to their last tile; all CTAs then walk the data in step, so a
+// tile comes from DRAM once for all of them (ranges that start anywhere made
+// the score kernel 5 % slower at n = 2^20, where the 268 MB data image exceeds
+// the L2).  The remaining rest < grid blocks form one line of rest * n_tiles
+// tiles of which every CTA takes an equal contiguous range, so small problems
+// neither leave the last wave empty nor pay for many short units (equal
+// splits of every query block gave the score kernel 5 units of 9 tiles per
+// CTA at n = 10007: 254 us against 49 us for its tiles at the large-n rate).
+struct WorkLine {
+  int64_t n_tiles;
+  int grid, whole, rest;
+  int line_grid;   // CTAs that share the line: min(grid, rest * n_tiles), at least 1
+  __host__ __device__ int64_t begin(int64_t b) const {
+    return imin<int64_t>(b, line_grid) * (rest * n_tiles) / line_grid;
+  }
+  // CTA holding tile L of the line: the largest b with begin(b) <= L
+  __host__ __device__ int64_t cta_of(int64_t L) const {
+    const int64_t total = rest * n_tiles;
+    return ((L + 1) * line_grid + total - 1) / total - 1;
+  }
+  // Segments of query block qb: numbers [first, first + count).  In the line
+  // both the CTA and the query block grow from one segment to the next, so
+  // their sum numbers them.
+  __host__ __device__ int64_t segments_of(int64_t qb, int& count) const {
+    const int64_t r = qb - (int64_t)whole * grid;
+    if (r < 0) {
+      count = 1;
+      return qb;
+    }
+    const int64_t b0 = cta_of(r * n_tiles);
+    count = (int)(cta_of((r + 1) * n_tiles - 1) - b0) + 1;
+    return qb + b0;
+  }
+  // number of the segment of query block qb that CTA b runs
+  __host__ __device__ int64_t segment_id(int qb, int b) const { return qb < whole * grid ? qb : (int64_t)qb + b; }
+  __host__ __device__ int64_t segment_bound() const { return (int64_t)(whole + 1) * grid + rest; }
+};
+
+struct Segment {
+  int qb, t0, count;   // query block, first data tile, tiles
+};
+
+// The segment of CTA b that begins after `done` of its tiles; count = 0 at the
+// end.  (`done` is the only state a role keeps across its tile loop, where
+// the epilogue warps have no registers to spare.)
+__host__ __device__ inline Segment segment_at(const WorkLine& w, int b, int done) {
+  Segment g;
+  const int n_tiles = (int)w.n_tiles, k = done / n_tiles;
+  if (k < w.whole) {
+    g.qb = b + k * w.grid;
+    g.t0 = 0;
+    g.count = n_tiles;
+  } else {
+    const int64_t L = w.begin(b) + (done - w.whole * n_tiles);
+    const int64_t r = L / n_tiles;
+    g.qb = (int)r + w.whole * w.grid;
+    g.t0 = (int)(L - r * n_tiles);
+    g.count = (int)imin<int64_t>(n_tiles - g.t0, w.begin((int64_t)b + 1) - L);
+  }
+  return g;
+}
+
 struct TcParams {
   const uint8_t* qimg;
   const uint8_t* ximg;
-  const float* qexact;
+  const float* q;         // original query rows (m, 16), for the exact recompute
   const TcScales* scales;
   int64_t m, n;
-  int64_t n_tiles;
-  int64_t q_blocks;
-  int64_t splits;
-  int64_t tiles_per_split;
+  WorkLine line;
   float c2, c2_lo, c1;
-  double* partials;
+  float2* partials;       // [segment][column half][row_stride] (value, error) pairs
+  int row_stride;         // rows per query block in the partials: min(m, 256)
   double* atomic_acc;
 };
 
 struct TcPlan {
-  int64_t m_pad, n_pad, n_tiles, q_blocks, splits, tiles_per_split;
-  int64_t part_rows;   // FP64 partial rows per query written by the kernel
-  int grid;
+  int64_t m_pad, n_pad, n_tiles, q_blocks;
+  WorkLine line;
 };
 
-// Fills splits / tiles_per_split / grid from q_blocks and n_tiles.
-void plan_splits(TcPlan& pl);
+// Fills line from q_blocks and n_tiles.
+void plan_line(TcPlan& pl);
 TcPlan plan_kde16(int64_t m, int64_t n);
+// Partial sums of the tensor-core KDE as the reductions read them.
+struct TcPartials {
+  const float2* part;
+  WorkLine line;
+  int row_stride;
+};
 
 // Prep kernels shared by the tensor-core kernels (fsk_tc_kde16.cu).
 __global__ void scale_init_kernel(TcScales* sc);
@@ -112,17 +182,59 @@ __global__ void prep_query_kernel(const float* __restrict__ q, int64_t m, int64_
                                   float* __restrict__ qexact);
 size_t tc_kde16_ws_bytes(const TcPlan& pl, int64_t m, bool atomic);
 int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, const float* mu, double h,
-                    bool laplace, bool single, bool poly, const TcPlan& pl, WsCarver& c, double** partials_out,
-                    bool atomic, cudaStream_t s);
+                    bool laplace, bool single, bool poly, const TcPlan& pl, WsCarver& c, TcPartials* partials_out,
+                    double** atomic_out, cudaStream_t s);
 TcPlan plan_score16(int64_t n);
-size_t tc_score16_ws_bytes(const TcPlan& pl, int64_t n);
-// Empirical-score partials: ppdf [2 * splits][n], pw [splits][n][16] (centred).
+size_t tc_score16_ws_bytes(const TcPlan& pl);
+// Empirical-score partials as (value, error) pairs, self pair excluded:
+// ppdf [segment][column half][256], pw [segment][256][16] (centred); both in
+// the kernel's scaled units (phi 2^15, x 2^ew).
+struct ScPartials {
+  const float2* ppdf;
+  const float2* pw;
+  const TcScales* scales;
+  WorkLine line;
+};
 int launch_score16_tc(const float* x, int64_t n, const float* mu, double h, const TcPlan& pl, WsCarver& c,
-                      double** ppdf_out, double** pw_out, cudaStream_t s);
+                      ScPartials* out, cudaStream_t s);
 int launch_mma_probe(const float* a, const float* b, float* d, cudaStream_t s);
 int launch_mma_ts_probe(const float* a, const float* b, float* d, cudaStream_t s);
 int launch_tmem_cp_probe(const float* a, uint32_t* out, cudaStream_t s);
 int launch_wait_timeout_probe(int* out, cudaStream_t s);
+
+// Sum of query i's partials (row = threadIdx.x % (blockDim.x / RL) of the
+// block's rows; RL threads per row take pairs l, l + RL, ... and are added in
+// thread order through shared memory).  True for the one thread that holds
+// the sum of a row i < m.  Call with blockDim.x = 256 and all threads.
+constexpr int TC_RED_THREADS = 256;
+// One thread per row where most query blocks have at most ~3 segments.
+inline bool tc_short_rows(const TcPartials& p) { return p.line.whole >= 8 || 2 * p.line.rest >= p.line.grid; }
+template <int RL>
+__device__ __forceinline__ bool reduce_tc_row(const TcPartials& p, int64_t i, int64_t m, double& sum) {
+  constexpr int ROWS = TC_RED_THREADS / RL;
+  const int l = threadIdx.x / ROWS;
+  float2 a = make_float2(0.f, 0.f);
+  if (i < m) {
+    const int64_t qb = i / (NQT * QT);
+    int segs;
+    const int64_t seg0 = p.line.segments_of(qb, segs);
+    const float2* row = p.part + seg0 * 2 * p.row_stride + i % (NQT * QT);
+    const int pairs = 2 * segs;
+#pragma unroll 4
+    for (int k = l; k < pairs; k += RL) a = df_add(a, row[(int64_t)k * p.row_stride]);
+  }
+  if (RL > 1) {
+    __shared__ float2 sh[RL][ROWS];
+    const int r = threadIdx.x % ROWS;
+    sh[l][r] = a;
+    __syncthreads();
+    if (l > 0) return false;
+#pragma unroll
+    for (int j = 1; j < RL; ++j) a = df_add(a, sh[j][r]);
+  }
+  sum = (double)a.x + (double)a.y;
+  return i < m;
+}
 
 // fp16 core-matrix offset of element (row r, k) in an image whose rows are
 // `row_bytes` wide (K = row_bytes / 2).

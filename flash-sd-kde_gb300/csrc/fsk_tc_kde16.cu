@@ -4,7 +4,7 @@
 // What it computes (per query q_i): sum_j exp(-||q_i - x_j||^2 / (2 h^2)),
 // optionally times the Laplace factor (1 + d/2 - ||q_i-x_j||^2/(2h^2)); the
 // quantity of kernels/kde_eval_16d_stream_splitk.py:14-81 (pass A) and
-// kernels/flash_sd_kde/kde.py:103-144, as FP64 partial sums per data split.
+// kernels/flash_sd_kde/kde.py:103-144, as partial sums per segment (fsk_reduce.cu adds them).
 //
 // How:
 //  * Coordinates are centred on the data mean mu (FP32).  With c2 =
@@ -24,8 +24,8 @@
 //  * Epilogue: tcgen05.ld one query row per thread, 2^D on the SFU
 //    (ex2.approx), 32-column chunk sums, compensated (TwoSum) per query.
 //  * Exact near-pair recompute: when a 32-column chunk holds more than 1/8
-//    of its query's running sum (carried across the data splits a CTA runs
-//    for that query block), the chunk's largest term is recomputed from
+//    of its query's running sum (of its segment: the data tiles one CTA runs
+//    for the query block), the chunk's largest term is recomputed from
 //    direct FP32 differences of the original coordinates (kept in the data
 //    stage) with the exponent product in double-float, and replaces its
 //    approximation.  The argmax rides in the low 5 mantissa bits, so all
@@ -41,10 +41,10 @@
 //             warp 17 owns TMEM (512 columns).
 //   warps 0-15: epilogue; warp w reads TMEM lanes 32*(w%4).. and columns
 //             64*((w/4)%2).. of query tile w/8.
-// A work unit is 256 queries (two M=128 tiles) x one data split; TMEM holds
-// two accumulator buffers x two query tiles x 128 columns.  Each query's sum
-// is kept as two column halves by two threads and written as two FP64
-// partial rows per split.
+// A work unit (segment, see WorkLine) is 256 queries (two M=128 tiles) x a run
+// of data tiles; TMEM holds two accumulator buffers x two query tiles x 128
+// columns.  Each query's sum is kept as two column halves by two threads and
+// written as two rows of (value, error) pairs per segment.
 #include <cuda_fp16.h>
 
 #include "fsk_kernels.cuh"
@@ -53,6 +53,12 @@
 
 namespace fsk {
 namespace tc {
+
+// Out of line: inlined into the three roles it costs the epilogue 8 bytes of
+// spills per tile (192 against 186 ms at n = m = 2^20).
+static __device__ __noinline__ Segment next_segment(const WorkLine& w, int done) {
+  return segment_at(w, blockIdx.x, done);
+}
 
 // SINGLE: the single-pass precision rung (FSK_PREC_FP16_SINGLE) - only the
 // hi.hi cross product (one fp16 product per feature, FP32 accumulation) and
@@ -102,15 +108,6 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // Work units are (query block, data split), query-block-major; each CTA
-  // takes one contiguous range of units so consecutive splits of a query
-  // block run back to back and the epilogue can carry its running sums.
-  const int64_t units = p.q_blocks * p.splits;
-  const int64_t u_begin = (int64_t)blockIdx.x * units / gridDim.x;
-  const int64_t u_end = (int64_t)(blockIdx.x + 1) * units / gridDim.x;
-  const int64_t qb_begin = u_begin / p.splits;
-  const int64_t sp_begin = u_begin - qb_begin * p.splits;
-
   if (warp == PRODUCER_WARP) {
     // the whole warp runs the loop (warp-uniform values stay in uniform
     // registers); lane 0 issues the copies
@@ -119,18 +116,18 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       uint32_t& k = n_query_copies;
       int s = 0;
       uint32_t ph = 0;
-      int64_t qb = qb_begin, sp = sp_begin;
-      for (int64_t u = u_begin; u < u_end; ++u) {
+      for (int done_tiles = 0;;) {
+        const Segment sg = next_segment(p.line, done_tiles);
+        if (sg.count == 0) break;
+        done_tiles += sg.count;
         if (!__all_sync(0xffffffffu, mbar_wait(qempty, (k & 1u) ^ 1u, 1))) goto done;
         if (lane == 0) {
           mbar_arrive_expect_tx(qready, A_BYTES);
-          bulk_g2s(sA, p.qimg + qb * (int64_t)A_BYTES, A_BYTES, qready);
+          bulk_g2s(sA, p.qimg + sg.qb * (int64_t)A_BYTES, A_BYTES, qready);
         }
         ++k;
-        const int64_t t0 = sp * p.tiles_per_split;
-        const int64_t t1 = imin<int64_t>(p.n_tiles, t0 + p.tiles_per_split);
-        const uint8_t* src = p.ximg + t0 * (int64_t)KB_STAGE_BYTES;
-        for (int64_t t = t0; t < t1; ++t, src += KB_STAGE_BYTES) {
+        const uint8_t* src = p.ximg + sg.t0 * (int64_t)KB_STAGE_BYTES;
+        for (int i = 0; i < sg.count; ++i, src += KB_STAGE_BYTES) {
           if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1u, 2))) goto done;
           if (lane == 0) {
             mbar_arrive_expect_tx(&full[s], KB_STAGE_BYTES);
@@ -141,10 +138,6 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
             s = 0;
             ph ^= 1u;
           }
-        }
-        if (++sp == p.splits) {
-          sp = 0;
-          ++qb;
         }
       }
     }
@@ -168,11 +161,11 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       const uint32_t d0 = tmem_base + (uint32_t)(a * KNT);
       uint32_t g = 0, k = 0, ph = 0;
       int s = 0;
-      int64_t sp = sp_begin;
-      for (int64_t u = u_begin; u < u_end; ++u, ++k) {
+      for (int done_tiles = 0;; ++k) {
+        const int nt = next_segment(p.line, done_tiles).count;
+        if (nt == 0) break;
+        done_tiles += nt;
         if (!__all_sync(0xffffffffu, mbar_wait(qready, k & 1u, 3))) goto done;
-        const int64_t t0 = sp * p.tiles_per_split;
-        const int nt = (int)(imin<int64_t>(p.n_tiles, t0 + p.tiles_per_split) - t0);
         for (int i = 0; i < nt; ++i, ++g) {
           const uint32_t b = g & 1u;
           if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, 4))) goto done;
@@ -195,7 +188,6 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         }
         if (lane == 0) mma_commit(qempty);
         __syncwarp();
-        if (++sp == p.splits) sp = 0;
       }
     }
   } else {
@@ -211,31 +203,29 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
     constexpr int QS_STRIDE = EPI_WARPS * 32;
     uint32_t g = 0;
     int s = 0;
-    int64_t prev_qb = -1;
-    int64_t qb = qb_begin, sp = sp_begin;
-    float s_carry = 0.f;   // approximate sum of this query's half over the splits already done here
-    for (int64_t u = u_begin; u < u_end; ++u) {
-      if (qb != prev_qb) {
-        s_carry = 0.f;
-        prev_qb = qb;
-      }
-      const int64_t gi = qb * (NQT * QT) + qt * QT + quarter * 32 + lane;   // padded query index
+    const int last_t = (int)p.line.n_tiles - 1;
+    // valid columns of this thread's half of the last (possibly ragged) data
+    // tile; every other tile has KNT / 2
+    const int last_valid = (int)imin<int64_t>(KNT / 2, p.n - ((int64_t)last_t * KNT + half * (KNT / 2)));
+    for (int done_tiles = 0;;) {
+      const Segment sg = next_segment(p.line, done_tiles);
+      if (sg.count == 0) break;
+      done_tiles += sg.count;
+      const int qrow = qt * QT + quarter * 32 + lane;                   // row in the query block
+      const int64_t gi = (int64_t)sg.qb * (NQT * QT) + qrow;            // padded query index
       // this query's FP32 row into the thread's own shared-memory slot (read
       // only by the exact recompute; the slot is rewritten only by this thread)
       {
-        const float4* src = reinterpret_cast<const float4*>(p.qexact + gi * FSK_D);
+        // scalar loads: the caller's rows need only 4-byte alignment
+        const float* src = p.q + (gi < p.m ? gi : 0) * FSK_D;
 #pragma unroll
-        for (int kk = 0; kk < FSK_D / 4; ++kk) qslot[kk * QS_STRIDE] = src[kk];
+        for (int kk = 0; kk < FSK_D / 4; ++kk)
+          qslot[kk * QS_STRIDE] = make_float4(src[4 * kk], src[4 * kk + 1], src[4 * kk + 2], src[4 * kk + 3]);
       }
       Comp acc{0.f, 0.f};
       float corr = 0.f;
-      const int64_t t0 = sp * p.tiles_per_split;
-      const int nt = (int)(imin<int64_t>(p.n_tiles, t0 + p.tiles_per_split) - t0);
-      // columns of this thread's half of tile t0 + i: first data index and valid count
-      // valid columns of this thread's half of the last (possibly ragged) data
-      // tile; every other tile has KNT / 2
-      const int last_i = (int)(p.n_tiles - 1 - t0);
-      const int last_valid = (int)imin<int64_t>(KNT / 2, p.n - ((p.n_tiles - 1) * KNT + half * (KNT / 2)));
+      const int last_i = last_t - sg.t0;
+      const int nt = sg.count;
       for (int i = 0; i < nt; ++i, ++g) {
         const uint32_t b = g & 1u;
         const int valid = i == last_i ? last_valid : KNT / 2;   // may be <= 0 on the last tile
@@ -303,7 +293,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
             float cs = pa.x + pa.y;
             // Near-pair test: a chunk holding more than NEAR_FRACTION of the
             // running sum (this chunk included) may contain a dominant term.
-            const float run = s_carry + fabsf(acc.s) + fabsf(tsum);
+            const float run = fabsf(acc.s) + fabsf(tsum);
             const bool trig = !SINGLE && fabsf(cs) > (run + fabsf(cs)) * NEAR_FRACTION;
             if (!SINGLE && __any_sync(0xffffffffu, trig)) {
               // Triggered lanes replace their chunk's largest term by its exact
@@ -365,19 +355,16 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         if (lane == 0) mbar_arrive(&empty[s]);
         if (++s == NS) s = 0;
       }
-      s_carry += fabsf(acc.s + corr);
       if (gi < p.m) {
-        const double v = (double)acc.s + (double)acc.c + (double)corr;
         if (p.atomic_acc) {
+          const double v = (double)acc.s + (double)acc.c + (double)corr;
           if (in_bounds(gi, p.m, 40)) atomicAdd(&p.atomic_acc[gi], v);
         } else {
-          const int64_t idx = (2 * sp + half) * p.m + gi;
-          if (in_bounds(idx, 2 * p.splits * p.m, 41)) p.partials[idx] = v;
+          // (value, error) pair: the FP64 unit (2 lanes per clock per SM) stays out of the segment's end
+          const int64_t idx = (p.line.segment_id(sg.qb, blockIdx.x) * 2 + half) * p.row_stride + qrow;
+          if (in_bounds(idx, p.line.segment_bound() * 2 * p.row_stride, 41))
+            p.partials[idx] = make_float2(acc.s, acc.c + corr);
         }
-      }
-      if (++sp == p.splits) {
-        sp = 0;
-        ++qb;
       }
     }
   }
@@ -494,8 +481,8 @@ __global__ void prep_data_kernel(const float* __restrict__ x, int64_t n, int64_t
   for (int k = 0; k < 4; ++k) xr[k] = make_float4(xo[4 * k], xo[4 * k + 1], xo[4 * k + 2], xo[4 * k + 3]);
 }
 
-// query tile image: [H (QT x 32 fp16) | L (QT x 16 fp16)], plus the original
-// coordinates for the exact recompute.
+// query tile image: [H (QT x 32 fp16) | M | L (QT x 16 fp16)], plus (score
+// kernel) the original coordinates, padded to whole query blocks.
 __global__ void prep_query_kernel(const float* __restrict__ q, int64_t m, int64_t m_pad,
                                   const float* __restrict__ mu, float c2, float alpha_off,
                                   const TcScales* __restrict__ sc, uint8_t* __restrict__ img,
@@ -517,33 +504,17 @@ __global__ void prep_query_kernel(const float* __restrict__ q, int64_t m, int64_
   const float alpha = ok ? (alpha_off - c2 * nrm) * sc->a_scale : 0.f;
   write_operand_row(tile, tile + A_M_OFFSET, tile + A_L_OFFSET, (int)(i % QT), v, alpha,
                     ok ? ldexpf(1.f, sc->pad[1]) : 0.f, false);
+  if (qexact == nullptr) return;
 #pragma unroll
   for (int k = 0; k < FSK_D; ++k) qexact[i * FSK_D + k] = qo[k];
 }
 
-void plan_splits(TcPlan& pl) {
-  const int64_t sms = sm_count();
-  // Data splits only add parallelism: pick the smallest split count giving
-  // every CTA >= 4 units with a near-integral number of units per CTA.
-  const int64_t s_min = imax<int64_t>(1, imin<int64_t>(pl.n_tiles, (4 * sms + pl.q_blocks - 1) / pl.q_blocks));
-  const int64_t s_max = imin<int64_t>(pl.n_tiles, 4 * s_min + 16);
-  int64_t best = s_min;
-  double best_eff = -1.0;
-  for (int64_t sp = s_min; sp <= s_max; ++sp) {
-    const int64_t tps = (pl.n_tiles + sp - 1) / sp;
-    const int64_t eff_splits = (pl.n_tiles + tps - 1) / tps;
-    const int64_t u = pl.q_blocks * eff_splits;
-    const int64_t g = imin<int64_t>(u, sms);
-    const double eff = (double)u / (double)(g * ((u + g - 1) / g));
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
-      best = sp;
-    }
-    if (eff >= 0.97) break;
-  }
-  pl.tiles_per_split = (pl.n_tiles + best - 1) / best;
-  pl.splits = (pl.n_tiles + pl.tiles_per_split - 1) / pl.tiles_per_split;  // all splits non-empty
-  pl.grid = (int)imin<int64_t>(pl.q_blocks * pl.splits, sms);
+void plan_line(TcPlan& pl) {
+  pl.line.n_tiles = pl.n_tiles;
+  pl.line.grid = (int)imin<int64_t>(pl.q_blocks * pl.n_tiles, sm_count());
+  pl.line.whole = (int)(pl.q_blocks / pl.line.grid);
+  pl.line.rest = (int)(pl.q_blocks % pl.line.grid);
+  pl.line.line_grid = (int)imax<int64_t>(1, imin<int64_t>(pl.line.grid, pl.line.rest * pl.n_tiles));
 }
 
 TcPlan plan_kde16(int64_t m, int64_t n) {
@@ -552,18 +523,18 @@ TcPlan plan_kde16(int64_t m, int64_t n) {
   pl.n_tiles = (n + KNT - 1) / KNT;
   pl.n_pad = pl.n_tiles * KNT;
   pl.q_blocks = pl.m_pad / (NQT * QT);
-  plan_splits(pl);
-  pl.part_rows = 2 * pl.splits;   // one row per (split, column half)
+  plan_line(pl);
   return pl;
 }
+
+static int kde16_row_stride(int64_t m) { return (int)imin<int64_t>(m, NQT * QT); }
 
 size_t tc_kde16_ws_bytes(const TcPlan& pl, int64_t m, bool atomic) {
   size_t b = 0;
   b += align_up(sizeof(TcScales), 256);
   b += align_up((size_t)pl.q_blocks * A_BYTES, 256);
-  b += align_up((size_t)pl.m_pad * FSK_D * sizeof(float), 256);
   b += align_up((size_t)pl.n_tiles * KB_STAGE_BYTES, 256);
-  b += align_up((size_t)(atomic ? 1 : pl.part_rows) * m * sizeof(double), 256);
+  b += align_up(atomic ? (size_t)m * sizeof(double) : (size_t)pl.line.segment_bound() * 2 * kde16_row_stride(m) * sizeof(float2), 256);
   return b;
 }
 
@@ -572,20 +543,23 @@ static cudaError_t launch_kde16_tc_kernel(const TcPlan& pl, const TcParams& p, c
   const cudaError_t e = cudaFuncSetAttribute(kde16_tc_kernel<LAPLACE, SINGLE, POLY>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return e;
-  kde16_tc_kernel<LAPLACE, SINGLE, POLY><<<pl.grid, THREADS, SMEM_BYTES, s>>>(p);
+  kde16_tc_kernel<LAPLACE, SINGLE, POLY><<<pl.line.grid, THREADS, SMEM_BYTES, s>>>(p);
   return cudaGetLastError();
 }
 
 int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, const float* mu, double h,
-                    bool laplace, bool single, bool poly, const TcPlan& pl, WsCarver& c, double** partials_out,
-                    bool atomic, cudaStream_t s) {
+                    bool laplace, bool single, bool poly, const TcPlan& pl, WsCarver& c, TcPartials* partials_out,
+                    double** atomic_out, cudaStream_t s) {
   TcScales* sc = c.take<TcScales>(1);
   uint8_t* qimg = c.take<uint8_t>((size_t)pl.q_blocks * A_BYTES);
-  float* qexact = c.take<float>((size_t)pl.m_pad * FSK_D);
   uint8_t* ximg = c.take<uint8_t>((size_t)pl.n_tiles * KB_STAGE_BYTES);
-  double* part = c.take<double>((size_t)(atomic ? 1 : pl.part_rows) * m);
+  const bool atomic = atomic_out != nullptr;
+  const int row_stride = kde16_row_stride(m);
+  double* acc = atomic ? c.take<double>((size_t)m) : nullptr;
+  float2* part = atomic ? nullptr : c.take<float2>((size_t)pl.line.segment_bound() * 2 * row_stride);
   if (!c.fits()) return FSK_ERR_WORKSPACE_TOO_SMALL;
-  *partials_out = part;
+  if (atomic) *atomic_out = acc;
+  *partials_out = TcPartials{part, pl.line, row_stride};
 
   const double c2d = FSK_LOG2E / (2.0 * h * h);
   const float c2 = (float)c2d;
@@ -603,26 +577,24 @@ int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, const 
   prep_data_kernel<<<(unsigned)((pl.n_pad + 255) / 256), 256, 0, s>>>(x, n, pl.n_pad, mu, c2, sc, ximg);
   count_launch();
   prep_query_kernel<<<(unsigned)((pl.m_pad + 255) / 256), 256, 0, s>>>(q, m, pl.m_pad, mu, c2, 0.f, sc, qimg,
-                                                                        qexact);
+                                                                        nullptr);
   count_launch();
-  if (atomic) launch_zero(part, m, s);
+  if (atomic) launch_zero(acc, m, s);
 
   TcParams p;
   p.qimg = qimg;
   p.ximg = ximg;
-  p.qexact = qexact;
+  p.q = q;
   p.scales = sc;
   p.m = m;
   p.n = n;
-  p.n_tiles = pl.n_tiles;
-  p.q_blocks = pl.q_blocks;
-  p.splits = pl.splits;
-  p.tiles_per_split = pl.tiles_per_split;
+  p.line = pl.line;
   p.c2 = c2;
   p.c2_lo = c2_lo;
   p.c1 = (float)(1.0 / (2.0 * h * h));
-  p.partials = atomic ? nullptr : part;
-  p.atomic_acc = atomic ? part : nullptr;
+  p.partials = part;
+  p.row_stride = row_stride;
+  p.atomic_acc = acc;
   cudaError_t e;
   TimerScope ts(K_KDE16_TC, (double)m * (double)n, s);
   if (laplace)

@@ -6,7 +6,7 @@
 //   weighted_sum_i = sum_j phi_ij x_j
 // the accumulators of kernels/flash_sd_kde/empirical.py:72-131 and
 // kernels/emp_score_16d_ordered_splitk.py:20-95 (both tl.dot products with
-// allow_tf32), as FP64 partials per data split; the weighted sum is kept
+// allow_tf32), as (value, error) partials per segment (see WorkLine); the weighted sum is kept
 // centred (sum_j phi_ij (x_j - mu)) and mu * pdf_sum is added back in FP64.
 //
 // How (per 256-query x 64-point tile):
@@ -41,7 +41,7 @@
 //             (0, hi), (0, lo), (1, hi), (1, lo).
 //   warps 0-15: epilogue; warp w: query tile w/8, data-column half (w/4)&1,
 //             TMEM lane quarter w&3.  The two column halves of a row keep
-//             separate pdf partials (written as two virtual splits) and
+//             separate pdf partials (two rows per segment) and
 //             read disjoint halves of the weighted-sum features.
 // TMEM: A operands [2 query tiles][hi 16 | mid 8 | lo 8]  (columns 0-63)
 //       | S / weights [NBUF buffers][2 query tiles][64]  (64-319)
@@ -96,7 +96,6 @@ constexpr int S_WACC_OFFSET = S_WCORR_OFFSET + S_WCORR_BYTES;
 constexpr int S_WACC_BYTES = 4 * S_EPI_WARPS * 32 * 16;                // 32 KB
 constexpr int S_MU_OFFSET = S_WACC_OFFSET + S_WACC_BYTES;             // data mean, 16 FP32
 constexpr int S_SMEM_BYTES = S_MU_OFFSET + FSK_D * 4;
-constexpr float PHI_LOG2_SCALE = 15.0f;                    // weights are phi * 2^15
 // Three-part S product as in the KDE kernel, so the same near-pair threshold
 // (1/8 of the running sum, the excluded self pair's weight included).
 constexpr float SCORE_NEAR_FRACTION = NEAR_FRACTION;
@@ -113,10 +112,13 @@ struct ScParams {
   const TcScales* scales;
   const float* mu;
   int64_t n;
-  int64_t n_tiles, q_blocks, splits, tiles_per_split;
+  WorkLine line;
   float c2, c2_lo;
-  double* ppdf;   // [2 * splits][n]  (split sp, column half h at 2 sp + h), self pair excluded
-  double* pw;     // [splits][n][16]  centred weighted sums, self pair excluded
+  // (value, error) pairs per segment, self pair excluded, in the kernel's
+  // scaled units: pdf [segment][column half][256], centred weighted sums
+  // [segment][256][16]
+  float2* ppdf;
+  float2* pw;
 };
 
 // f32 pair -> packed fp16 hi and lo parts (hi + lo = v to ~22 bits).  The
@@ -132,30 +134,6 @@ __device__ __forceinline__ void split_pack(float v0, float v1, uint32_t& hi, uin
       : "r"(hi), "f"(v0), "f"(v1), "h"(minus_one));
   asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(r1), "f"(r0));
 }
-
-// Walks the (unit, data tile) sequence of one CTA: units are (query block,
-// data split), each split covers tiles [t0, t1).
-struct TileCursor {
-  int u, u_end, splits, tps, n_tiles, t0, t1, t;
-  __device__ void start(int ub, int ue, int sp_count, int tiles_per_split, int tiles) {
-    u = ub; u_end = ue; splits = sp_count; tps = tiles_per_split; n_tiles = tiles;
-    enter();
-  }
-  __device__ void enter() {
-    if (u < u_end) {
-      t0 = (u % splits) * tps;
-      t1 = min(n_tiles, t0 + tps);
-      t = t0;
-    }
-  }
-  __device__ bool done() const { return u >= u_end; }
-  __device__ void next() {
-    if (++t >= t1) {
-      ++u;
-      enter();
-    }
-  }
-};
 
 __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -216,9 +194,6 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const int64_t units = p.q_blocks * p.splits;
-  const int64_t u_begin = (int64_t)blockIdx.x * units / gridDim.x;
-  const int64_t u_end = (int64_t)(blockIdx.x + 1) * units / gridDim.x;
 
   if (warp == S_PRODUCER_WARP) {
     // whole warp runs the loop (32-bit stage / phase counters), lane 0 copies
@@ -227,19 +202,19 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       int64_t& k = n_query_copies;
       int st = 0;
       uint32_t ph = 0;
-      for (int64_t u = u_begin; u < u_end; ++u) {
-        const int64_t qb = u / p.splits, sp = u % p.splits;
+      for (int done_tiles = 0;;) {
+        const Segment sg = segment_at(p.line, blockIdx.x, done_tiles);
+        if (sg.count == 0) break;
+        done_tiles += sg.count;
         if (!__all_sync(0xffffffffu, mbar_wait(qempty, (uint32_t)((k & 1) ^ 1), 21))) goto done;
         if (lane == 0) {
           mbar_arrive_expect_tx(qready, S_A_BYTES + S_QX_BYTES);
-          bulk_g2s(sA, p.qimg + qb * (int64_t)S_A_BYTES, S_A_BYTES, qready);
-          bulk_g2s(smem_raw + S_QX_OFFSET, p.qexact + qb * (int64_t)(SNQT * QT * FSK_D), S_QX_BYTES, qready);
+          bulk_g2s(sA, p.qimg + sg.qb * (int64_t)S_A_BYTES, S_A_BYTES, qready);
+          bulk_g2s(smem_raw + S_QX_OFFSET, p.qexact + sg.qb * (int64_t)(SNQT * QT * FSK_D), S_QX_BYTES, qready);
         }
         ++k;
-        const int64_t t0 = sp * p.tiles_per_split;
-        const int64_t t1 = imin<int64_t>(p.n_tiles, t0 + p.tiles_per_split);
-        const uint8_t* src = p.ximg + t0 * (int64_t)S_STAGE_BYTES;
-        for (int64_t t = t0; t < t1; ++t, src += S_STAGE_BYTES) {
+        const uint8_t* src = p.ximg + sg.t0 * (int64_t)S_STAGE_BYTES;
+        for (int i = 0; i < sg.count; ++i, src += S_STAGE_BYTES) {
           if (!__all_sync(0xffffffffu, mbar_wait(&empty[st], ph ^ 1u, 22))) goto done;
           if (lane == 0) {
             mbar_arrive_expect_tx(&full[st], S_STAGE_BYTES);
@@ -270,39 +245,39 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       const uint64_t dh0 = smem_desc_kmajor(b0, 128, 8 * H_ROW_BYTES);
       const uint64_t dm0 = smem_desc_kmajor(b0 + B_M_OFFSET, 128, 8 * L_ROW_BYTES);
       const uint64_t dl0 = smem_desc_kmajor(b0 + B_L_OFFSET, 128, 8 * L_ROW_BYTES);
-      TileCursor cs;
-      cs.start((int)u_begin, (int)u_end, (int)p.splits, (int)p.tiles_per_split, (int)p.n_tiles);
       int gs = 0, ku = 0;
-      while (!cs.done()) {
-        const int s = gs % SNS;
-        const int b = gs % NBUF;
-        if (cs.t == cs.t0) {   // first tile of a unit: its A operand in TMEM
-          if (!__all_sync(0xffffffffu, mbar_wait(&aready[a], (uint32_t)(ku & 1), 23))) goto done;
-          ++ku;
+      for (int done_tiles = 0;;) {
+        const int count = segment_at(p.line, blockIdx.x, done_tiles).count;
+        if (count == 0) break;
+        done_tiles += count;
+        // the segment's A operand in TMEM
+        if (!__all_sync(0xffffffffu, mbar_wait(&aready[a], (uint32_t)(ku & 1), 23))) goto done;
+        ++ku;
+        for (int i = 0; i < count; ++i, ++gs) {
+          const int s = gs % SNS;
+          const int b = gs % NBUF;
+          if (gs >= NBUF &&
+              !__all_sync(0xffffffffu, mbar_wait(&sfree[b * SNQT + a], (uint32_t)(((gs / NBUF) - 1) & 1), 25)))
+            goto done;
+          if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)((gs / SNS) & 1), 24))) goto done;
+          tc_fence_after();
+          const uint64_t so = (uint64_t)((s * S_STAGE_BYTES) >> 4);
+          const uint32_t d = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
+          const uint64_t b_h = dh0 + so;
+          // three-part product, small terms first (the order of mma_s_tile)
+          const uint64_t b_m = dm0 + so, b_l = dl0 + so;
+          if (lane == 0) {
+            mma_f16_ts(d, a_h + 16u, b_m, idesc_s, 0u);                    // mid . mid
+            mma_f16_ts(d, a_h, b_l, idesc_s, 1u);                          // hi . lo
+            mma_f16_ts(d, a_h + 24u, b_h, idesc_s, 1u);                    // lo . hi
+            mma_f16_ts(d, a_h, b_m, idesc_s, 1u);                          // hi . mid
+            mma_f16_ts(d, a_h + 16u, b_h, idesc_s, 1u);                    // mid . hi
+            mma_f16_ts(d, a_h, b_h, idesc_s, 1u);                          // hi . hi
+            mma_f16_ts(d, a_h + 8u, b_h + (uint64_t)(256 >> 4), idesc_s, 1u);   // bias . bias
+            mma_commit(&tfull[b * SNQT + a]);
+          }
+          __syncwarp();
         }
-        if (gs >= NBUF &&
-            !__all_sync(0xffffffffu, mbar_wait(&sfree[b * SNQT + a], (uint32_t)(((gs / NBUF) - 1) & 1), 25)))
-          goto done;
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)((gs / SNS) & 1), 24))) goto done;
-        tc_fence_after();
-        const uint64_t so = (uint64_t)((s * S_STAGE_BYTES) >> 4);
-        const uint32_t d = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
-        const uint64_t b_h = dh0 + so;
-        // three-part product, small terms first (the order of mma_s_tile)
-        const uint64_t b_m = dm0 + so, b_l = dl0 + so;
-        if (lane == 0) {
-          mma_f16_ts(d, a_h + 16u, b_m, idesc_s, 0u);                    // mid . mid
-          mma_f16_ts(d, a_h, b_l, idesc_s, 1u);                          // hi . lo
-          mma_f16_ts(d, a_h + 24u, b_h, idesc_s, 1u);                    // lo . hi
-          mma_f16_ts(d, a_h, b_m, idesc_s, 1u);                          // hi . mid
-          mma_f16_ts(d, a_h + 16u, b_h, idesc_s, 1u);                    // mid . hi
-          mma_f16_ts(d, a_h, b_h, idesc_s, 1u);                          // hi . hi
-          mma_f16_ts(d, a_h + 8u, b_h + (uint64_t)(256 >> 4), idesc_s, 1u);   // bias . bias
-          mma_commit(&tfull[b * SNQT + a]);
-        }
-        __syncwarp();
-        ++gs;
-        cs.next();
       }
     }
   } else if (warp >= W_MMA_WARP) {
@@ -314,39 +289,40 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       const int a = wi >> 1, part = wi & 1;   // part 0: hi weights x [X_hi | X_lo]; 1: lo weights x X_hi
       const uint32_t idesc_w = idesc_f16_f32(QT, part ? WN_LO : WN);
       const uint64_t dx0 = smem_desc_kmajor(smem_u32(sB) + S_XTH_OFFSET, 128, 8 * XT_ROW_BYTES);
-      TileCursor cw;
-      cw.start((int)u_begin, (int)u_end, (int)p.splits, (int)p.tiles_per_split, (int)p.n_tiles);
       int gw = 0, grp = 0;
-      while (!cw.done()) {
-        const int b = gw % NBUF;
-        const int s = gw % SNS;
-        const int pos = (cw.t - cw.t0) % S_GROUP;
-        const bool first = pos == 0;
-        const bool last = pos == S_GROUP - 1 || cw.t == cw.t1 - 1;
-        const int par = grp & 1;
-        if (first &&
-            !__all_sync(0xffffffffu, mbar_wait(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
-          goto done;
-        if (!__all_sync(0xffffffffu, mbar_wait(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
-        tc_fence_after();
-        const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
-        const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT + part * 16);
-        const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS + part * WN);
-        if (lane == 0) {
+      for (int done_tiles = 0;;) {
+        const int count = segment_at(p.line, blockIdx.x, done_tiles).count;
+        if (count == 0) break;
+        done_tiles += count;
+        for (int i = 0; i < count; ++i, ++gw) {
+          const int b = gw % NBUF;
+          const int s = gw % SNS;
+          const int pos = i % S_GROUP;
+          const bool first = pos == 0;
+          const bool last = pos == S_GROUP - 1 || i == count - 1;
+          const int par = grp & 1;
+          if (first &&
+              !__all_sync(0xffffffffu, mbar_wait(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
+            goto done;
+          if (!__all_sync(0xffffffffu, mbar_wait(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
+          tc_fence_after();
+          const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
+          const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT + part * 16);
+          const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS + part * WN);
+          if (lane == 0) {
 #pragma unroll
-          for (int ks = 0; ks < NT / 16; ++ks) {
-            // data columns 16 ks .. +15: column half ks/2; weights hi at +0, lo at +16
-            const uint32_t wa = ph + (uint32_t)(32 * (ks >> 1) + 8 * (ks & 1));
-            mma_f16_ts(d, wa, xd0 + (uint64_t)(ks * (256 >> 4)), idesc_w, (first && ks == 0) ? 0u : 1u);
+            for (int ks = 0; ks < NT / 16; ++ks) {
+              // data columns 16 ks .. +15: column half ks/2; weights hi at +0, lo at +16
+              const uint32_t wa = ph + (uint32_t)(32 * (ks >> 1) + 8 * (ks & 1));
+              mma_f16_ts(d, wa, xd0 + (uint64_t)(ks * (256 >> 4)), idesc_w, (first && ks == 0) ? 0u : 1u);
+            }
+            mma_commit(&sfree[b * SNQT + a]);
+            mma_commit(&empty[s]);
+            if (last) mma_commit(&wfull[par * SNQT + a]);
           }
-          mma_commit(&sfree[b * SNQT + a]);
-          mma_commit(&empty[s]);
-          if (last) mma_commit(&wfull[par * SNQT + a]);
+          __syncwarp();
+          if (last) ++grp;
         }
-        __syncwarp();
-        if (last) ++grp;
-        ++gw;
-        cw.next();
       }
     }
   } else {
@@ -374,17 +350,13 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
     int g = 0, grp = 0, k_unit = 0;
     int s = 0;   // data stage of tile g (g % SNS, advanced per tile)
     // valid columns of the last (possibly ragged) data tile; every other tile has NT
-    const int last_t = (int)p.n_tiles - 1;
+    const int last_t = (int)p.line.n_tiles - 1;
     const int last_valid = (int)(p.n - (int64_t)last_t * NT);
-    int prev_qb = -1;
-    float s_carry = 0.f;
-    const int splits = (int)p.splits, tps = (int)p.tiles_per_split, n_tiles = (int)p.n_tiles;
-    for (int u = (int)u_begin; u < (int)u_end; ++u, ++k_unit) {
-      const int qb = u / splits, sp = u % splits;
-      if (qb != prev_qb) {
-        s_carry = phi_scale;   // the self pair
-        prev_qb = qb;
-      }
+    for (int done_tiles = 0;; ++k_unit) {
+      const Segment sg = segment_at(p.line, blockIdx.x, done_tiles);
+      if (sg.count == 0) break;
+      done_tiles += sg.count;
+      const int qb = sg.qb;
       const int gi = qb * (SNQT * QT) + qt * QT + row;
       const int diag_col = qb * (SNQT * QT) + qt * QT + quarter * 32;   // this warp's rows
       float* wc = wcorr + (k_unit & 1) * WC_PAR + half * WC_HALF + wc_row;
@@ -423,8 +395,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       constexpr int EPI_T = S_EPI_WARPS * 32;
 #pragma unroll
       for (int k = 0; k < 4; ++k) wacc[k * EPI_T + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int t0 = sp * tps;
-      const int t1 = imin(n_tiles, t0 + tps);
+      const int t0 = sg.t0;
+      const int t1 = t0 + sg.count;
       bool pend = false;     // a W group ended at the previous tile and is not read yet
       for (int t = t0; t < t1; ++t, ++g, s = (s + 1 == SNS) ? 0 : s + 1) {
         const int b = g % NBUF;
@@ -466,7 +438,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         }
         pa = __fadd2_rn(pa, pb);
         const float cs = pa.x + pa.y;
-        const bool trig = cs > (s_carry + acc.s + cs) * SCORE_NEAR_FRACTION;
+        const bool trig = cs > (phi_scale + acc.s + cs) * SCORE_NEAR_FRACTION;   // phi_scale: the self pair
         if (__any_sync(0xffffffffu, trig)) {
           // The chunk's largest weight is recomputed exactly (argmax on keys
           // = value bits with the column in the low 5 bits, as in the KDE
@@ -580,7 +552,6 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         }
         if (last && t != t1 - 1) pend = true;
       }
-      s_carry += acc.s + corr;
       // Combine the two column halves' corrections of this row for the 8
       // features this warp outputs.  Buffers alternate by unit parity; the
       // previous parity is cleared once every warp has passed this unit's
@@ -598,25 +569,26 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
           *reinterpret_cast<float4*>(wc_next + k) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
       if (gi < p.n) {
-        const double p_unscale = 1.0 / 32768.0;   // 2^-PHI_LOG2_SCALE
-        const double c_unscale = p_unscale;
-        const double w_unscale = ldexp(p_unscale, -p.scales->pad[2]);
-        const int64_t pidx = (int64_t)(2 * sp + half) * p.n + gi;
-        if (in_bounds(pidx, 2 * p.splits * p.n, 42))
-          p.ppdf[pidx] = ((double)acc.s + (double)acc.c + (double)corr) * p_unscale;
-        const int64_t wbase = ((int64_t)sp * p.n + gi) * FSK_D + half * 8;   // 8 features from here
-        const bool w_ok = in_bounds(wbase, p.splits * p.n * FSK_D - 7, 43);
-        double* wrow = p.pw + wbase;
-        const float* c0 = wcorr + (k_unit & 1) * WC_PAR + wc_row + half * 8;
-        const float* c1 = c0 + WC_HALF;
-        const float4 s0 = wacc[threadIdx.x], s1 = wacc[EPI_T + threadIdx.x];
-        const float4 e0 = wacc[2 * EPI_T + threadIdx.x], e1 = wacc[3 * EPI_T + threadIdx.x];
-        const float ws[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-        const float we[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+        // (value, error) pairs in the kernel's units: the FP64 unit (2 lanes
+        // per clock per SM) took ~8 us per unit here when these were FP64 sums
+        const float w_mul = ldexpf(1.f, p.scales->pad[2]);   // weighted-sum operand scale 2^ew
+        const int64_t seg = p.line.segment_id(qb, blockIdx.x);
+        const int64_t n_seg = p.line.segment_bound();
+        const int64_t pidx = (2 * seg + half) * (SNQT * QT) + qt * QT + row;
+        if (in_bounds(pidx, 2 * n_seg * (SNQT * QT), 42)) p.ppdf[pidx] = make_float2(acc.s, acc.c + corr);
+        const int64_t wbase = (seg * (SNQT * QT) + qt * QT + row) * FSK_D + half * 8;   // 8 features from here
+        const bool w_ok = in_bounds(wbase, n_seg * (SNQT * QT) * FSK_D - 7, 43);
+        float4* wrow = reinterpret_cast<float4*>(p.pw + wbase);
+        const float4* c0 = reinterpret_cast<const float4*>(wcorr + (k_unit & 1) * WC_PAR + wc_row + half * 8);
+        const float4* c1 = c0 + WC_HALF / 4;
         if (w_ok) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            wrow[k] = ((double)ws[k] + (double)we[k]) * w_unscale + ((double)c0[k] + (double)c1[k]) * c_unscale;
+          for (int k = 0; k < 2; ++k) {
+            const float4 v = wacc[k * EPI_T + threadIdx.x], e = wacc[(2 + k) * EPI_T + threadIdx.x];
+            const float4 a = c0[k], b = c1[k];
+            wrow[2 * k] = make_float4(v.x, fmaf(a.x + b.x, w_mul, e.x), v.y, fmaf(a.y + b.y, w_mul, e.y));
+            wrow[2 * k + 1] = make_float4(v.z, fmaf(a.z + b.z, w_mul, e.z), v.w, fmaf(a.w + b.w, w_mul, e.w));
+          }
         }
       }
     }
@@ -680,33 +652,31 @@ TcPlan plan_score16(int64_t n) {
   pl.n_tiles = (n + NT - 1) / NT;
   pl.n_pad = pl.n_tiles * NT;
   pl.q_blocks = pl.m_pad / (SNQT * QT);
-  plan_splits(pl);
-  pl.part_rows = 2 * pl.splits;   // pdf rows: one per (split, column half)
+  plan_line(pl);
   return pl;
 }
 
-size_t tc_score16_ws_bytes(const TcPlan& pl, int64_t n) {
+size_t tc_score16_ws_bytes(const TcPlan& pl) {
   size_t b = 0;
   b += align_up(sizeof(TcScales), 256);
   b += align_up((size_t)pl.q_blocks * S_A_BYTES, 256);
   b += align_up((size_t)pl.m_pad * FSK_D * sizeof(float), 256);
   b += align_up((size_t)pl.n_tiles * S_STAGE_BYTES, 256);
-  b += align_up((size_t)2 * pl.splits * n * sizeof(double), 256);
-  b += align_up((size_t)pl.splits * n * FSK_D * sizeof(double), 256);
+  b += align_up((size_t)pl.line.segment_bound() * 2 * SNQT * QT * sizeof(float2), 256);
+  b += align_up((size_t)pl.line.segment_bound() * SNQT * QT * FSK_D * sizeof(float2), 256);
   return b;
 }
 
 int launch_score16_tc(const float* x, int64_t n, const float* mu, double h, const TcPlan& pl, WsCarver& c,
-                      double** ppdf_out, double** pw_out, cudaStream_t s) {
+                      ScPartials* out, cudaStream_t s) {
   TcScales* sc = c.take<TcScales>(1);
   uint8_t* qimg = c.take<uint8_t>((size_t)pl.q_blocks * S_A_BYTES);
   float* qexact = c.take<float>((size_t)pl.m_pad * FSK_D);
   uint8_t* ximg = c.take<uint8_t>((size_t)pl.n_tiles * S_STAGE_BYTES);
-  double* ppdf = c.take<double>((size_t)2 * pl.splits * n);
-  double* pw = c.take<double>((size_t)pl.splits * n * FSK_D);
+  float2* ppdf = c.take<float2>((size_t)pl.line.segment_bound() * 2 * SNQT * QT);
+  float2* pw = c.take<float2>((size_t)pl.line.segment_bound() * SNQT * QT * FSK_D);
   if (!c.fits()) return FSK_ERR_WORKSPACE_TOO_SMALL;
-  *ppdf_out = ppdf;
-  *pw_out = pw;
+  *out = ScPartials{ppdf, pw, sc, pl.line};
 
   const double c2d = FSK_LOG2E / (2.0 * h * h);
   const float c2 = (float)c2d;
@@ -733,10 +703,7 @@ int launch_score16_tc(const float* x, int64_t n, const float* mu, double h, cons
   p.scales = sc;
   p.mu = mu;
   p.n = n;
-  p.n_tiles = pl.n_tiles;
-  p.q_blocks = pl.q_blocks;
-  p.splits = pl.splits;
-  p.tiles_per_split = pl.tiles_per_split;
+  p.line = pl.line;
   p.c2 = c2;
   p.c2_lo = c2_lo;
   p.ppdf = ppdf;
@@ -745,7 +712,7 @@ int launch_score16_tc(const float* x, int64_t n, const float* mu, double h, cons
                                        S_SMEM_BYTES);
   if (e != cudaSuccess) return cuda_status(e);
   TimerScope ts(K_SCORE16_TC, (double)n * (double)n, s);
-  score16_tc_kernel<<<pl.grid, S_THREADS, S_SMEM_BYTES, s>>>(p);
+  score16_tc_kernel<<<pl.line.grid, S_THREADS, S_SMEM_BYTES, s>>>(p);
   count_launch();
   return cuda_status(cudaGetLastError());
 }
