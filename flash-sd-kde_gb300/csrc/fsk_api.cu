@@ -70,7 +70,6 @@ CenterBufs take_center(WsCarver& c, int64_t n) {
 
 size_t kde16_bytes(int64_t m, int64_t n, const Kde16Plan& p) {
   WsCarver c(nullptr, 0);
-  take_center(c, n);
   if (p.ieee) {
     c.take<double>((size_t)(p.atomic ? 1 : p.simt_splits) * m);
   } else {
@@ -158,7 +157,6 @@ int fsk_kde16(const float* queries, int64_t m, const float* data, int64_t n, dou
   const Kde16Plan p = plan16(m, n, flags);
   if (!workspace || workspace_bytes < kde16_bytes(m, n, p)) return FSK_ERR_WORKSPACE_TOO_SMALL;
   WsCarver c(workspace, workspace_bytes);
-  CenterBufs cb = take_center(c, n);
   const bool laplace = (flags & FSK_LAPLACE) != 0;
   double* part = nullptr;
   tc::TcPartials tcp{};
@@ -171,8 +169,7 @@ int fsk_kde16(const float* queries, int64_t m, const float* data, int64_t n, dou
     launch_kde16_simt(queries, m, data, n, bandwidth, laplace, p.simt_splits,
                       p.atomic ? nullptr : part, p.atomic ? part : nullptr, s);
   } else {
-    launch_mean16(data, n, cb.scratch, cb.mu, cb.mu64, s);
-    st = tc::launch_kde16_tc(queries, m, data, n, cb.mu, bandwidth, laplace, (flags & FSK_PREC_FP16_SINGLE) != 0,
+    st = tc::launch_kde16_tc(queries, m, data, n, bandwidth, laplace, (flags & FSK_PREC_FP16_SINGLE) != 0,
                              (flags & FSK_EXP_OFFLOAD) != 0, p.tcp, c, &tcp, p.atomic ? &part : nullptr, s);
     if (st) return st;
   }
@@ -197,24 +194,19 @@ int fsk_kde16(const float* queries, int64_t m, const float* data, int64_t n, dou
 // CUDA-core split-K kernel (FSK_PREC_IEEE).  Symmetric variant: the
 // upper-triangle kernel, each pair's exp evaluated once, row and column sums
 // scattered with FP64 atomics.
+static bool score_on_tensor_cores(int variant, int flags) {
+  return variant != FSK_SCORE_SYMMETRIC && !(flags & FSK_PREC_IEEE);
+}
+
 static size_t empscore_bytes(int64_t n, int variant, int flags) {
+  if (score_on_tensor_cores(variant, flags)) return tc::tc_score16_ws_bytes(tc::plan_score16(n));
   WsCarver c(nullptr, 0);
   take_center(c, n);
   c.take<double>(reduce_score_scratch_doubles(n));
-  size_t b = c.used;
-  if (variant == FSK_SCORE_SYMMETRIC) {
-    c.take<double>((size_t)n);
-    c.take<double>((size_t)n * FSK_D);
-    b = c.used;
-  } else if (!(flags & FSK_PREC_IEEE)) {
-    b = align_up(b, 256) + tc::tc_score16_ws_bytes(tc::plan_score16(n));
-  } else {
-    const int splits = simt_score16_splits(n);
-    c.take<double>((size_t)splits * n);
-    c.take<double>((size_t)splits * n * FSK_D);
-    b = c.used;
-  }
-  return align_up(b, 256);
+  const size_t splits = variant == FSK_SCORE_SYMMETRIC ? 1 : simt_score16_splits(n);
+  c.take<double>(splits * n);
+  c.take<double>(splits * n * FSK_D);
+  return align_up(c.used, 256);
 }
 
 size_t fsk_empscore16_workspace_bytes(int64_t n, int variant, int flags) {
@@ -222,41 +214,98 @@ size_t fsk_empscore16_workspace_bytes(int64_t n, int variant, int flags) {
   return empscore_bytes(n, variant, flags);
 }
 
+// pdf_sum and weighted_sum on the CUDA cores.
+static void run_empscore_simt(const float* data, int64_t n, double bandwidth, int variant, float* pdf_sum,
+                              float* weighted_sum, int64_t ws_row, int64_t ws_col, WsCarver& c, cudaStream_t s) {
+  CenterBufs cb = take_center(c, n);
+  double* rscratch = c.take<double>(reduce_score_scratch_doubles(n));
+  launch_mean16(data, n, cb.scratch, cb.mu, cb.mu64, s);
+  const int splits = variant == FSK_SCORE_SYMMETRIC ? 1 : simt_score16_splits(n);
+  double* ppdf = c.take<double>((size_t)splits * n);
+  double* pw = c.take<double>((size_t)splits * n * FSK_D);
+  if (variant == FSK_SCORE_SYMMETRIC) {
+    launch_zero(ppdf, n, s);
+    launch_zero(pw, n * FSK_D, s);
+    launch_score16_sym_simt(data, n, cb.mu, bandwidth, ppdf, pw, s);
+  } else {
+    launch_score16_simt(data, n, cb.mu, bandwidth, splits, ppdf, pw, s);
+  }
+  launch_reduce_score(ppdf, pw, splits, n, cb.mu64, pdf_sum, weighted_sum, ws_row, ws_col, rscratch, s);
+}
+
+static int bad_empscore_args(const float* data, int64_t n, double bandwidth, int variant, int flags) {
+  if (!data || n < 1 || bad_bw(bandwidth)) return 1;
+  if (variant != FSK_SCORE_ORDERED && variant != FSK_SCORE_SYMMETRIC) return 1;
+  return (flags & ~(KNOWN_FLAGS & ~(FSK_PREC_FP16_SINGLE | FSK_EXP_OFFLOAD))) != 0;
+}
+
 int fsk_empscore16(const float* data, int64_t n, double bandwidth, int variant, int flags, float* pdf_sum,
                    float* weighted_sum, void* workspace, size_t workspace_bytes, void* stream) {
   NvtxRange nvtx_range("fsk_empscore16");
-  if (!data || !pdf_sum || !weighted_sum || n < 1 || bad_bw(bandwidth)) return FSK_ERR_INVALID_ARGUMENT;
-  if (variant != FSK_SCORE_ORDERED && variant != FSK_SCORE_SYMMETRIC) return FSK_ERR_INVALID_ARGUMENT;
-  if (flags & ~(KNOWN_FLAGS & ~(FSK_PREC_FP16_SINGLE | FSK_EXP_OFFLOAD))) return FSK_ERR_INVALID_ARGUMENT;
+  if (!pdf_sum || !weighted_sum || bad_empscore_args(data, n, bandwidth, variant, flags))
+    return FSK_ERR_INVALID_ARGUMENT;
   int st = check_device();
   if (st) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (!workspace || workspace_bytes < empscore_bytes(n, variant, flags)) return FSK_ERR_WORKSPACE_TOO_SMALL;
   WsCarver c(workspace, workspace_bytes);
-  CenterBufs cb = take_center(c, n);
-  double* rscratch = c.take<double>(reduce_score_scratch_doubles(n));
-  launch_mean16(data, n, cb.scratch, cb.mu, cb.mu64, s);
   const bool fm = (flags & FSK_WEIGHTED_FEATURE_MAJOR) != 0;
   const int64_t ws_row = fm ? 1 : FSK_D, ws_col = fm ? n : 1;
-  if (variant == FSK_SCORE_SYMMETRIC) {
-    double* apdf = c.take<double>((size_t)n);
-    double* aw = c.take<double>((size_t)n * FSK_D);
-    launch_zero(apdf, n, s);
-    launch_zero(aw, n * FSK_D, s);
-    launch_score16_sym_simt(data, n, cb.mu, bandwidth, apdf, aw, s);
-    launch_reduce_score(apdf, aw, 1, n, cb.mu64, pdf_sum, weighted_sum, ws_row, ws_col, rscratch, s);
-  } else if (!(flags & FSK_PREC_IEEE)) {
-    const tc::TcPlan pl = tc::plan_score16(n);
+  if (score_on_tensor_cores(variant, flags)) {
     tc::ScPartials parts{};
-    st = tc::launch_score16_tc(data, n, cb.mu, bandwidth, pl, c, &parts, s);
+    st = tc::launch_score16_tc(data, n, bandwidth, tc::plan_score16(n), c, &parts, s);
     if (st) return st;
-    launch_reduce_score_tc(parts, n, cb.mu, data, pdf_sum, weighted_sum, ws_row, ws_col, s);
+    launch_reduce_score_tc(parts, n, data, ScoreOut{pdf_sum, weighted_sum, ws_row, ws_col, nullptr, nullptr}, bandwidth,
+                           0.0, s);
   } else {
-    const int splits = simt_score16_splits(n);
-    double* ppdf = c.take<double>((size_t)splits * n);
-    double* pw = c.take<double>((size_t)splits * n * FSK_D);
-    launch_score16_simt(data, n, cb.mu, bandwidth, splits, ppdf, pw, s);
-    launch_reduce_score(ppdf, pw, splits, n, cb.mu64, pdf_sum, weighted_sum, ws_row, ws_col, rscratch, s);
+    run_empscore_simt(data, n, bandwidth, variant, pdf_sum, weighted_sum, ws_row, ws_col, c, s);
+  }
+  return cuda_status(cudaGetLastError());
+}
+
+// ---- score and debias shift in one call --------------------------------------------
+// Tensor cores: the reduction of the score partials writes the shifted points
+// itself.  CUDA cores: pdf_sum and weighted_sum (in the workspace where the
+// caller does not take them), then the shift of fsk_debias16.
+static size_t sdshift_bytes(int64_t n, int variant, int flags) {
+  if (score_on_tensor_cores(variant, flags)) return empscore_bytes(n, variant, flags);
+  WsCarver c(nullptr, 0);
+  c.take<float>((size_t)n);
+  c.take<float>((size_t)n * FSK_D);
+  return align_up(c.used, 256) + empscore_bytes(n, variant, flags);
+}
+
+size_t fsk_sdshift16_workspace_bytes(int64_t n, int variant, int flags) {
+  if (n < 1) return 0;
+  return sdshift_bytes(n, variant, flags);
+}
+
+int fsk_sdshift16(const float* data, int64_t n, double bandwidth, int variant, int flags, double eps, float* debiased,
+                  float* pdf_sum, float* weighted_sum, float* score, void* workspace, size_t workspace_bytes,
+                  void* stream) {
+  NvtxRange nvtx_range("fsk_sdshift16");
+  if (!debiased || bad_empscore_args(data, n, bandwidth, variant, flags) || !(eps >= 0.0))
+    return FSK_ERR_INVALID_ARGUMENT;
+  int st = check_device();
+  if (st) return st;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!workspace || workspace_bytes < sdshift_bytes(n, variant, flags)) return FSK_ERR_WORKSPACE_TOO_SMALL;
+  const bool fm = (flags & FSK_WEIGHTED_FEATURE_MAJOR) != 0;
+  const int64_t ws_row = fm ? 1 : FSK_D, ws_col = fm ? n : 1;
+  WsCarver c(workspace, workspace_bytes);
+  if (score_on_tensor_cores(variant, flags)) {
+    tc::ScPartials parts{};
+    st = tc::launch_score16_tc(data, n, bandwidth, tc::plan_score16(n), c, &parts, s);
+    if (st) return st;
+    launch_reduce_score_tc(parts, n, data, ScoreOut{pdf_sum, weighted_sum, ws_row, ws_col, debiased, score}, bandwidth,
+                           eps, s);
+  } else {
+    float* pdf_ws = c.take<float>((size_t)n);
+    float* w_ws = c.take<float>((size_t)n * FSK_D);
+    float* pdf = pdf_sum ? pdf_sum : pdf_ws;
+    float* w = weighted_sum ? weighted_sum : w_ws;
+    run_empscore_simt(data, n, bandwidth, variant, pdf, w, ws_row, ws_col, c, s);
+    launch_debias16(data, n, pdf, w, ws_row, ws_col, bandwidth, eps, debiased, score, s);
   }
   return cuda_status(cudaGetLastError());
 }
@@ -275,18 +324,16 @@ int fsk_debias16(const float* data, int64_t n, const float* pdf_sum, const float
 }
 
 // ---- one-call SD-KDE: score -> debias -> KDE --------------------------------------
-// Workspace: pdf_sum (n) | weighted_sum (n, 16) | debiased (n, 16) unless the
-// caller takes it | the larger of the score and KDE workspaces (they run one
-// after the other on the stream and share it).
+// Workspace: debiased (n, 16) unless the caller takes it | the larger of the
+// shift and KDE workspaces (they run one after the other on the stream and
+// share it).
 static const int kSdkdeScoreFlags = FSK_PREC_IEEE;
 static const int kSdkdeKdeFlags = FSK_PREC_IEEE | FSK_OUT_LOG | FSK_OUT_LOG_EXACT | FSK_ATOMIC;
 
 static size_t sdkde_bytes(int64_t n, int64_t m, int flags) {
   WsCarver c(nullptr, 0);
-  c.take<float>((size_t)n);
   c.take<float>((size_t)n * FSK_D);
-  c.take<float>((size_t)n * FSK_D);
-  const size_t a = fsk_empscore16_workspace_bytes(n, FSK_SCORE_ORDERED, flags & kSdkdeScoreFlags);
+  const size_t a = fsk_sdshift16_workspace_bytes(n, FSK_SCORE_ORDERED, flags & kSdkdeScoreFlags);
   const size_t b = fsk_kde16_workspace_bytes(m, n, flags & kSdkdeKdeFlags);
   c.used = align_up(c.used, 256) + (a > b ? a : b);
   return align_up(c.used, 256);
@@ -310,17 +357,13 @@ int fsk_sdkde16(const float* data, int64_t n, const float* queries, int64_t m, d
   if (st) return st;
   if (!workspace || workspace_bytes < sdkde_bytes(n, m, flags)) return FSK_ERR_WORKSPACE_TOO_SMALL;
   WsCarver c(workspace, workspace_bytes);
-  float* pdf = c.take<float>((size_t)n);
-  float* w = c.take<float>((size_t)n * FSK_D);
   float* deb_ws = c.take<float>((size_t)n * FSK_D);
   float* deb = debiased ? debiased : deb_ws;
   c.used = align_up(c.used, 256);
   void* rest = static_cast<char*>(workspace) + c.used;
   const size_t rest_bytes = workspace_bytes - c.used;
-  st = fsk_empscore16(data, n, bandwidth, FSK_SCORE_ORDERED, flags & kSdkdeScoreFlags, pdf, w, rest, rest_bytes,
-                      stream);
-  if (st) return st;
-  st = fsk_debias16(data, n, pdf, w, FSK_D, 1, bandwidth, eps, deb, nullptr, stream);
+  st = fsk_sdshift16(data, n, bandwidth, FSK_SCORE_ORDERED, flags & kSdkdeScoreFlags, eps, deb, nullptr, nullptr,
+                     nullptr, rest, rest_bytes, stream);
   if (st) return st;
   return fsk_kde16(queries, m, deb, n, bandwidth, flags & kSdkdeKdeFlags, out_scale, out_eps, out, rest, rest_bytes,
                    stream);

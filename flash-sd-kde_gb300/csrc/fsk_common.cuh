@@ -103,6 +103,29 @@ class TimerScope {
   cudaStream_t s_;
 };
 
+// ---- programmatic dependent launch -------------------------------------------
+// A kernel launched with launch_pdl may start while the kernel before it in
+// the stream still runs; each of its threads calls pdl_wait() before it touches
+// global memory, which returns when that kernel has completed.  Every kernel
+// of such a chain waits, so completion is transitive.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 template <typename T> __host__ __device__ __forceinline__ T imin(T a, T b) { return a < b ? a : b; }

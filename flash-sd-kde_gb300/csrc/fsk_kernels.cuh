@@ -58,10 +58,18 @@ void launch_reduce_tc_rows(const tc::TcPartials& p, int64_t m, double scale, dou
 size_t reduce_score_scratch_doubles(int64_t n);
 void launch_reduce_score(const double* ppdf, const double* pw, int splits, int64_t n, const double* mu64, float* pdf,
                          float* w, int64_t ws_row, int64_t ws_col, double* scratch, cudaStream_t s);
-// The same from the tensor-core score's segment partials, which leave out the
-// self pair (added here exactly).
-void launch_reduce_score_tc(const tc::ScPartials& p, int64_t n, const float* mu, const float* x, float* pdf, float* w,
-                            int64_t ws_row, int64_t ws_col, cudaStream_t s);
+// Outputs of the score reduction; any pointer may be null (score needs debiased).
+struct ScoreOut {
+  float* pdf;                // (n)
+  float* w;                  // element (i, k) at w[i * ws_row + k * ws_col]
+  int64_t ws_row, ws_col;
+  float* debiased;           // (n, 16)
+  float* score;              // (n, 16)
+};
+// From the tensor-core score's segment partials, which leave out the self pair
+// (added here exactly), with the debias shift.
+void launch_reduce_score_tc(const tc::ScPartials& p, int64_t n, const float* x, const ScoreOut& o, double h, double eps,
+                            cudaStream_t s);
 void launch_debias16(const float* x, int64_t n, const float* pdf, const float* w, int64_t ws_row,
                      int64_t ws_col, double h, double eps, float* debiased, float* score,
                      cudaStream_t s);

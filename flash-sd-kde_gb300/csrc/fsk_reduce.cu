@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_tc_rows_kernel(tc::TcParti
                                                                      float* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * (RED_THREADS / RL) + threadIdx.x % (RED_THREADS / RL);
   double sum;
+  pdl_wait();
   if (!tc::reduce_tc_row<RL>(p, i, m, sum)) return;
   double v = sum * scale;
   if (log_out) v = log(v + eps);
@@ -132,27 +133,28 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_tc_rows_kernel(tc::TcParti
 void launch_reduce_tc_rows(const tc::TcPartials& p, int64_t m, double scale, double eps, bool log_out, float* out,
                            cudaStream_t s) {
   if (tc::tc_short_rows(p))
-    reduce_tc_rows_kernel<1><<<(unsigned)((m + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
-        p, m, scale, eps, log_out ? 1 : 0, out);
+    launch_pdl(reduce_tc_rows_kernel<1>, (int)((m + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s, p, m, scale,
+               eps, log_out ? 1 : 0, out);
   else
-    reduce_tc_rows_kernel<RED_LANES><<<(unsigned)((m + RED_THREADS / RED_LANES - 1) / (RED_THREADS / RED_LANES)),
-                                       RED_THREADS, 0, s>>>(p, m, scale, eps, log_out ? 1 : 0, out);
+    launch_pdl(reduce_tc_rows_kernel<RED_LANES>,
+               (int)((m + RED_THREADS / RED_LANES - 1) / (RED_THREADS / RED_LANES)), RED_THREADS, 0, s, p, m, scale,
+               eps, log_out ? 1 : 0, out);
   count_launch();
 }
 
-// Tensor-core score partials -> pdf_sum and weighted_sum, 16 threads per row
-// (thread k: feature k of every segment's centred weighted sum, and the pdf
-// pairs k, k + 16, ... of the row, added across the 16 threads by shuffles).
-// The self pair, which the partials leave out, is added exactly (phi = 1,
-// weight x_i), then mu * pdf undoes the centring.  Everything is carried as
-// double-float and rounded to FP32 once; in FP64 the pass was bound by the
-// FP64 unit (26 us at n = 65536 for 38 MB of traffic).
+// Tensor-core score partials -> any of pdf_sum, weighted_sum, the debiased
+// point and the score, 16 threads per row (thread k: feature k of every
+// segment's centred weighted sum, and the pdf pairs k, k + 16, ... of the row,
+// added across the 16 threads by shuffles).  The self pair, which the
+// partials leave out, is added exactly (phi = 1, weight x_i), then mu * pdf
+// undoes the centring; the shift is (x + W / (pdf + eps)) / 2.  Everything is
+// carried as double-float and rounded to FP32 once; in FP64 the reduction and
+// the shift were bound by the FP64 unit (26 + 18 us at n = 65536).
 __global__ void __launch_bounds__(RED_THREADS) reduce_score_tc_kernel(tc::ScPartials p, int64_t n,
-                                                                      const float* __restrict__ mu,
-                                                                      const float* __restrict__ x,
-                                                                      float* __restrict__ pdf, float* __restrict__ w,
-                                                                      int64_t ws_row, int64_t ws_col) {
+                                                                      const float* __restrict__ x, ScoreOut o,
+                                                                      float eps_hi, float eps_lo, double inv_h2) {
   constexpr int QB = 256;   // rows per query block
+  pdl_wait();
   const int64_t e = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
   const int64_t i = e / FSK_D;
   const int k = (int)(threadIdx.x % FSK_D);
@@ -165,8 +167,8 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_score_tc_kernel(tc::ScPart
   float2 ps = make_float2(0.f, 0.f);
   for (int j = k; j < 2 * segs; j += FSK_D) ps = df_add(ps, p.ppdf[(2 * seg0 + j) * QB + r]);
 #pragma unroll
-  for (int o = 1; o < FSK_D; o <<= 1)
-    ps = df_add(ps, make_float2(__shfl_xor_sync(group, ps.x, o), __shfl_xor_sync(group, ps.y, o)));
+  for (int d = 1; d < FSK_D; d <<= 1)
+    ps = df_add(ps, make_float2(__shfl_xor_sync(group, ps.x, d), __shfl_xor_sync(group, ps.y, d)));
   float2 ws = make_float2(0.f, 0.f);
   const float2* wp = p.pw + (seg0 * QB + r) * FSK_D + k;
 #pragma unroll 4
@@ -178,20 +180,36 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_score_tc_kernel(tc::ScPart
   ps.y *= phi_unscale;
   ws.x = ws.x * phi_unscale * w_unscale;
   ws.y = ws.y * phi_unscale * w_unscale;
-  // W + mu * p + x_i
-  const float m = mu[k];
-  float2 mp = two_prod(m, ps.x);
-  mp.y = fmaf(m, ps.y, mp.y);
-  const float2 wt = df_add(df_add(ws, mp), make_float2(x[e], 0.f));
-  const int64_t o = i * ws_row + k * ws_col;
-  if (in_bounds(o, n * FSK_D, 53)) w[o] = wt.x;
-  if (k == 0) pdf[i] = df_add(ps, make_float2(1.0f, 0.f)).x;
+  // pdf = p + 1, W + mu * p + x_i
+  const float mk = p.mu[k], xi = x[e];
+  float2 mp = two_prod(mk, ps.x);
+  mp.y = fmaf(mk, ps.y, mp.y);
+  const float2 wt = df_add(df_add(ws, mp), make_float2(xi, 0.f));
+  const float2 pdf = df_add(ps, make_float2(1.0f, 0.f));
+  if (o.w) {
+    const int64_t at = i * o.ws_row + k * o.ws_col;
+    if (in_bounds(at, n * FSK_D, 53)) o.w[at] = wt.x;
+  }
+  if (o.pdf && k == 0) o.pdf[i] = pdf.x;
+  if (o.debiased) {
+    // m = W / (pdf + eps) as a quotient and its remainder over the divisor (pdf >= 1)
+    const float2 d = df_add(pdf, make_float2(eps_hi, eps_lo));
+    const float q = wt.x / d.x;
+    const float rem = (fmaf(-q, d.x, wt.x) + wt.y) - q * d.y;
+    const float2 m = two_sum(q, rem / d.x);
+    o.debiased[e] = 0.5f * df_add(m, make_float2(xi, 0.f)).x;
+    if (o.score) {
+      const float2 df = df_add(m, make_float2(-xi, 0.f));
+      o.score[e] = (float)(((double)df.x + (double)df.y) * inv_h2);
+    }
+  }
 }
 
-void launch_reduce_score_tc(const tc::ScPartials& p, int64_t n, const float* mu, const float* x, float* pdf, float* w,
-                            int64_t ws_row, int64_t ws_col, cudaStream_t s) {
-  reduce_score_tc_kernel<<<(unsigned)((n * FSK_D + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
-      p, n, mu, x, pdf, w, ws_row, ws_col);
+void launch_reduce_score_tc(const tc::ScPartials& p, int64_t n, const float* x, const ScoreOut& o, double h, double eps,
+                            cudaStream_t s) {
+  const float eps_hi = (float)eps, eps_lo = (float)(eps - (double)eps_hi);
+  launch_pdl(reduce_score_tc_kernel, (int)((n * FSK_D + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s, p, n, x, o,
+             eps_hi, eps_lo, 1.0 / (h * h));
   count_launch();
 }
 

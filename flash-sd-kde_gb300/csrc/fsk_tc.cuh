@@ -66,9 +66,17 @@ static_assert(TMEM_COLS == 512, "TMEM budget");
 static_assert(KB_STAGE_BYTES % 16 == 0 && A_BYTES % 16 == 0, "bulk copy granularity");
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 
-// Device-side scale state written by the prep kernels (see fsk_tc_kde16.cu).
+// Score kernel data stage (64 points):
+// [H | M | L | XT hi (16 x 64 fp16) | XT lo | x (64 x 16 FP32)]
+constexpr int XT_ROW_BYTES = NT * 2;                       // one feature row over 64 points, fp16
+constexpr int XT_BYTES = FSK_D * XT_ROW_BYTES;             // 2 KB
+constexpr int S_XTH_OFFSET = B_L_OFFSET + B_L_BYTES;       // 8 KB
+constexpr int S_XTL_OFFSET = S_XTH_OFFSET + XT_BYTES;      // 10 KB
+constexpr int S_X_OFFSET = S_XTL_OFFSET + XT_BYTES;        // 12 KB: original FP32 rows
+constexpr int S_STAGE_BYTES = S_X_OFFSET + NT * FSK_D * 4; // 16 KB
+
+// Device-side scale state written by the prep kernels (see fsk_tc_prep.cu).
 struct TcScales {
-  unsigned int qmax_bits, xmax_bits, amax_bits, bmax_bits;  // maxima (FP32 bits, >= 0)
   float q_scale;   // q' = q_scale * (q - mu)       (= 2 c2 2^eq)
   float x_scale;   // x' = x_scale * (x - mu)       (= 2^ex)
   float a_scale;   // alpha part scale  2^-ea  (A bias col holds alpha*a_scale, B holds 1/a_scale)
@@ -171,17 +179,18 @@ struct TcPartials {
   int row_stride;
 };
 
-// Prep kernels shared by the tensor-core kernels (fsk_tc_kde16.cu).
-__global__ void scale_init_kernel(TcScales* sc);
-__global__ void scale_stats_kernel(const float* __restrict__ pts, int64_t count, const float* __restrict__ mu,
-                                   float c2, int is_query, float alpha_off, TcScales* __restrict__ sc);
-__global__ void scale_select_kernel(TcScales* sc);
-__global__ void prep_query_kernel(const float* __restrict__ q, int64_t m, int64_t m_pad,
-                                  const float* __restrict__ mu, float c2, float alpha_off,
-                                  const TcScales* __restrict__ sc, uint8_t* __restrict__ img,
-                                  float* __restrict__ qexact);
+// Operand preparation (fsk_tc_prep.cu): data mean, scale state and images.
+struct TcPrep {
+  const float* mu;
+  const TcScales* scales;
+};
+void take_tc_prep(WsCarver& c);   // its scratch in the workspace
+int launch_kde16_prep(const float* x, int64_t n, const float* q, int64_t m, double h, const TcPlan& pl, uint8_t* ximg,
+                      uint8_t* qimg, WsCarver& c, TcPrep* out, cudaStream_t s);
+int launch_score16_prep(const float* x, int64_t n, double h, const TcPlan& pl, uint8_t* ximg, uint8_t* qimg,
+                        float* qexact, WsCarver& c, TcPrep* out, cudaStream_t s);
 size_t tc_kde16_ws_bytes(const TcPlan& pl, int64_t m, bool atomic);
-int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, const float* mu, double h,
+int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, double h,
                     bool laplace, bool single, bool poly, const TcPlan& pl, WsCarver& c, TcPartials* partials_out,
                     double** atomic_out, cudaStream_t s);
 TcPlan plan_score16(int64_t n);
@@ -193,9 +202,10 @@ struct ScPartials {
   const float2* ppdf;
   const float2* pw;
   const TcScales* scales;
+  const float* mu;
   WorkLine line;
 };
-int launch_score16_tc(const float* x, int64_t n, const float* mu, double h, const TcPlan& pl, WsCarver& c,
+int launch_score16_tc(const float* x, int64_t n, double h, const TcPlan& pl, WsCarver& c,
                       ScPartials* out, cudaStream_t s);
 int launch_mma_probe(const float* a, const float* b, float* d, cudaStream_t s);
 int launch_mma_ts_probe(const float* a, const float* b, float* d, cudaStream_t s);

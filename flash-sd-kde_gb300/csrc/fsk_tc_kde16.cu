@@ -28,8 +28,8 @@
 //    for the query block), the chunk's largest term is recomputed from
 //    direct FP32 differences of the original coordinates (kept in the data
 //    stage) with the exponent product in double-float, and replaces its
-//    approximation.  The argmax rides in the low 5 mantissa bits, so all
-//    triggered lanes of a warp recompute one pair each in lock-step.  Other
+//    approximation; all triggered lanes of a warp recompute one pair each in
+//    lock-step.  Other
 //    terms carry the ~2^-25 relative error of the accumulation, which
 //    averages out.
 //
@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();   // the images and scales of the preparation
   if (warp == PRODUCER_WARP) {
     // the whole warp runs the loop (warp-uniform values stay in uniform
     // registers); lane 0 issues the copies
@@ -297,39 +298,20 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
             const bool trig = !SINGLE && fabsf(cs) > (run + fabsf(cs)) * NEAR_FRACTION;
             if (!SINGLE && __any_sync(0xffffffffu, trig)) {
               // Triggered lanes replace their chunk's largest term by its exact
-              // value.  The argmax rides in the low 5 mantissa bits of each term
-              // (key = |e| with bits[4:0] := column); the chunk is re-summed
-              // from those keyed values, so subtracting the keyed maximum
-              // removes exactly what was added.  All triggered lanes recompute
-              // one pair each, in lock-step.
+              // value, one pair each, in lock-step.  The term is found by
+              // value (its bits are what the sum holds, so subtracting it
+              // removes exactly what was added).
               if (trig) {
-                uint32_t key[32];
-                float2 qa = make_float2(0.f, 0.f), qc = make_float2(0.f, 0.f);
+                float mx = LAPLACE ? fabsf(e[0]) : e[0];   // terms are >= 0 except with the Laplace factor
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                  // terms are >= 0 except with the Laplace factor
-                  const float a0 = LAPLACE ? fabsf(e[j]) : e[j], a1 = LAPLACE ? fabsf(e[j + 1]) : e[j + 1];
-                  key[j] = (__float_as_uint(a0) & ~31u) | (uint32_t)j;
-                  key[j + 1] = (__float_as_uint(a1) & ~31u) | (uint32_t)(j + 1);
-                  const float v0 = LAPLACE ? copysignf(__uint_as_float(key[j]), e[j]) : __uint_as_float(key[j]);
-                  const float v1 = LAPLACE ? copysignf(__uint_as_float(key[j + 1]), e[j + 1]) : __uint_as_float(key[j + 1]);
-                  if (j & 2) qc = __fadd2_rn(qc, make_float2(v0, v1));
-                  else qa = __fadd2_rn(qa, make_float2(v0, v1));
-                }
-                // max tree over the keys
+                for (int jj = 1; jj < 32; ++jj) mx = fmaxf(mx, LAPLACE ? fabsf(e[jj]) : e[jj]);
+                int j = 0;
+                float approx = mx;
 #pragma unroll
-                for (int w = 16; w >= 1; w >>= 1)
-#pragma unroll
-                  for (int j = 0; j < w; ++j) key[j] = max(key[j], key[j + w]);
-                const uint32_t kmax = key[0];
-                qa = __fadd2_rn(qa, qc);
-                cs = qa.x + qa.y;
-                const int j = (int)(kmax & 31u);
-                float approx = __uint_as_float(kmax);
-                if (LAPLACE) {
-#pragma unroll
-                  for (int jj = 0; jj < 32; ++jj)
-                    if (jj == j) approx = copysignf(approx, e[jj]);
+                for (int jj = 0; jj < 32; ++jj) {
+                  const bool hit = (LAPLACE ? fabsf(e[jj]) : e[jj]) == mx;
+                  j = hit ? jj : j;
+                  if (LAPLACE) approx = hit ? e[jj] : approx;
                 }
                 float qx[FSK_D];
 #pragma unroll
@@ -369,6 +351,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
     }
   }
 done:
+  pdl_launch_dependents();
   // Exit path (also after a timed-out wait): let this CTA's bulk copies and
   // MMAs finish before shared and tensor memory are released.
   if (warp == PRODUCER_WARP && lane == 0) {
@@ -384,129 +367,6 @@ done:
   __syncthreads();
   tc_fence_after();
   if (warp == MMA_WARP) tmem_dealloc(tmem_base, TMEM_COLS);
-}
-
-// ---- prep ----------------------------------------------------------------------------
-// Maxima for the scale selection: |2 c2 (q-mu)|, c2 |q-mu|^2 over queries and
-// |x-mu|, c2 |x-mu|^2 over data.  One thread per row; block-reduced.
-__global__ void scale_stats_kernel(const float* __restrict__ pts, int64_t count, const float* __restrict__ mu,
-                                   float c2, int is_query, float alpha_off, TcScales* __restrict__ sc) {
-  float vmax = 0.f, nmax = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float nrm = 0.f, mx = 0.f;
-#pragma unroll
-    for (int k = 0; k < FSK_D; ++k) {
-      const float v = pts[i * FSK_D + k] - mu[k];
-      nrm = fmaf(v, v, nrm);
-      mx = fmaxf(mx, fabsf(v));
-    }
-    vmax = fmaxf(vmax, is_query ? 2.0f * c2 * mx : mx);
-    nmax = fmaxf(nmax, fabsf(c2 * nrm - (is_query ? alpha_off : 0.f)));
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, off));
-    nmax = fmaxf(nmax, __shfl_xor_sync(0xffffffffu, nmax, off));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomic_max_pos(is_query ? &sc->qmax_bits : &sc->xmax_bits, vmax);
-    atomic_max_pos(is_query ? &sc->amax_bits : &sc->bmax_bits, nmax);
-  }
-}
-
-__global__ void scale_init_kernel(TcScales* sc) {
-  if (threadIdx.x == 0) {
-    sc->qmax_bits = sc->xmax_bits = sc->amax_bits = sc->bmax_bits = 0u;
-  }
-}
-
-// Chooses the power-of-two scales (one thread).  q' max and x' max are
-// balanced around sqrt(Lq Lx 2^-es) <= FP16_TARGET; alpha and beta parts are
-// scaled into range against exact powers of two (<= 2^15) in the other
-// operand's bias columns.
-__global__ void scale_select_kernel(TcScales* sc) {
-  if (threadIdx.x != 0) return;
-  const float T = FP16_TARGET;
-  float lq = fmaxf(__uint_as_float(sc->qmax_bits), 1e-30f);
-  float lx = fmaxf(__uint_as_float(sc->xmax_bits), 1e-30f);
-  const float am = __uint_as_float(sc->amax_bits), bm = __uint_as_float(sc->bmax_bits);
-  int es = 0;
-  for (int it = 0; it < 64; ++it) {
-    const double prod = (double)lq * (double)lx * ldexp(1.0, -es);
-    const int eaa = am * ldexpf(1.f, -es) > T ? (int)ceil(log2((double)am * ldexp(1.0, -es) / T)) : 0;
-    const int ebb = bm * ldexpf(1.f, -es) > T ? (int)ceil(log2((double)bm * ldexp(1.0, -es) / T)) : 0;
-    if (prod <= (double)T * T && eaa <= 15 && ebb <= 15) break;
-    ++es;
-  }
-  // x' = (x-mu) 2^ex, q' = 2c2 (q-mu) 2^eq, eq + ex = -es, balanced
-  const int ex = (int)floor(0.5 * (log2((double)lq) - log2((double)lx) - es));
-  const int eq = -es - ex;
-  const int ea = am * ldexpf(1.f, -es) > T ? (int)ceil(log2((double)am * ldexp(1.0, -es) / T)) : 0;
-  const int eb = bm * ldexpf(1.f, -es) > T ? (int)ceil(log2((double)bm * ldexp(1.0, -es) / T)) : 0;
-  sc->x_scale = ldexpf(1.f, ex);
-  sc->q_scale = ldexpf(1.f, eq);          // times 2 c2, applied in the prep kernel
-  sc->a_scale = ldexpf(1.f, -es - ea);    // alpha * a_scale in A, 2^ea in B
-  sc->b_scale = ldexpf(1.f, -es - eb);    // beta * b_scale in B, 2^eb in A
-  sc->pad[0] = ea;
-  sc->pad[1] = eb;
-  // scale of the (x - mu) operand of the weighted-sum product: max |x'| <= T
-  sc->pad[2] = (int)floor(log2((double)T / (double)lx));
-  sc->out_mul = ldexpf(1.f, es);
-}
-
-// data tile image: [H (128 x 32 fp16) | M (128 x 16 fp16) | L (128 x 16 fp16) | x (128 x 16 FP32)]
-__global__ void prep_data_kernel(const float* __restrict__ x, int64_t n, int64_t n_pad,
-                                 const float* __restrict__ mu, float c2, const TcScales* __restrict__ sc,
-                                 uint8_t* __restrict__ img) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n_pad) return;
-  const bool ok = j < n;
-  float xo[FSK_D], v[FSK_D];
-  float nrm = 0.f;
-#pragma unroll
-  for (int k = 0; k < FSK_D; ++k) {
-    xo[k] = ok ? x[j * FSK_D + k] : 0.f;
-    const float cv = xo[k] - mu[k];
-    nrm = fmaf(cv, cv, nrm);
-    v[k] = ok ? cv * sc->x_scale : 0.f;
-  }
-  uint8_t* tile = img + (j / KNT) * (int64_t)KB_STAGE_BYTES;
-  const int r = (int)(j % KNT);
-  const float beta = ok ? -c2 * nrm * sc->b_scale : 0.f;
-  write_operand_row(tile, tile + KB_M_OFFSET, tile + KB_L_OFFSET, r, v, beta, ok ? ldexpf(1.f, sc->pad[0]) : 0.f,
-                    true);
-  float4* xr = reinterpret_cast<float4*>(tile + KB_X_OFFSET + r * (FSK_D * 4));
-#pragma unroll
-  for (int k = 0; k < 4; ++k) xr[k] = make_float4(xo[4 * k], xo[4 * k + 1], xo[4 * k + 2], xo[4 * k + 3]);
-}
-
-// query tile image: [H (QT x 32 fp16) | M | L (QT x 16 fp16)], plus (score
-// kernel) the original coordinates, padded to whole query blocks.
-__global__ void prep_query_kernel(const float* __restrict__ q, int64_t m, int64_t m_pad,
-                                  const float* __restrict__ mu, float c2, float alpha_off,
-                                  const TcScales* __restrict__ sc, uint8_t* __restrict__ img,
-                                  float* __restrict__ qexact) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m_pad) return;
-  const bool ok = i < m;
-  float qo[FSK_D], v[FSK_D];
-  float nrm = 0.f;
-  const float qs = 2.0f * c2 * sc->q_scale;
-#pragma unroll
-  for (int k = 0; k < FSK_D; ++k) {
-    qo[k] = ok ? q[i * FSK_D + k] : 0.f;
-    const float cv = qo[k] - mu[k];
-    nrm = fmaf(cv, cv, nrm);
-    v[k] = ok ? cv * qs : 0.f;
-  }
-  uint8_t* tile = img + (i / QT) * (int64_t)A_TILE_BYTES;
-  const float alpha = ok ? (alpha_off - c2 * nrm) * sc->a_scale : 0.f;
-  write_operand_row(tile, tile + A_M_OFFSET, tile + A_L_OFFSET, (int)(i % QT), v, alpha,
-                    ok ? ldexpf(1.f, sc->pad[1]) : 0.f, false);
-  if (qexact == nullptr) return;
-#pragma unroll
-  for (int k = 0; k < FSK_D; ++k) qexact[i * FSK_D + k] = qo[k];
 }
 
 void plan_line(TcPlan& pl) {
@@ -530,12 +390,13 @@ TcPlan plan_kde16(int64_t m, int64_t n) {
 static int kde16_row_stride(int64_t m) { return (int)imin<int64_t>(m, NQT * QT); }
 
 size_t tc_kde16_ws_bytes(const TcPlan& pl, int64_t m, bool atomic) {
-  size_t b = 0;
-  b += align_up(sizeof(TcScales), 256);
-  b += align_up((size_t)pl.q_blocks * A_BYTES, 256);
-  b += align_up((size_t)pl.n_tiles * KB_STAGE_BYTES, 256);
-  b += align_up(atomic ? (size_t)m * sizeof(double) : (size_t)pl.line.segment_bound() * 2 * kde16_row_stride(m) * sizeof(float2), 256);
-  return b;
+  WsCarver c(nullptr, 0);
+  c.take<uint8_t>((size_t)pl.q_blocks * A_BYTES);
+  c.take<uint8_t>((size_t)pl.n_tiles * KB_STAGE_BYTES);
+  if (atomic) c.take<double>((size_t)m);
+  else c.take<float2>((size_t)pl.line.segment_bound() * 2 * kde16_row_stride(m));
+  take_tc_prep(c);
+  return align_up(c.used, 256);
 }
 
 template <bool LAPLACE, bool SINGLE, bool POLY = false>
@@ -543,14 +404,12 @@ static cudaError_t launch_kde16_tc_kernel(const TcPlan& pl, const TcParams& p, c
   const cudaError_t e = cudaFuncSetAttribute(kde16_tc_kernel<LAPLACE, SINGLE, POLY>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return e;
-  kde16_tc_kernel<LAPLACE, SINGLE, POLY><<<pl.line.grid, THREADS, SMEM_BYTES, s>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(kde16_tc_kernel<LAPLACE, SINGLE, POLY>, pl.line.grid, THREADS, SMEM_BYTES, s, p);
 }
 
-int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, const float* mu, double h,
+int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, double h,
                     bool laplace, bool single, bool poly, const TcPlan& pl, WsCarver& c, TcPartials* partials_out,
                     double** atomic_out, cudaStream_t s) {
-  TcScales* sc = c.take<TcScales>(1);
   uint8_t* qimg = c.take<uint8_t>((size_t)pl.q_blocks * A_BYTES);
   uint8_t* ximg = c.take<uint8_t>((size_t)pl.n_tiles * KB_STAGE_BYTES);
   const bool atomic = atomic_out != nullptr;
@@ -561,31 +420,19 @@ int launch_kde16_tc(const float* q, int64_t m, const float* x, int64_t n, const 
   if (atomic) *atomic_out = acc;
   *partials_out = TcPartials{part, pl.line, row_stride};
 
+  TcPrep prep;
+  const int st = launch_kde16_prep(x, n, q, m, h, pl, ximg, qimg, c, &prep, s);
+  if (st) return st;
   const double c2d = FSK_LOG2E / (2.0 * h * h);
   const float c2 = (float)c2d;
   const float c2_lo = (float)(c2d - (double)c2);
-  scale_init_kernel<<<1, 32, 0, s>>>(sc);
-  count_launch();
-  const int sblocks_q = (int)imin<int64_t>(1024, (m + 255) / 256);
-  const int sblocks_x = (int)imin<int64_t>(1024, (n + 255) / 256);
-  scale_stats_kernel<<<sblocks_q, 256, 0, s>>>(q, m, mu, c2, 1, 0.f, sc);
-  count_launch();
-  scale_stats_kernel<<<sblocks_x, 256, 0, s>>>(x, n, mu, c2, 0, 0.f, sc);
-  count_launch();
-  scale_select_kernel<<<1, 32, 0, s>>>(sc);
-  count_launch();
-  prep_data_kernel<<<(unsigned)((pl.n_pad + 255) / 256), 256, 0, s>>>(x, n, pl.n_pad, mu, c2, sc, ximg);
-  count_launch();
-  prep_query_kernel<<<(unsigned)((pl.m_pad + 255) / 256), 256, 0, s>>>(q, m, pl.m_pad, mu, c2, 0.f, sc, qimg,
-                                                                        nullptr);
-  count_launch();
   if (atomic) launch_zero(acc, m, s);
 
   TcParams p;
   p.qimg = qimg;
   p.ximg = ximg;
   p.q = q;
-  p.scales = sc;
+  p.scales = prep.scales;
   p.m = m;
   p.n = n;
   p.line = pl.line;

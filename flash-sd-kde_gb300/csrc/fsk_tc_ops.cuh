@@ -60,10 +60,6 @@ __device__ __forceinline__ float exact_dist(const uint8_t* stage, int r, const f
   return sqdist16(q, xv);
 }
 
-__device__ __forceinline__ void atomic_max_pos(unsigned int* addr, float v) {
-  atomicMax(addr, __float_as_uint(fmaxf(v, 0.f)));  // non-negative floats order as integers
-}
-
 // Splits v into three fp16 parts (hi, mid, lo) that sum to v to ~33 bits.
 __device__ __forceinline__ void split3_f16(float v, __half& a, __half& b, __half& c) {
   a = __float2half_rn(v);

@@ -59,12 +59,6 @@ namespace {
 
 constexpr int SNQT = 2;                                    // query tiles per unit (256 queries)
 constexpr int SNS = 4;                                     // data stages
-constexpr int XT_ROW_BYTES = NT * 2;                       // one feature row over 64 points, fp16
-constexpr int XT_BYTES = FSK_D * XT_ROW_BYTES;             // 2 KB
-constexpr int S_XTH_OFFSET = B_L_OFFSET + B_L_BYTES;       // 8 KB
-constexpr int S_XTL_OFFSET = S_XTH_OFFSET + XT_BYTES;      // 10 KB
-constexpr int S_X_OFFSET = S_XTL_OFFSET + XT_BYTES;        // 12 KB: original FP32 rows
-constexpr int S_STAGE_BYTES = S_X_OFFSET + NT * FSK_D * 4; // 16 KB
 constexpr int S_A_BYTES = SNQT * A_TILE_BYTES;             // 32 KB
 constexpr int S_EPI_WARPS = 8 * SNQT;
 constexpr int S_PRODUCER_WARP = S_EPI_WARPS;
@@ -189,6 +183,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
     tmem_alloc(tmem_slot, S_TMEM_COLS);
     tmem_relinquish();
   }
+  pdl_wait();   // the images, mean and scales of the preparation
   if (threadIdx.x < FSK_D) sMu[threadIdx.x] = p.mu[threadIdx.x];
   tc_fence_before();
   __syncthreads();
@@ -594,6 +589,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
     }
   }
 done:
+  pdl_launch_dependents();
   // Exit path (also after a timed-out wait): let this CTA's bulk copies and
   // MMAs finish before shared and tensor memory are released.
   if (warp == S_PRODUCER_WARP && lane == 0) {
@@ -611,39 +607,6 @@ done:
   if (warp == S_MMA_WARP) tmem_dealloc(tmem_base, S_TMEM_COLS);
 }
 
-// Data stage image: [H (64 x 32 fp16) | M (64 x 16 fp16) | L (64 x 16 fp16)
-// | XT hi (16 x 64 fp16) | XT lo | x (64 x 16 FP32)].  XT rows are features, K-major over the points.
-__global__ void prep_score_data_kernel(const float* __restrict__ x, int64_t n, int64_t n_pad,
-                                       const float* __restrict__ mu, float c2,
-                                       const TcScales* __restrict__ sc, uint8_t* __restrict__ img) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n_pad) return;
-  const bool ok = j < n;
-  float xo[FSK_D], v[FSK_D];
-  float nrm = 0.f;
-  const float ws = ldexpf(1.f, sc->pad[2]);
-  uint8_t* tile = img + (j / NT) * (int64_t)S_STAGE_BYTES;
-  const int r = (int)(j % NT);
-#pragma unroll
-  for (int k = 0; k < FSK_D; ++k) {
-    xo[k] = ok ? x[j * FSK_D + k] : 0.f;
-    const float cv = xo[k] - mu[k];
-    nrm = fmaf(cv, cv, nrm);
-    v[k] = ok ? cv * sc->x_scale : 0.f;
-    const float w = ok ? cv * ws : 0.f;
-    const __half wh = __float2half_rn(w);
-    const __half wl = __float2half_rn(w - __half2float(wh));
-    put_h(tile + S_XTH_OFFSET, k, r, XT_ROW_BYTES, wh);
-    put_h(tile + S_XTL_OFFSET, k, r, XT_ROW_BYTES, wl);
-  }
-  const float beta = ok ? -c2 * nrm * sc->b_scale : 0.f;
-  write_operand_row(tile, tile + B_M_OFFSET, tile + B_L_OFFSET, r, v, beta, ok ? ldexpf(1.f, sc->pad[0]) : 0.f,
-                    true);
-  float4* xr = reinterpret_cast<float4*>(tile + S_X_OFFSET + r * (FSK_D * 4));
-#pragma unroll
-  for (int k = 0; k < 4; ++k) xr[k] = make_float4(xo[4 * k], xo[4 * k + 1], xo[4 * k + 2], xo[4 * k + 3]);
-}
-
 }  // namespace
 
 TcPlan plan_score16(int64_t n) {
@@ -657,51 +620,38 @@ TcPlan plan_score16(int64_t n) {
 }
 
 size_t tc_score16_ws_bytes(const TcPlan& pl) {
-  size_t b = 0;
-  b += align_up(sizeof(TcScales), 256);
-  b += align_up((size_t)pl.q_blocks * S_A_BYTES, 256);
-  b += align_up((size_t)pl.m_pad * FSK_D * sizeof(float), 256);
-  b += align_up((size_t)pl.n_tiles * S_STAGE_BYTES, 256);
-  b += align_up((size_t)pl.line.segment_bound() * 2 * SNQT * QT * sizeof(float2), 256);
-  b += align_up((size_t)pl.line.segment_bound() * SNQT * QT * FSK_D * sizeof(float2), 256);
-  return b;
+  WsCarver c(nullptr, 0);
+  c.take<uint8_t>((size_t)pl.q_blocks * S_A_BYTES);
+  c.take<float>((size_t)pl.m_pad * FSK_D);
+  c.take<uint8_t>((size_t)pl.n_tiles * S_STAGE_BYTES);
+  c.take<float2>((size_t)pl.line.segment_bound() * 2 * SNQT * QT);
+  c.take<float2>((size_t)pl.line.segment_bound() * SNQT * QT * FSK_D);
+  take_tc_prep(c);
+  return align_up(c.used, 256);
 }
 
-int launch_score16_tc(const float* x, int64_t n, const float* mu, double h, const TcPlan& pl, WsCarver& c,
+int launch_score16_tc(const float* x, int64_t n, double h, const TcPlan& pl, WsCarver& c,
                       ScPartials* out, cudaStream_t s) {
-  TcScales* sc = c.take<TcScales>(1);
   uint8_t* qimg = c.take<uint8_t>((size_t)pl.q_blocks * S_A_BYTES);
   float* qexact = c.take<float>((size_t)pl.m_pad * FSK_D);
   uint8_t* ximg = c.take<uint8_t>((size_t)pl.n_tiles * S_STAGE_BYTES);
   float2* ppdf = c.take<float2>((size_t)pl.line.segment_bound() * 2 * SNQT * QT);
   float2* pw = c.take<float2>((size_t)pl.line.segment_bound() * SNQT * QT * FSK_D);
   if (!c.fits()) return FSK_ERR_WORKSPACE_TOO_SMALL;
-  *out = ScPartials{ppdf, pw, sc, pl.line};
-
+  TcPrep prep;
+  const int st = launch_score16_prep(x, n, h, pl, ximg, qimg, qexact, c, &prep, s);
+  if (st) return st;
+  *out = ScPartials{ppdf, pw, prep.scales, prep.mu, pl.line};
   const double c2d = FSK_LOG2E / (2.0 * h * h);
   const float c2 = (float)c2d;
   const float c2_lo = (float)(c2d - (double)c2);
-  scale_init_kernel<<<1, 32, 0, s>>>(sc);
-  count_launch();
-  const int sblocks = (int)imin<int64_t>(1024, (n + 255) / 256);
-  scale_stats_kernel<<<sblocks, 256, 0, s>>>(x, n, mu, c2, 1, PHI_LOG2_SCALE, sc);
-  count_launch();
-  scale_stats_kernel<<<sblocks, 256, 0, s>>>(x, n, mu, c2, 0, 0.f, sc);
-  count_launch();
-  scale_select_kernel<<<1, 32, 0, s>>>(sc);
-  count_launch();
-  prep_score_data_kernel<<<(unsigned)((pl.n_pad + 255) / 256), 256, 0, s>>>(x, n, pl.n_pad, mu, c2, sc, ximg);
-  count_launch();
-  prep_query_kernel<<<(unsigned)((pl.m_pad + 255) / 256), 256, 0, s>>>(x, n, pl.m_pad, mu, c2, PHI_LOG2_SCALE,
-                                                                        sc, qimg, qexact);
-  count_launch();
 
   ScParams p;
   p.qimg = qimg;
   p.ximg = ximg;
   p.qexact = qexact;
-  p.scales = sc;
-  p.mu = mu;
+  p.scales = prep.scales;
+  p.mu = prep.mu;
   p.n = n;
   p.line = pl.line;
   p.c2 = c2;
@@ -712,9 +662,9 @@ int launch_score16_tc(const float* x, int64_t n, const float* mu, double h, cons
                                        S_SMEM_BYTES);
   if (e != cudaSuccess) return cuda_status(e);
   TimerScope ts(K_SCORE16_TC, (double)n * (double)n, s);
-  score16_tc_kernel<<<pl.line.grid, S_THREADS, S_SMEM_BYTES, s>>>(p);
+  const cudaError_t le = launch_pdl(score16_tc_kernel, pl.line.grid, S_THREADS, S_SMEM_BYTES, s, p);
   count_launch();
-  return cuda_status(cudaGetLastError());
+  return cuda_status(le);
 }
 
 // ---- layout probe: D (128 x 16) = A (128 x 64) . B (16 x 64)^T, fp16 ------------

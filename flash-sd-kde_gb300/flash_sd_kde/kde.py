@@ -33,7 +33,6 @@ from globals import (
     DEFAULT_KDE_BACKEND,
     DEFAULT_PRECISION_MODE,
     EMP_SCORE_BACKEND_FLASH_SD_KDE,
-    EMP_SCORE_BACKEND_ORDERED_SPLITK,
     EMP_SCORE_BACKEND_SYMMETRIC_ATOMIC,
     KDE_BACKEND_ATOMIC,
     KDE_BACKEND_SPLITK_STREAM,
@@ -229,19 +228,15 @@ def emp_sd_kde_fit_transform(
     if train.shape[0] == 0:
         raise ValueError("data must be non-empty.")
     prec = "ieee" if precision_mode == PRECISION_FP32_IEEE else "tensor"
-    if emp_score_backend == EMP_SCORE_BACKEND_SYMMETRIC_ATOMIC:
-        pdf_sum, weighted_sum = ops.empscore16(train, bandwidth, variant="symmetric", precision=prec)
-    else:
-        pdf_sum, weighted_sum = ops.empscore16(
-            train, bandwidth, variant="ordered", precision=prec,
-            feature_major=emp_score_backend == EMP_SCORE_BACKEND_FLASH_SD_KDE)
+    symmetric = emp_score_backend == EMP_SCORE_BACKEND_SYMMETRIC_ATOMIC
+    out = ops.sdshift16(train, bandwidth, eps, variant="symmetric" if symmetric else "ordered", precision=prec,
+                        feature_major=emp_score_backend == EMP_SCORE_BACKEND_FLASH_SD_KDE, return_debug=return_debug)
     if return_debug:
-        debiased, score = ops.debias16(train, pdf_sum, weighted_sum, bandwidth, eps, return_score=True)
+        debiased, pdf_sum, weighted_sum, score = out
         if d < ND_FEATURES:   # the padded columns are 0 in every output
             return debiased[:, :d].contiguous(), pdf_sum, weighted_sum[:, :d], score[:, :d].contiguous()
         return debiased, pdf_sum, weighted_sum, score
-    debiased = ops.debias16(train, pdf_sum, weighted_sum, bandwidth, eps)
-    return debiased[:, :d].contiguous() if d < ND_FEATURES else debiased
+    return out[:, :d].contiguous() if d < ND_FEATURES else out
 
 
 def sd_kde_eval(

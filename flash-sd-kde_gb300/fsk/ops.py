@@ -174,6 +174,42 @@ def empscore16(
     return pdf, (w.t() if feature_major else w)
 
 
+def sdshift16(
+    data: torch.Tensor,
+    bandwidth: float,
+    eps: float,
+    *,
+    variant: str = "ordered",
+    feature_major: bool = False,
+    precision: str = "tensor",
+    return_debug: bool = False,
+):
+    """The debiased points (n, 16) in one library call (fsk_sdshift16); with
+    return_debug also pdf_sum, weighted_sum (as empscore16) and the score."""
+    h = _check_bw(bandwidth)
+    dev = _device(data.device)
+    x = as_matrix(data, dev)
+    n = x.shape[0]
+    if n == 0:
+        raise ValueError("data must contain at least one element.")
+    var = L.FSK_SCORE_SYMMETRIC if variant == "symmetric" else L.FSK_SCORE_ORDERED
+    flags = L.FSK_WEIGHTED_FEATURE_MAJOR if feature_major else 0
+    flags |= L.FSK_PREC_IEEE if precision == "ieee" else L.FSK_PREC_TENSOR
+    lib = L.load()
+    pdf = w = score = None
+    with torch.cuda.device(dev):
+        deb = torch.empty_like(x)
+        if return_debug:
+            pdf = torch.empty(n, dtype=torch.float32, device=dev)
+            w = torch.empty((ND_FEATURES, n) if feature_major else (n, ND_FEATURES), dtype=torch.float32, device=dev)
+            score = torch.empty_like(x)
+        ws = _workspace(lib.fsk_sdshift16_workspace_bytes(n, var, flags), dev)
+        st = lib.fsk_sdshift16(x.data_ptr(), n, h, var, flags, float(eps), deb.data_ptr(), _ptr(pdf), _ptr(w),
+                               _ptr(score), ws.data_ptr(), ws.numel(), _stream(dev))
+    L.check(st, "fsk_sdshift16")
+    return (deb, pdf, w.t() if feature_major else w, score) if return_debug else deb
+
+
 def sdkde16(
     data: torch.Tensor,
     queries: torch.Tensor,

@@ -64,8 +64,7 @@ def empirical_sd_kde_triton_nd(
     train = _to_matrix_tensor(data, dev, dim=_ND_FEATURES)
     if train.shape[0] == 0:
         raise ValueError("data must contain at least one element.")
-    pdf, w = ops.empscore16(train, bandwidth, variant="ordered", feature_major=True)
-    debiased = ops.debias16(train, pdf, w, bandwidth, _EPS)
+    debiased = ops.sdshift16(train, bandwidth, _EPS)
     _finish(dev, synchronize)
     if return_tensor:
         return debiased, bandwidth

@@ -170,6 +170,16 @@ FSK_API int fsk_empscore16(const float* data, int64_t n, double bandwidth, int v
                    int flags, float* pdf_sum, float* weighted_sum,
                    void* workspace, size_t workspace_bytes, void* stream);
 
+/* Score and one-step debias shift in one call (flash_sd_kde/kde.py:258-326):
+ * debiased = x + h^2/2 * (W / (pdf_sum + eps) - x) / h^2, without the FP32
+ * rounding of the accumulators in between.  variant, flags and the layout of
+ * weighted_sum as fsk_empscore16; pdf_sum, weighted_sum and score (n, 16) may
+ * be NULL. */
+FSK_API size_t fsk_sdshift16_workspace_bytes(int64_t n, int variant, int flags);
+FSK_API int fsk_sdshift16(const float* data, int64_t n, double bandwidth, int variant, int flags, double eps,
+                          float* debiased, float* pdf_sum, float* weighted_sum, float* score, void* workspace,
+                          size_t workspace_bytes, void* stream);
+
 /* ---- SD-KDE in one call: score -> debias -> KDE ----------------------- */
 /* The pipeline the reference runs as empirical_sd_kde_triton_nd followed by
  * gaussian_kde_triton_nd (experiments/runtime/benchmark_triton_kde.py:344-388,
