@@ -133,7 +133,8 @@ int fsk_device_status(void* stream) {
     if (v != 0u) return (int)(v & 0xFFu);
 #ifdef FSK_BOUNDS_CHECK
   // units whose only device errors are the bounds checks
-  const unsigned int checked[3] = {simt_take_device_error(), reduce_take_device_error(), logspace_take_device_error()};
+  const unsigned int checked[4] = {simt_take_device_error(), reduce_take_device_error(), logspace_take_device_error(),
+                                   cell1d_take_device_error()};
   for (unsigned int v : checked)
     if (v != 0u) return (int)(v & 0xFFu);
 #endif
@@ -184,7 +185,7 @@ int fsk_kde16(const float* queries, int64_t m, const float* data, int64_t n, dou
   } else if (segments) {
     launch_reduce_tc_rows(tcp, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, s);
   } else {
-    launch_reduce_rows(part, splits, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, s);
+    launch_reduce_rows(part, splits, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, nullptr, s);
   }
   return cuda_status(cudaGetLastError());
 }
@@ -389,7 +390,7 @@ int fsk_kde_nd(const float* queries, int64_t m, const float* data, int64_t n, in
   const int splits = kde_nd_splits(m, n, d);
   double* part = static_cast<double*>(workspace);
   launch_kde_nd(queries, m, data, n, d, bandwidth, (flags & FSK_LAPLACE) != 0, splits, part, s);
-  launch_reduce_rows(part, splits, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, s);
+  launch_reduce_rows(part, splits, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, nullptr, s);
   return cuda_status(cudaGetLastError());
 }
 
@@ -445,7 +446,10 @@ size_t fsk_kde1d_workspace_bytes(int64_t m, int64_t n, int flags) {
   if (m < 1 || n < 1) return 0;
   const int splits = (flags & FSK_ATOMIC) ? 1 : kde1d_splits(m, n);
   // the score variant needs two partial arrays
-  return align_up((size_t)2 * splits * m * sizeof(double), 256);
+  WsCarver c(nullptr, 0);
+  c.take<double>((size_t)2 * splits * m);
+  if (cell1d_applies(m, n)) take_cell1d(c);
+  return align_up(c.used, 256);
 }
 
 int fsk_kde1d(const float* queries, int64_t m, const float* data, int64_t n, double bandwidth, int flags,
@@ -460,11 +464,21 @@ int fsk_kde1d(const float* queries, int64_t m, const float* data, int64_t n, dou
   if (!workspace || workspace_bytes < fsk_kde1d_workspace_bytes(m, n, flags)) return FSK_ERR_WORKSPACE_TOO_SMALL;
   const bool atomic = (flags & FSK_ATOMIC) != 0;
   const int splits = kde1d_splits(m, n);
-  double* part = static_cast<double*>(workspace);
+  const bool laplace = (flags & FSK_LAPLACE) != 0, log_out = (flags & FSK_OUT_LOG) != 0;
+  WsCarver c(workspace, workspace_bytes);
+  double* part = c.take<double>((size_t)2 * (atomic ? 1 : splits) * m);
+  // Cell expansions where they apply (plain densities; the Laplace factor's
+  // sums cancel and stay with the pair kernel); their flag tells the pair
+  // kernel on the device whether it is still needed.
+  const int* skip = nullptr;
+  if (!laplace && cell1d_applies(m, n)) {
+    st = launch_cell1d(queries, m, data, n, bandwidth, out_scale, out_eps, log_out, c, out, &skip, s);
+    if (st) return st;
+  }
   if (atomic) launch_zero(part, m, s);
-  launch_kde1d(queries, m, data, n, bandwidth, (flags & FSK_LAPLACE) != 0, splits, atomic ? nullptr : part,
-               atomic ? part : nullptr, s);
-  launch_reduce_rows(part, atomic ? 1 : splits, m, out_scale, out_eps, (flags & FSK_OUT_LOG) != 0, out, s);
+  launch_kde1d(queries, m, data, n, bandwidth, laplace, splits, atomic ? nullptr : part, atomic ? part : nullptr, skip,
+               s);
+  launch_reduce_rows(part, atomic ? 1 : splits, m, out_scale, out_eps, log_out, out, skip, s);
   return cuda_status(cudaGetLastError());
 }
 

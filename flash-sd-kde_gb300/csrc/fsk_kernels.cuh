@@ -34,10 +34,21 @@ void launch_score16_sym_simt(const float* x, int64_t n, const float* mu, double 
                              double* acc_w, cudaStream_t s);
 int64_t sym_simt_pairs(int64_t n);
 int kde1d_splits(int64_t m, int64_t n);
+// skip: device flag (or null); the kernel returns at once where it is not 0.
 void launch_kde1d(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace,
-                  int splits, double* partials, double* atomic_acc, cudaStream_t s);
+                  int splits, double* partials, double* atomic_acc, const int* skip, cudaStream_t s);
 void launch_kde1d_score(const float* q, int64_t m, const float* x, int64_t n, double h, int splits,
                         double* p0, double* p1, cudaStream_t s);
+
+// ---- fsk_cell1d.cu ------------------------------------------------------------
+// 1-D KDE by cell expansions for many points at many queries.  *taken: device
+// flag, 0 when the data is too spread for them and the direct kernels (given
+// the flag) have to run.
+bool cell1d_applies(int64_t m, int64_t n);
+void take_cell1d(WsCarver& c);
+int launch_cell1d(const float* q, int64_t m, const float* x, int64_t n, double h, double scale, double eps,
+                  bool log_out, WsCarver& c, float* out, const int** taken, cudaStream_t s);
+unsigned int cell1d_take_device_error();   // bounds checks only
 
 // ---- fsk_reduce.cu ------------------------------------------------------------
 // Column means of an (n, 16) FP32 matrix in FP64, deterministic; writes mu
@@ -46,8 +57,9 @@ size_t mean_scratch_doubles(int64_t n);
 void launch_mean16(const float* x, int64_t n, double* scratch, float* mu, double* mu64,
                    cudaStream_t s);
 // out[i] = g(scale * sum_s partials[s*m + i]), g = identity or log(. + eps).
+// skip: as launch_kde1d.
 void launch_reduce_rows(const double* partials, int splits, int64_t m, double scale, double eps,
-                        bool log_out, float* out, cudaStream_t s);
+                        bool log_out, float* out, const int* skip, cudaStream_t s);
 // The same over the tensor-core KDE's segment partials.
 void launch_reduce_tc_rows(const tc::TcPartials& p, int64_t m, double scale, double eps, bool log_out, float* out,
                            cudaStream_t s);

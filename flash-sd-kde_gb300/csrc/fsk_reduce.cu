@@ -82,7 +82,9 @@ constexpr int RED_LANES = 8;
 template <int RL>
 __global__ void __launch_bounds__(RED_THREADS) reduce_rows_kernel(const double* __restrict__ partials, int splits,
                                                                   int64_t m, double scale, double eps, int log_out,
-                                                                  float* __restrict__ out) {
+                                                                  float* __restrict__ out,
+                                                                  const int* __restrict__ skip) {
+  if (skip != nullptr && *skip != 0) return;
   constexpr int ROWS = RED_THREADS / RL;
   const int r = threadIdx.x % ROWS, l = threadIdx.x / ROWS;
   const int64_t i = (int64_t)blockIdx.x * ROWS + r;
@@ -106,14 +108,14 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_rows_kernel(const double* 
 }
 
 void launch_reduce_rows(const double* partials, int splits, int64_t m, double scale, double eps,
-                        bool log_out, float* out, cudaStream_t s) {
+                        bool log_out, float* out, const int* skip, cudaStream_t s) {
   // one thread per row while the chain is short
   if (splits <= 4)
     reduce_rows_kernel<1><<<(unsigned)((m + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
-        partials, splits, m, scale, eps, log_out ? 1 : 0, out);
+        partials, splits, m, scale, eps, log_out ? 1 : 0, out, skip);
   else
     reduce_rows_kernel<RED_LANES><<<(unsigned)((m + RED_THREADS / RED_LANES - 1) / (RED_THREADS / RED_LANES)),
-                                    RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out);
+                                    RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out, skip);
   count_launch();
 }
 

@@ -461,7 +461,9 @@ __device__ __forceinline__ void for_points(const float* xs, int r0, int rend, F&
 template <bool LAPLACE>
 __global__ void __launch_bounds__(K1_THREADS) kde1d_kernel(
     const float* __restrict__ q, int64_t m, const float* __restrict__ x, int64_t n, float nc2,
-    float c1, int64_t tiles_per_split, double* __restrict__ partials, double* __restrict__ atomic_acc) {
+    float c1, int64_t tiles_per_split, double* __restrict__ partials, double* __restrict__ atomic_acc,
+    const int* __restrict__ skip) {
+  if (skip != nullptr && *skip != 0) return;
   __shared__ __align__(16) float xs[K1_T];
   const int64_t q0 = (int64_t)blockIdx.x * (K1_THREADS * K1_Q);
   float2 nq[K1_P];   // -q of queries (2p, 2p + 1)
@@ -531,7 +533,7 @@ int kde1d_splits(int64_t m, int64_t n) {
 }
 
 void launch_kde1d(const float* q, int64_t m, const float* x, int64_t n, double h, bool laplace,
-                  int splits, double* partials, double* atomic_acc, cudaStream_t s) {
+                  int splits, double* partials, double* atomic_acc, const int* skip, cudaStream_t s) {
   const int64_t n_tiles = (n + K1_T - 1) / K1_T;
   const int64_t tps = (n_tiles + splits - 1) / splits;
   dim3 grid((unsigned)((m + K1_THREADS * K1_Q - 1) / (K1_THREADS * K1_Q)), (unsigned)((n_tiles + tps - 1) / tps));
@@ -539,9 +541,9 @@ void launch_kde1d(const float* q, int64_t m, const float* x, int64_t n, double h
   const float c1 = (float)(1.0 / (2.0 * h * h));
   TimerScope ts(K_KDE1D, (double)m * (double)n, s);
   if (laplace)
-    kde1d_kernel<true><<<grid, K1_THREADS, 0, s>>>(q, m, x, n, nc2, c1, tps, partials, atomic_acc);
+    kde1d_kernel<true><<<grid, K1_THREADS, 0, s>>>(q, m, x, n, nc2, c1, tps, partials, atomic_acc, skip);
   else
-    kde1d_kernel<false><<<grid, K1_THREADS, 0, s>>>(q, m, x, n, nc2, c1, tps, partials, atomic_acc);
+    kde1d_kernel<false><<<grid, K1_THREADS, 0, s>>>(q, m, x, n, nc2, c1, tps, partials, atomic_acc, skip);
   count_launch();
 }
 
