@@ -27,8 +27,8 @@
 //  * W += Phi_hi [X_hi | X_lo] + Phi_lo X_hi: tcgen05.mma with the A operand
 //    (weights, M=128 x K=16 per step) read from tensor memory and the B
 //    operand ((x_j - mu) 2^ew as fp16 hi and lo rows, K-major over the data
-//    points) from the data stage, FP32 accumulation over a group of S_GROUP
-//    tiles, then added into compensated FP32 sums.  Four issuing threads,
+//    points) from the data stage, FP32 accumulation over a group of tiles
+//    (score_group), then added into compensated FP32 sums.  Four issuing threads,
 //    one per (query tile, weight part), each with its own accumulator: a
 //    single thread issues an M=128, K=16, N=32 MMA every ~46 cycles, four
 //    reach the tensor core's math rate.
@@ -67,7 +67,6 @@ constexpr int S_MMA_WARP2 = S_EPI_WARPS + 2;    // issues the S MMAs of query ti
 constexpr int W_MMA_WARP = S_EPI_WARPS + 3;     // first of the W_ISSUERS weighted-sum issuers
 constexpr int W_ISSUERS = 2 * SNQT;             // (query tile, weight part hi / lo)
 constexpr int S_THREADS = (S_EPI_WARPS + 3 + W_ISSUERS) * 32;
-constexpr int S_GROUP = 16;                                // data tiles per W accumulation
 constexpr int NBUF = 2;                                    // S / weight buffers in TMEM
 constexpr int WN = 2 * FSK_D;                              // W MMA N, hi weights: X_hi and X_lo rows
 constexpr int WN_LO = FSK_D;                               // W MMA N, lo weights: X_hi rows
@@ -107,6 +106,7 @@ struct ScParams {
   const float* mu;
   int64_t n;
   WorkLine line;
+  int group;      // data tiles per W accumulation in tensor memory
   float c2, c2_lo;
   // (value, error) pairs per segment, self pair excluded, in the kernel's
   // scaled units: pdf [segment][column half][256], centred weighted sums
@@ -289,12 +289,13 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         const int count = segment_at(p.line, blockIdx.x, done_tiles).count;
         if (count == 0) break;
         done_tiles += count;
+        int left = 0;   // tiles left in the group
         for (int i = 0; i < count; ++i, ++gw) {
           const int b = gw % NBUF;
           const int s = gw % SNS;
-          const int pos = i % S_GROUP;
-          const bool first = pos == 0;
-          const bool last = pos == S_GROUP - 1 || i == count - 1;
+          const bool first = left == 0;
+          if (first) left = p.group;
+          const bool last = --left == 0 || i == count - 1;
           const int par = grp & 1;
           if (first &&
               !__all_sync(0xffffffffu, mbar_wait(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
@@ -393,6 +394,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       const int t0 = sg.t0;
       const int t1 = t0 + sg.count;
       bool pend = false;     // a W group ended at the previous tile and is not read yet
+      int left = p.group;    // tiles left in the group
       for (int t = t0; t < t1; ++t, ++g, s = (s + 1 == SNS) ? 0 : s + 1) {
         const int b = g % NBUF;
         const int valid = t == last_t ? last_valid : NT;
@@ -506,8 +508,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         }
         // read a W group that ended at the previous tile (its MMAs were
         // issued after that tile's weights, so by now they are usually done)
-        const int pos = (t - t0) % S_GROUP;
-        const bool last = pos == S_GROUP - 1 || t == t1 - 1;
+        const bool last = --left == 0 || t == t1 - 1;
+        if (last) left = p.group;
         for (int pass = 0; pass < 2; ++pass) {
           const bool do_read = pass == 0 ? pend : (last && t == t1 - 1);
           if (!do_read) continue;
@@ -609,6 +611,17 @@ done:
 
 }  // namespace
 
+// Data tiles per W accumulation.  The tensor core's FP32 accumulation over a
+// group is the largest error of the weighted sums (debiased points against
+// FP64 at n = 6258: 3.2e-7 with one group of 16 tiles, 6e-8 with groups of 1
+// or 2), each group's read-out costs about half a tile.  Small problems, bound
+// by launches and not by tiles, take short groups; 14 below and 16 above 1024
+// tiles per CTA.
+static int score_group(const TcPlan& pl) {
+  const int64_t tiles = pl.q_blocks * pl.n_tiles / pl.line.grid;
+  return tiles >= 1024 ? 16 : (int)imin<int64_t>(14, imax<int64_t>(1, tiles / 8));
+}
+
 TcPlan plan_score16(int64_t n) {
   TcPlan pl;
   pl.m_pad = (n + SNQT * QT - 1) / (SNQT * QT) * (SNQT * QT);
@@ -654,6 +667,7 @@ int launch_score16_tc(const float* x, int64_t n, double h, const TcPlan& pl, WsC
   p.mu = prep.mu;
   p.n = n;
   p.line = pl.line;
+  p.group = score_group(pl);
   p.c2 = c2;
   p.c2_lo = c2_lo;
   p.ppdf = ppdf;
