@@ -129,8 +129,8 @@ cudaError_t launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem, c
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-template <typename T> __host__ __device__ __forceinline__ T imin(T a, T b) { return a < b ? a : b; }
-template <typename T> __host__ __device__ __forceinline__ T imax(T a, T b) { return a < b ? b : a; }
+template <typename T> __host__ __device__ __forceinline__ constexpr T imin(T a, T b) { return a < b ? a : b; }
+template <typename T> __host__ __device__ __forceinline__ constexpr T imax(T a, T b) { return a < b ? b : a; }
 
 // Carves aligned sub-buffers out of a caller workspace.
 struct WsCarver {

@@ -1,5 +1,7 @@
 // fsk_mlp.cuh - surrogate MLP: parameter layout and launchers.
 #pragma once
+#include <cuda_bf16.h>
+
 #include "fsk_common.cuh"
 
 namespace fsk {
@@ -22,10 +24,11 @@ static_assert(MLP_PARAMS == 136193, "parameter layout");
 
 // Activations kept between the training forward and backward (caller workspace).
 struct TrainBufs {
-  float* a0;       // [batch][16]
-  float* z[3];     // [members][batch][256] pre-activations (overwritten by dz in backward)
-  float* a[3];     // [members][batch][256] bf16-exact activations
-  float* da;       // [members][batch][256] dz of the last hidden layer
+  __nv_bfloat16* a0;     // [batch][16]
+  __nv_bfloat16* w;      // [members][W1 | W2 | W3] bf16 weights of the current call
+  float* z[3];           // [members][batch][256] pre-activations
+  __nv_bfloat16* a[3];   // [members][batch][256] activations
+  float* dz[3];          // [members][batch][256] gradients of the pre-activations
 };
 
 TrainBufs carve_train(WsCarver& c, int members, int64_t batch);
