@@ -5,10 +5,20 @@
 // h = 0.4 * min(std, IQR / 1.34) * n^(-1/9)                   (FSK_RULE_SDKDE_1D)
 //   kernels/flash_sd_kde/empirical.py:328-333
 //
-// std is the population standard deviation (ddof=0) in FP64.  The 25th/75th
-// percentiles use numpy's default linear interpolation between the order
+// std is the population standard deviation (ddof=0) in FP64, two passes.  The
+// 25th/75th percentiles use numpy's default linear interpolation between the order
 // statistics floor(p(n-1)) and floor(p(n-1))+1, which are found exactly by a
 // 4-pass, 8-bit radix selection on order-preserving integer keys.
+//
+// Five launches: column sums and the first digits' histogram; deviations and
+// the second histogram; two more histograms; the result.  Each kernel finishes
+// the previous one's work itself - every block adds up the per-block sums it
+// needs and picks the next digit of every order statistic from the previous
+// histogram, a warp per statistic - where single-block kernels with one thread
+// per statistic scanning 256 bins took 28 us a pass (n = 10007, d = 16: 230 us
+// in 14 launches).
+#include <math.h>
+
 #include "fsk_kernels.cuh"
 
 namespace fsk {
@@ -17,13 +27,23 @@ namespace {
 constexpr int SV_MAXD = 64;
 constexpr int SV_TARGETS = 4;        // ranks: lo25, hi25, lo75, hi75
 constexpr int SV_THREADS = 256;
-constexpr int SV_BLOCKS = 256;
+constexpr int SV_WARPS = SV_THREADS / 32;
+constexpr int SV_BLOCKS = 304;
+constexpr int SV_BINS = 256;
+constexpr int SV_PASSES = 4;
+constexpr int SV_SLICE = 48;         // columns per block: 4 x 256 counters each in shared memory
 
-struct SvState {
-  uint32_t prefix[SV_MAXD][SV_TARGETS];
-  int64_t rank[SV_MAXD][SV_TARGETS];   // rank still to find inside the prefix bucket
-  double mean[SV_MAXD];
-  double m2[SV_MAXD];
+// A selection's state after some digits: the digits chosen so far and the rank
+// among the elements that share them.
+struct SvPick {
+  uint32_t prefix;
+  uint32_t rank;
+};
+
+struct SvBufs {
+  unsigned int* hist;     // [SV_PASSES][d][SV_TARGETS][SV_BINS], cleared before the first kernel
+  SvPick* pick;           // [SV_PASSES][d][SV_TARGETS] after 1, 2, ... digits
+  double* sum;            // [2][SV_BLOCKS][SV_MAXD] per-block column sums, then squared deviations
 };
 }  // namespace
 
@@ -36,170 +56,234 @@ __device__ __forceinline__ float key_to_float(uint32_t k) {
   return __uint_as_float(u);
 }
 
-// per-block FP64 column sums (pass 0) or centred sums of squares (pass 1)
-__global__ void __launch_bounds__(SV_THREADS) sv_moment_kernel(const float* __restrict__ x, int64_t n, int d,
-                                                               int pass, const SvState* __restrict__ st,
-                                                               double* __restrict__ part) {
-  __shared__ double sh[SV_MAXD];
-  for (int k = threadIdx.x; k < d; k += blockDim.x) sh[k] = 0.0;
-  __syncthreads();
-  // thread t owns column t % d of rows (t / d), (t / d) + rows_per_iter, ...
-  const int rows_per_iter = blockDim.x / d;
-  const int k = threadIdx.x % d;
-  const int lane_row = threadIdx.x / d;
-  if (lane_row < rows_per_iter) {
-    const double mk = pass == 1 ? st->mean[k] : 0.0;
-    double acc = 0.0;
-    for (int64_t r = (int64_t)blockIdx.x * rows_per_iter + lane_row; r < n;
-         r += (int64_t)gridDim.x * rows_per_iter) {
-      double v = (double)x[r * d + k];
-      if (pass == 1) {
-        v -= mk;
-        v *= v;
-      }
-      acc += v;
-    }
-    atomicAdd(&sh[k], acc);
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < d; k += blockDim.x) part[(int64_t)blockIdx.x * d + k] = sh[k];
+// floor(p (n - 1)) and its successor for p = 1/4, 3/4
+__device__ __forceinline__ int64_t target_rank(int64_t n, int t) {
+  const int64_t i = t < 2 ? (n - 1) / 4 : (3 * (n - 1)) / 4;
+  return (t & 1) ? imin<int64_t>(i + 1, n - 1) : i;
 }
 
-__global__ void sv_moment_final(const double* __restrict__ part, int blocks, int64_t n, int d, int pass,
-                                SvState* __restrict__ st) {
-  const int k = threadIdx.x;
-  if (k >= d) return;
-  double s = 0.0;
-  for (int b = 0; b < blocks; ++b) s += part[(int64_t)b * d + k];
-  if (pass == 0) st->mean[k] = s / (double)n;
-  else st->m2[k] = s / (double)n;
-}
-
-__global__ void sv_init_kernel(SvState* st, int64_t n, int d) {
-  const int k = threadIdx.x;
-  if (k >= d) return;
-  const double v25 = 0.25 * (double)(n - 1), v75 = 0.75 * (double)(n - 1);
-  const int64_t i25 = (int64_t)floor(v25), i75 = (int64_t)floor(v75);
-  const int64_t r[SV_TARGETS] = {i25, min(i25 + 1, n - 1), i75, min(i75 + 1, n - 1)};
-  for (int t = 0; t < SV_TARGETS; ++t) {
-    st->prefix[k][t] = 0u;
-    st->rank[k][t] = r[t];
-  }
-}
-
-// histogram of digit `pass` (bits [24-8*pass, 32-8*pass)) for elements whose
-// higher digits match each target's prefix.  hist: [d][SV_TARGETS][256] uint32.
-__global__ void __launch_bounds__(SV_THREADS) sv_hist_kernel(const float* __restrict__ x, int64_t n, int d,
-                                                             int pass, const SvState* __restrict__ st,
-                                                             unsigned int* __restrict__ hist) {
-  extern __shared__ unsigned int sh_hist[];  // d * SV_TARGETS * 256
-  const int nb = d * SV_TARGETS * 256;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) sh_hist[i] = 0u;
-  __syncthreads();
-  const int shift = 24 - 8 * pass;
-  const int64_t total = n * d;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e % d);
-    const uint32_t key = sortable_key(x[e]);
-    const uint32_t digit = (key >> shift) & 255u;
+// Digit of one statistic from its 256-bin histogram, by one warp holding 8 bins
+// per lane: the bin where the running count passes the rank.
+__device__ __forceinline__ SvPick pick_digit(uint4 u, uint4 v, SvPick p) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int c[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+  unsigned int total = 0;
 #pragma unroll
-    for (int t = 0; t < SV_TARGETS; ++t) {
-      const bool match = pass == 0 ? true : ((key >> (shift + 8)) == st->prefix[k][t]);
-      if (match) atomicAdd(&sh_hist[(k * SV_TARGETS + t) * 256 + digit], 1u);
+  for (int i = 0; i < 8; ++i) total += c[i];
+  unsigned int below = total;   // inclusive scan over lanes
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned int w = __shfl_up_sync(0xffffffffu, below, o);
+    if (lane >= o) below += w;
+  }
+  below -= total;
+  const bool mine = p.rank >= below && p.rank - below < total;
+  unsigned int left = p.rank - below;
+  int bin = 0;
+#pragma unroll
+  for (int i = 0; i < 7; ++i) {
+    const bool past = mine && bin == i && left >= c[i];
+    if (past) {
+      left -= c[i];
+      bin = i + 1;
     }
   }
+  const unsigned int who = __ballot_sync(0xffffffffu, mine);
+  const int src = who ? __ffs(who) - 1 : 31;
+  const uint32_t digit = (uint32_t)__shfl_sync(0xffffffffu, 8 * lane + bin, src);
+  return SvPick{(p.prefix << 8) | digit, __shfl_sync(0xffffffffu, left, src)};
+}
+
+// The selections after `digits` digits of columns [c0, c0 + dc) into shared
+// memory, a warp per statistic, from those after one digit less (written by
+// the previous kernel) and that kernel's histogram.  `keep`: write them for
+// the next kernel.
+__device__ __forceinline__ void block_picks(const SvBufs& b, int64_t n, int d, int c0, int dc, int digits, bool keep,
+                                            SvPick* pick) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = digits - 1, stats = dc * SV_TARGETS;
+  constexpr int U = 4;   // statistics in flight per warp
+  for (int s0 = warp * U; s0 < stats; s0 += SV_WARPS * U) {
+    uint4 u[U], v[U];
+    SvPick p[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+      const int s = c0 * SV_TARGETS + min(s0 + i, stats - 1);
+      // in the first pass all statistics of a column share one histogram
+      const int at = q == 0 ? s - s % SV_TARGETS : s;
+      const uint4* h = reinterpret_cast<const uint4*>(b.hist + ((int64_t)q * d * SV_TARGETS + at) * SV_BINS) + 2 * lane;
+      u[i] = h[0];
+      v[i] = h[1];
+      p[i] = q == 0 ? SvPick{0u, (uint32_t)target_rank(n, s % SV_TARGETS)}
+                    : b.pick[(int64_t)(q - 1) * d * SV_TARGETS + s];
+    }
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+      p[i] = pick_digit(u[i], v[i], p[i]);
+      if (lane == 0 && s0 + i < stats) {
+        pick[s0 + i] = p[i];
+        if (keep) b.pick[(int64_t)q * d * SV_TARGETS + c0 * SV_TARGETS + s0 + i] = p[i];
+      }
+    }
+  }
+}
+
+// Column sums of the per-block sums, by all threads of the block: thread t
+// adds column t % d of blocks t / d, t / d + rows, ..., thread k < d then its
+// column's strided sums, in a fixed order (same bits in every block).
+__device__ __forceinline__ double block_column_sum(const double* __restrict__ part, int blocks, int d,
+                                                   double (&sh)[SV_THREADS]) {
+  const int rows = SV_THREADS / d, k = threadIdx.x % d, l = threadIdx.x / d;
+  double s = 0.0;
+  if (l < rows) {
+#pragma unroll 4
+    for (int i = l; i < blocks; i += rows) s += part[(int64_t)i * SV_MAXD + k];
+  }
+  sh[threadIdx.x] = s;
   __syncthreads();
-  for (int i = threadIdx.x; i < nb; i += blockDim.x)
-    if (sh_hist[i]) atomicAdd(&hist[i], sh_hist[i]);
-}
-
-__global__ void sv_select_kernel(int d, SvState* __restrict__ st, unsigned int* __restrict__ hist) {
-  const int idx = threadIdx.x;  // one thread per (k, t)
-  if (idx >= d * SV_TARGETS) return;
-  const int k = idx / SV_TARGETS, t = idx % SV_TARGETS;
-  unsigned int* h = hist + (int64_t)idx * 256;
-  int64_t r = st->rank[k][t];
-  int b = 0;
-  for (; b < 256; ++b) {
-    if (r < (int64_t)h[b]) break;
-    r -= h[b];
+  if (threadIdx.x < d) {
+    for (int j = 1; j < rows; ++j) s += sh[j * d + threadIdx.x];
   }
-  if (b > 255) b = 255;  // unreachable for consistent counts
-  st->prefix[k][t] = (st->prefix[k][t] << 8) | (uint32_t)b;
-  st->rank[k][t] = r;
-  for (int i = 0; i < 256; ++i) h[i] = 0u;  // ready for the next pass
+  __syncthreads();
+  return s;   // threads below d
 }
 
-__global__ void sv_finish_kernel(int64_t n, int d, int rule, const SvState* __restrict__ st,
-                                 double* __restrict__ h_out) {
+// Pass 0: column sums; pass 1: squared deviations; all passes: histogram of
+// digit `pass` of the elements that match a statistic's earlier digits.
+__global__ void __launch_bounds__(SV_THREADS) sv_pass_kernel(const float* __restrict__ x, int64_t n, int d, int pass,
+                                                             SvBufs b) {
+  extern __shared__ unsigned int hist[];   // [d][SV_TARGETS][SV_BINS] (pass 0: [d][SV_BINS])
+  __shared__ SvPick pick[SV_SLICE * SV_TARGETS];
+  __shared__ double mean[SV_SLICE];
+  __shared__ double sums[SV_THREADS];
+  if (pass > 0) pdl_wait();   // (pass 0 follows an ordinary operation)
+  pdl_launch_dependents();
+  const int c0 = blockIdx.y * SV_SLICE, dc = min(SV_SLICE, d - c0);   // this block's columns
+  const int per = pass == 0 ? 1 : SV_TARGETS;
+  const int nb = dc * per * SV_BINS;
+  for (int i = threadIdx.x; i < nb; i += SV_THREADS) hist[i] = 0u;
+  if (pass > 0) block_picks(b, n, d, c0, dc, pass, blockIdx.x == 0, pick);
+  if (pass == 1) {
+    const double total = block_column_sum(b.sum + c0, gridDim.x, dc, sums);
+    if (threadIdx.x < dc) mean[threadIdx.x] = total / (double)n;
+  }
+  __syncthreads();
+  // thread t owns column t % dc of rows t / dc, t / dc + rows, ...
+  const int rows = SV_THREADS / dc, k = threadIdx.x % dc, lane_row = threadIdx.x / dc;
+  double acc = 0.0;
+  if (lane_row < rows) {
+    const int shift = 24 - 8 * pass;
+    const double mk = pass == 1 ? mean[k] : 0.0;
+    uint32_t want[SV_TARGETS];
+#pragma unroll
+    for (int t = 0; t < SV_TARGETS; ++t) want[t] = pass > 0 ? pick[k * SV_TARGETS + t].prefix : 0u;
+    unsigned int* h = hist + k * per * SV_BINS;
+    for (int64_t r = (int64_t)blockIdx.x * rows + lane_row; r < n; r += (int64_t)gridDim.x * rows) {
+      const float v = x[r * d + c0 + k];
+      const uint32_t key = sortable_key(v);
+      const uint32_t digit = (key >> shift) & 255u;
+      if (pass == 0) {
+        atomicAdd(&h[digit], 1u);
+        acc += (double)v;
+      } else {
+        const uint32_t top = key >> (shift + 8);
+#pragma unroll
+        for (int t = 0; t < SV_TARGETS; ++t)
+          if (top == want[t]) atomicAdd(&h[t * SV_BINS + digit], 1u);
+        if (pass == 1) {
+          const double c = (double)v - mk;
+          acc += c * c;
+        }
+      }
+    }
+  }
+  sums[threadIdx.x] = acc;
+  __syncthreads();
+  unsigned int* out = b.hist + ((int64_t)pass * d + c0) * SV_TARGETS * SV_BINS;
+  for (int i = threadIdx.x; i < nb; i += SV_THREADS) {
+    const unsigned int c = hist[i];
+    if (c) atomicAdd(&out[pass == 0 ? (i / SV_BINS) * SV_TARGETS * SV_BINS + i % SV_BINS : i], c);
+  }
+  if (pass < 2 && threadIdx.x < dc) {
+    double s = sums[threadIdx.x];
+    for (int j = 1; j < rows; ++j) s += sums[j * dc + threadIdx.x];
+    b.sum[((int64_t)pass * SV_BLOCKS + blockIdx.x) * SV_MAXD + c0 + threadIdx.x] = s;
+  }
+}
+
+__global__ void __launch_bounds__(SV_THREADS) sv_finish_kernel(int64_t n, int d, int rule, int blocks, double factor,
+                                                               SvBufs b, double* __restrict__ h_out) {
+  __shared__ SvPick pick[SV_MAXD * SV_TARGETS];
+  __shared__ double sig[SV_MAXD];
+  __shared__ double sums[SV_THREADS];
+  pdl_wait();
+  block_picks(b, n, d, 0, d, SV_PASSES, false, pick);
+  const double m2 = block_column_sum(b.sum + (int64_t)SV_BLOCKS * SV_MAXD, blocks, d, sums);
+  if (threadIdx.x < d) {
+    const int k = threadIdx.x;
+    const double sd = sqrt(m2 / (double)n);
+    // weights of the upper order statistic: the fraction of p (n - 1)
+    const double g25 = 0.25 * (double)((n - 1) % 4), g75 = 0.25 * (double)((3 * (n - 1)) % 4);
+    auto lerp = [](double a, double c, double t) {
+      const double diff = c - a;
+      return t >= 0.5 ? c - diff * (1.0 - t) : a + diff * t;
+    };
+    const double a25 = key_to_float(pick[k * 4].prefix), b25 = key_to_float(pick[k * 4 + 1].prefix);
+    const double a75 = key_to_float(pick[k * 4 + 2].prefix), b75 = key_to_float(pick[k * 4 + 3].prefix);
+    sig[k] = fmin(sd, (lerp(a75, b75, g75) - lerp(a25, b25, g25)) / 1.34);
+  }
+  __syncthreads();
   if (threadIdx.x != 0) return;
-  const double v25 = 0.25 * (double)(n - 1), v75 = 0.75 * (double)(n - 1);
-  const double g25 = v25 - floor(v25), g75 = v75 - floor(v75);
-  auto lerp = [](double a, double b, double t) {
-    const double diff = b - a;
-    return t >= 0.5 ? b - diff * (1.0 - t) : a + diff * t;
-  };
-  double sig_sum = 0.0;
-  for (int k = 0; k < d; ++k) {
-    const double a25 = key_to_float(st->prefix[k][0]), b25 = key_to_float(st->prefix[k][1]);
-    const double a75 = key_to_float(st->prefix[k][2]), b75 = key_to_float(st->prefix[k][3]);
-    const double iqr = lerp(a75, b75, g75) - lerp(a25, b25, g25);
-    const double sd = sqrt(st->m2[k]);
-    sig_sum += fmin(sd, iqr / 1.34);
-  }
-  double sigma = sig_sum / (double)d;
-  double h;
-  if (rule == FSK_RULE_SDKDE_1D) {
-    h = 0.4 * sigma * pow((double)n, -1.0 / 9.0);
-  } else {
-    if (sigma <= 0.0) sigma = 1.0;
-    h = 0.9 * sigma * pow((double)n, -1.0 / (double)(d + 4));
-  }
-  *h_out = h;
+  double sum = 0.0;
+  for (int k = 0; k < d; ++k) sum += sig[k];
+  double sigma = sum / (double)d;
+  if (rule != FSK_RULE_SDKDE_1D && sigma <= 0.0) sigma = 1.0;
+  *h_out = factor * sigma;
+}
+
+static SvBufs take_silverman(WsCarver& c, int d) {
+  SvBufs b;
+  b.hist = c.take<unsigned int>((size_t)SV_PASSES * d * SV_TARGETS * SV_BINS);
+  b.pick = c.take<SvPick>((size_t)SV_PASSES * d * SV_TARGETS);
+  b.sum = c.take<double>((size_t)2 * SV_BLOCKS * SV_MAXD);
+  return b;
 }
 
 size_t silverman_ws_bytes(int64_t n, int d) {
   (void)n;
-  size_t b = align_up(sizeof(SvState), 256);
-  b += align_up((size_t)SV_BLOCKS * SV_MAXD * sizeof(double), 256);
-  b += align_up((size_t)d * SV_TARGETS * 256 * sizeof(unsigned int), 256);
-  return b;
+  WsCarver c(nullptr, 0);
+  take_silverman(c, d);
+  return align_up(c.used, 256);
 }
 
 int run_silverman(const float* x, int64_t n, int d, int rule, double* h_out, void* ws, size_t ws_bytes,
                   cudaStream_t s) {
-  WsCarver c(ws, ws_bytes);
-  SvState* st = c.take<SvState>(1);
-  double* part = c.take<double>((size_t)SV_BLOCKS * SV_MAXD);
-  unsigned int* hist = c.take<unsigned int>((size_t)d * SV_TARGETS * 256);
-  if (!c.fits()) return FSK_ERR_WORKSPACE_TOO_SMALL;
   if (d < 1 || d > SV_MAXD) return FSK_ERR_INVALID_ARGUMENT;
-  const int blocks = (int)imax<int64_t>(1, imin<int64_t>(SV_BLOCKS, (n * d + SV_THREADS - 1) / SV_THREADS));
-  cudaError_t e = cudaMemsetAsync(hist, 0, (size_t)d * SV_TARGETS * 256 * sizeof(unsigned int), s);
+  WsCarver c(ws, ws_bytes);
+  const SvBufs b = take_silverman(c, d);
+  if (!c.fits()) return FSK_ERR_WORKSPACE_TOO_SMALL;
+  const int slices = (d + SV_SLICE - 1) / SV_SLICE;
+  const int rows = SV_THREADS / imin(d, SV_SLICE);
+  const int blocks = (int)imax<int64_t>(1, imin<int64_t>(SV_BLOCKS, (n + 4 * rows - 1) / (4 * rows)));
+  cudaError_t e = cudaMemsetAsync(b.hist, 0, (size_t)SV_PASSES * d * SV_TARGETS * SV_BINS * sizeof(unsigned int), s);
   if (e != cudaSuccess) return cuda_status(e);
-  sv_init_kernel<<<1, SV_MAXD, 0, s>>>(st, n, d);
-  count_launch();
-  for (int pass = 0; pass < 2; ++pass) {
-    sv_moment_kernel<<<blocks, SV_THREADS, 0, s>>>(x, n, d, pass, st, part);
-    count_launch();
-    sv_moment_final<<<1, SV_MAXD, 0, s>>>(part, blocks, n, d, pass, st);
-    count_launch();
-  }
-  const size_t hsm = (size_t)d * SV_TARGETS * 256 * sizeof(unsigned int);
-  if (hsm > 48 * 1024) {
-    e = cudaFuncSetAttribute(sv_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
+  const size_t hsm = (size_t)imin(d, SV_SLICE) * SV_TARGETS * SV_BINS * sizeof(unsigned int);
+  if (hsm > 32 * 1024) {
+    e = cudaFuncSetAttribute(sv_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
     if (e != cudaSuccess) return cuda_status(e);
   }
-  for (int pass = 0; pass < 4; ++pass) {
-    sv_hist_kernel<<<blocks, SV_THREADS, hsm, s>>>(x, n, d, pass, st, hist);
-    count_launch();
-    sv_select_kernel<<<1, SV_MAXD * SV_TARGETS, 0, s>>>(d, st, hist);
+  const dim3 grid((unsigned)blocks, (unsigned)slices);
+  sv_pass_kernel<<<grid, SV_THREADS, hsm / SV_TARGETS, s>>>(x, n, d, 0, b);
+  count_launch();
+  for (int pass = 1; pass < SV_PASSES; ++pass) {
+    launch_pdl(sv_pass_kernel, grid, SV_THREADS, hsm, s, x, n, d, pass, b);
     count_launch();
   }
-  sv_finish_kernel<<<1, 32, 0, s>>>(n, d, rule, st, h_out);
+  const double factor = rule == FSK_RULE_SDKDE_1D ? 0.4 * pow((double)n, -1.0 / 9.0)
+                                                  : 0.9 * pow((double)n, -1.0 / (double)(d + 4));
+  e = launch_pdl(sv_finish_kernel, 1, SV_THREADS, 0, s, n, d, rule, blocks, factor, b, h_out);
   count_launch();
-  return cuda_status(cudaGetLastError());
+  return e != cudaSuccess ? cuda_status(e) : cuda_status(cudaGetLastError());
 }
 
 }  // namespace fsk
