@@ -26,6 +26,7 @@ from flash_sd_kde.config import (
     validate_kde_backend,
     validate_precision_mode,
 )
+from fsk import _lib as L
 from fsk import ops
 from globals import (
     DEFAULT_EMP_SCORE_BACKEND,
@@ -67,8 +68,6 @@ def _require_cuda(device, name: str) -> torch.device:
     device = torch.device(device)
     if device.type != "cuda":
         raise ValueError(f"{name} currently expects a CUDA device.")
-    if not torch.cuda.is_available():
-        raise RuntimeError("CUDA is not available but was requested.")
     return ops._device(device)
 
 
@@ -115,10 +114,15 @@ def _kde_eval_impl(data, queries, bandwidth, *, device, precision_mode, kde_back
         if n_data == 0 or query.shape[0] == 0:
             raise ValueError("data and queries must be non-empty.")
         norm = 1.0 / ((2.0 * math.pi) ** (d / 2.0) * (bandwidth ** d) * n_data)
-        prec = "ieee" if precision_mode == PRECISION_FP32_IEEE else "tensor"
-        return ops.kde16_sum(query, train, bandwidth, precision=prec, laplace=apply_laplacian_correction,
-                             atomic=atomic, out_scale=norm, log_eps=None if log_exact else log_eps,
-                             log_exact=log_exact)
+        # the rows are checked: straight to the launch
+        flags = L.FSK_PREC_IEEE if precision_mode == PRECISION_FP32_IEEE else L.FSK_PREC_TENSOR
+        flags |= (L.FSK_LAPLACE if apply_laplacian_correction else 0) | (L.FSK_ATOMIC if atomic else 0)
+        if log_exact:
+            flags |= L.FSK_OUT_LOG | L.FSK_OUT_LOG_EXACT
+            log_eps = 0.0
+        elif log_eps is not None:
+            flags |= L.FSK_OUT_LOG
+        return ops._kde16(query, train, ops._check_bw(bandwidth), device, flags, norm, float(log_eps or 0.0))
     raise ValueError("data must be 1D or 2D.")
 
 
@@ -228,9 +232,9 @@ def emp_sd_kde_fit_transform(
     if train.shape[0] == 0:
         raise ValueError("data must be non-empty.")
     prec = "ieee" if precision_mode == PRECISION_FP32_IEEE else "tensor"
-    symmetric = emp_score_backend == EMP_SCORE_BACKEND_SYMMETRIC_ATOMIC
-    out = ops.sdshift16(train, bandwidth, eps, variant="symmetric" if symmetric else "ordered", precision=prec,
-                        feature_major=emp_score_backend == EMP_SCORE_BACKEND_FLASH_SD_KDE, return_debug=return_debug)
+    out = ops._sdshift16(train, ops._check_bw(bandwidth), eps, device,
+                         emp_score_backend == EMP_SCORE_BACKEND_SYMMETRIC_ATOMIC,
+                         emp_score_backend == EMP_SCORE_BACKEND_FLASH_SD_KDE, prec == "ieee", return_debug)
     if return_debug:
         debiased, pdf_sum, weighted_sum, score = out
         if d < ND_FEATURES:   # the padded columns are 0 in every output

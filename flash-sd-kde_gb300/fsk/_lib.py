@@ -107,6 +107,8 @@ _lib = None
 def load(path: str | os.PathLike | None = None):
     """Load libfsk.so (once) and attach the ctypes signatures."""
     global _lib
+    if path is None and _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None and path is None:
             return _lib

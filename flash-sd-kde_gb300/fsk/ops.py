@@ -10,6 +10,7 @@ error.
 from __future__ import annotations
 
 import math
+from contextlib import nullcontext
 from typing import Sequence
 
 import torch
@@ -20,7 +21,7 @@ ND_FEATURES = 16
 
 
 def _device(device) -> torch.device:
-    dev = torch.device(device)
+    dev = device if isinstance(device, torch.device) else torch.device(device)
     if dev.type != "cuda":
         raise ValueError("the GB300 kernels require a CUDA device.")
     if not torch.cuda.is_available():
@@ -28,6 +29,14 @@ def _device(device) -> torch.device:
     if dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
     return dev
+
+
+_HERE = nullcontext()
+
+
+def _on(dev: torch.device):
+    """Context with `dev` current (nothing to do where it already is)."""
+    return _HERE if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
 
 
 def as_matrix(x: Sequence[Sequence[float]] | torch.Tensor, device: torch.device, dim: int = ND_FEATURES) -> torch.Tensor:
@@ -73,7 +82,8 @@ def _ptr(t: torch.Tensor | None):
 
 
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the handle alone: building a Stream object costs 2 us of every call
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
@@ -115,12 +125,11 @@ def kde16_sum(
     dev = _device(queries.device)
     q = as_matrix(queries, dev)
     x = as_matrix(data, dev)
-    m, n = q.shape[0], x.shape[0]
-    if m == 0 or n == 0:
+    if q.shape[0] == 0 or x.shape[0] == 0:
         raise ValueError("data and queries must contain at least one sample.")
-    if precision not in ("tensor", "ieee", "fp16_single"):
+    if precision not in _KDE16_PRECISION:
         raise ValueError(f"unknown precision {precision!r}")
-    flags = {"tensor": L.FSK_PREC_TENSOR, "ieee": L.FSK_PREC_IEEE, "fp16_single": L.FSK_PREC_FP16_SINGLE}[precision]
+    flags = _KDE16_PRECISION[precision]
     flags |= (L.FSK_LAPLACE if laplace else 0) | (L.FSK_ATOMIC if atomic else 0)
     flags |= L.FSK_EXP_OFFLOAD if exp_offload else 0
     if log_exact:
@@ -130,15 +139,26 @@ def kde16_sum(
         flags |= L.FSK_OUT_LOG_EXACT
     if log_eps is not None:
         flags |= L.FSK_OUT_LOG
+    return _kde16(q, x, h, dev, flags, float(out_scale), float(log_eps or 0.0), out)
+
+
+_KDE16_PRECISION = {"tensor": L.FSK_PREC_TENSOR, "ieee": L.FSK_PREC_IEEE, "fp16_single": L.FSK_PREC_FP16_SINGLE}
+
+
+def _kde16(q: torch.Tensor, x: torch.Tensor, h: float, dev: torch.device, flags: int, out_scale: float,
+           out_eps: float, out: torch.Tensor | None = None) -> torch.Tensor:
+    """fsk_kde16 on checked, contiguous (., 16) FP32 tensors of `dev`."""
+    m, n = q.shape[0], x.shape[0]
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         if out is None:
             out = torch.empty(m, dtype=torch.float32, device=dev)
         ws_bytes = lib.fsk_kde16_workspace_bytes(m, n, flags)
         ws = _workspace(ws_bytes, dev)
-        st = lib.fsk_kde16(q.data_ptr(), m, x.data_ptr(), n, h, flags, float(out_scale),
-                           float(log_eps or 0.0), out.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev))
-    L.check(st, "fsk_kde16")
+        st = lib.fsk_kde16(q.data_ptr(), m, x.data_ptr(), n, h, flags, out_scale, out_eps, out.data_ptr(),
+                           ws.data_ptr(), ws.numel(), _stream(dev))
+    if st:
+        L.check(st, "fsk_kde16")
     return out
 
 
@@ -164,7 +184,7 @@ def empscore16(
     flags = L.FSK_WEIGHTED_FEATURE_MAJOR if feature_major else 0
     flags |= L.FSK_PREC_IEEE if precision == "ieee" else L.FSK_PREC_TENSOR
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         pdf = torch.empty(n, dtype=torch.float32, device=dev)
         w = torch.empty((ND_FEATURES, n) if feature_major else (n, ND_FEATURES), dtype=torch.float32, device=dev)
         ws = _workspace(lib.fsk_empscore16_workspace_bytes(n, var, flags), dev)
@@ -189,15 +209,20 @@ def sdshift16(
     h = _check_bw(bandwidth)
     dev = _device(data.device)
     x = as_matrix(data, dev)
-    n = x.shape[0]
-    if n == 0:
+    if x.shape[0] == 0:
         raise ValueError("data must contain at least one element.")
-    var = L.FSK_SCORE_SYMMETRIC if variant == "symmetric" else L.FSK_SCORE_ORDERED
-    flags = L.FSK_WEIGHTED_FEATURE_MAJOR if feature_major else 0
-    flags |= L.FSK_PREC_IEEE if precision == "ieee" else L.FSK_PREC_TENSOR
+    return _sdshift16(x, h, eps, dev, variant == "symmetric", feature_major, precision == "ieee", return_debug)
+
+
+def _sdshift16(x: torch.Tensor, h: float, eps: float, dev: torch.device, symmetric: bool, feature_major: bool,
+               ieee: bool, return_debug: bool):
+    """fsk_sdshift16 on a checked, contiguous (n, 16) FP32 tensor of `dev`."""
+    n = x.shape[0]
+    var = L.FSK_SCORE_SYMMETRIC if symmetric else L.FSK_SCORE_ORDERED
+    flags = (L.FSK_WEIGHTED_FEATURE_MAJOR if feature_major else 0) | (L.FSK_PREC_IEEE if ieee else L.FSK_PREC_TENSOR)
     lib = L.load()
     pdf = w = score = None
-    with torch.cuda.device(dev):
+    with _on(dev):
         deb = torch.empty_like(x)
         if return_debug:
             pdf = torch.empty(n, dtype=torch.float32, device=dev)
@@ -206,7 +231,8 @@ def sdshift16(
         ws = _workspace(lib.fsk_sdshift16_workspace_bytes(n, var, flags), dev)
         st = lib.fsk_sdshift16(x.data_ptr(), n, h, var, flags, float(eps), deb.data_ptr(), _ptr(pdf), _ptr(w),
                                _ptr(score), ws.data_ptr(), ws.numel(), _stream(dev))
-    L.check(st, "fsk_sdshift16")
+    if st:
+        L.check(st, "fsk_sdshift16")
     return (deb, pdf, w.t() if feature_major else w, score) if return_debug else deb
 
 
@@ -250,7 +276,7 @@ def sdkde16(
     if out_scale is None:
         out_scale = 1.0 / ((2.0 * math.pi) ** 8 * h ** 16 * n)
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         if out is None:
             out = torch.empty(m, dtype=torch.float32, device=dev)
         deb = torch.empty_like(x) if return_debiased else None
@@ -317,7 +343,7 @@ def kde_nd_sum(queries, data, bandwidth: float, *, laplace: bool = False, out_sc
         raise ValueError("data and queries must contain at least one sample.")
     flags = (L.FSK_LAPLACE if laplace else 0) | (L.FSK_OUT_LOG if log_eps is not None else 0)
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty(m, dtype=torch.float32, device=dev)
         ws = _workspace(lib.fsk_kde_nd_workspace_bytes(m, n, d, flags), dev)
         st = lib.fsk_kde_nd(q.data_ptr(), m, x.data_ptr(), n, d, h, flags, float(out_scale), float(log_eps or 0.0),
@@ -335,7 +361,7 @@ def empscore_nd(data, bandwidth: float) -> tuple[torch.Tensor, torch.Tensor]:
     if n == 0:
         raise ValueError("data must contain at least one element.")
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         pdf = torch.empty(n, dtype=torch.float32, device=dev)
         w = torch.empty((n, d), dtype=torch.float32, device=dev)
         ws = _workspace(lib.fsk_empscore_nd_workspace_bytes(n, d), dev)
@@ -357,7 +383,7 @@ def debias_nd(data, pdf_sum: torch.Tensor, weighted_sum: torch.Tensor, bandwidth
     if w.shape != (n, d) or pdf.shape != (n,):
         raise ValueError("pdf_sum must be (n,) and weighted_sum (n, d).")
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         deb = torch.empty_like(x)
         score = torch.empty_like(x) if return_score else None
         st = lib.fsk_debias_nd(x.data_ptr(), n, d, pdf.data_ptr(), w.data_ptr(), h, float(eps), deb.data_ptr(),
@@ -385,7 +411,7 @@ def debias16(
     if w.shape != (n, ND_FEATURES) or pdf.shape != (n,):
         raise ValueError("pdf_sum must be (n,) and weighted_sum (n, 16).")
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         deb = torch.empty_like(x)
         score = torch.empty_like(x) if return_score else None
         st = lib.fsk_debias16(x.data_ptr(), n, pdf.data_ptr(), w.data_ptr(), w.stride(0), w.stride(1), h,
@@ -415,7 +441,7 @@ def kde1d_sum(
     if log_eps is not None:
         flags |= L.FSK_OUT_LOG
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty(m, dtype=torch.float32, device=dev)
         ws = _workspace(lib.fsk_kde1d_workspace_bytes(m, n, flags), dev)
         st = lib.fsk_kde1d(q.data_ptr(), m, x.data_ptr(), n, h, flags, float(out_scale), float(log_eps or 0.0),
@@ -434,7 +460,7 @@ def kde1d_score(queries: torch.Tensor, data: torch.Tensor, bandwidth: float):
     if m == 0 or n == 0:
         raise ValueError("data and queries must be non-empty.")
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         score = torch.empty(m, dtype=torch.float32, device=dev)
         pdf = torch.empty_like(score)
         deriv = torch.empty_like(score)
@@ -459,7 +485,7 @@ def silverman(data: torch.Tensor, *, rule: str = "silverman") -> torch.Tensor:
         raise ValueError("data must contain at least one element.")
     r = L.FSK_RULE_SDKDE_1D if rule == "sdkde_1d" else L.FSK_RULE_SILVERMAN
     lib = L.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         h = torch.empty((), dtype=torch.float64, device=dev)
         ws = _workspace(lib.fsk_silverman_workspace_bytes(n, d), dev)
         st = lib.fsk_silverman(x.data_ptr(), n, d, r, h.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev))
@@ -470,7 +496,7 @@ def silverman(data: torch.Tensor, *, rule: str = "silverman") -> torch.Tensor:
 def device_status(device=None) -> None:
     """Synchronise and raise if a bounded in-kernel wait recorded a timeout."""
     dev = _device(device if device is not None else "cuda")
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = L.load().fsk_device_status(_stream(dev))
     L.check(st, "device status")
 
@@ -482,7 +508,7 @@ def mma_probe(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     b = b.to(device=dev, dtype=torch.float32).contiguous()
     if a.shape != (128, 32) or b.shape != (64, 32):
         raise ValueError("probe operands must be (128, 32) and (64, 32)")
-    with torch.cuda.device(dev):
+    with _on(dev):
         d = torch.empty((128, 64), dtype=torch.float32, device=dev)
         st = L.load().fsk_diag_mma_probe(a.data_ptr(), b.data_ptr(), d.data_ptr(), _stream(dev))
     L.check(st, "fsk_diag_mma_probe")
@@ -496,7 +522,7 @@ def mma_ts_probe(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     b = b.to(device=dev, dtype=torch.float32).contiguous()
     if a.shape != (128, 64) or b.shape != (16, 64):
         raise ValueError("probe operands must be (128, 64) and (16, 64)")
-    with torch.cuda.device(dev):
+    with _on(dev):
         d = torch.empty((128, 16), dtype=torch.float32, device=dev)
         st = L.load().fsk_diag_mma_ts_probe(a.data_ptr(), b.data_ptr(), d.data_ptr(), _stream(dev))
     L.check(st, "fsk_diag_mma_ts_probe")
@@ -510,7 +536,7 @@ def tmem_cp_probe(a: torch.Tensor) -> torch.Tensor:
     a = a.to(device=dev, dtype=torch.float32).contiguous()
     if a.shape != (128, 32):
         raise ValueError("probe operand must be (128, 32)")
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty((128, 16), dtype=torch.int32, device=dev)
         st = L.load().fsk_diag_tmem_cp_probe(a.data_ptr(), out.data_ptr(), _stream(dev))
     L.check(st, "fsk_diag_tmem_cp_probe")
@@ -537,7 +563,7 @@ def mlp_fwd(params, members, x, in_mean, in_inv_std, ws, y=None) -> torch.Tensor
     batch = x.shape[0]
     if y is None:
         y = torch.empty((members, batch), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = L.load().fsk_mlp_fwd(params.data_ptr(), members, x.data_ptr(), batch, in_mean.data_ptr(),
                                   in_inv_std.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev))
     L.check(st, "fsk_mlp_fwd")
@@ -549,7 +575,7 @@ def mlp_bwd(params, members, batch, dy, ws, grads=None) -> torch.Tensor:
     dev = _device(params.device)
     if grads is None:
         grads = torch.empty_like(params)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = L.load().fsk_mlp_bwd(params.data_ptr(), members, batch, dy.data_ptr(), grads.data_ptr(),
                                   ws.data_ptr(), ws.numel(), _stream(dev))
     L.check(st, "fsk_mlp_bwd")
@@ -559,7 +585,7 @@ def mlp_bwd(params, members, batch, dy, ws, grads=None) -> torch.Tensor:
 def mlp_mse(y, target, dy, loss=None) -> None:
     members, batch = y.shape
     dev = _device(y.device)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = L.load().fsk_mlp_mse(y.data_ptr(), target.data_ptr(), batch, members, dy.data_ptr(),
                                   _ptr(loss), _stream(dev))
     L.check(st, "fsk_mlp_mse")
@@ -567,7 +593,7 @@ def mlp_mse(y, target, dy, loss=None) -> None:
 
 def mlp_adam(params, grads, m, v, step, lr, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0) -> None:
     dev = _device(params.device)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = L.load().fsk_mlp_adam(params.data_ptr(), grads.data_ptr(), m.data_ptr(), v.data_ptr(),
                                    params.numel(), float(lr), float(beta1), float(beta2), float(eps),
                                    float(weight_decay), int(step), _stream(dev))
@@ -579,7 +605,7 @@ def mlp_pack(params, members, in_mean, in_inv_std, out_scale=1.0, out_shift=0.0)
     dev = _device(params.device)
     lib = L.load()
     packed = torch.empty(lib.fsk_mlp_packed_bytes(members), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = lib.fsk_mlp_pack(params.data_ptr(), members, in_mean.data_ptr(), in_inv_std.data_ptr(),
                               float(out_scale), float(out_shift), packed.data_ptr(), _stream(dev))
     L.check(st, "fsk_mlp_pack")
@@ -592,7 +618,7 @@ def mlp_infer(packed, members, x, y=None) -> torch.Tensor:
     batch = x.shape[0]
     if y is None:
         y = torch.empty((members, batch), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = L.load().fsk_mlp_infer(packed.data_ptr(), members, x.data_ptr(), batch, y.data_ptr(), _stream(dev))
     L.check(st, "fsk_mlp_infer")
     return y
@@ -606,7 +632,7 @@ def mlp_combine(y, x=None, in_mean=None, in_inv_std=None, base_a=0.0, base_b=0.0
     mean = torch.empty(batch, dtype=torch.float32, device=dev)
     spread = torch.empty(batch, dtype=torch.float32, device=dev)
     served = torch.empty(batch, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         st = L.load().fsk_mlp_combine(y.data_ptr(), members, batch, _ptr(x), _ptr(in_mean), _ptr(in_inv_std),
                                       float(base_a), float(base_b), float(spread_tol), float(r2_max),
                                       mean.data_ptr(), spread.data_ptr(), served.data_ptr(), _stream(dev))
