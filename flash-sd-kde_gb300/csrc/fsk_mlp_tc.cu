@@ -3,9 +3,9 @@
 // activations, FP32 accumulation, one ensemble member per CTA.
 //
 // Per tile of 128 queries (one TMEM lane each):
-//   A0 = bf16((x - mean) * inv_std)         epilogue warps -> TMEM cols 256..263
+//   A0 = bf16((x - mean) * inv_std)         epilogue warps -> TMEM
 //   D  = A0 . W1^T                           1 MMA, M=128, N=256, K=16
-//   A1 = bf16(silu(D + b1))                  TMEM -> registers -> TMEM cols 256..383
+//   A1 = bf16(silu(D + b1))                  TMEM -> registers -> TMEM
 //   D  = A1 . W2^T                           16 MMAs (K steps), N=256
 //   A2 = bf16(silu(D + b2)); D = A2 . W3^T   16 MMAs
 //   y  = bf16(silu(D + b3)) . bf16(w4) + b4  per-thread dot, four feature quarters combined
@@ -13,9 +13,22 @@
 // (tcgen05.mma with A in TMEM), so nothing is transposed through shared
 // memory.  W2 and W3 (128 KB each in bf16) do not fit in shared memory next
 // to anything else, so they stream from L2 as 8 KB K slices ([256 out][16 in],
-// core-matrix K-major) through a ring of RING slots; W1, the biases, w4 and
-// the input normalisation are loaded once per CTA.
+// core-matrix K-major), four to a copy, through a ring of RING 32 KB slots; W1,
+// the biases, w4 and the input normalisation are loaded once per CTA.
 //
+// Two tiles run in turn on one accumulator: the epilogue warps drain the whole
+// accumulator of one tile into registers (64 per thread) and hand it to the
+// other tile's MMAs before they start on bias and SiLU, so tensor core and
+// tanh unit work at the same time, and each weight slice serves both tiles.
+// 2^20 queries x 4 members: 3.06 ms with one tile at a time and a wait and a
+// release per slice (the issuing thread then takes 250-400 cycles per MMA, of
+// which the tensor core needs 133); 1.82 ms with two tiles, 1.04 with four
+// slices per wait, inputs by bulk copy and one bf16 conversion per pair, 0.94
+// with packed FMAs.  The tanh unit is busy 0.69 ms of that (3.2e9 tanh at 16
+// per cycle and SM), the tensor core 0.47.  Where every block has one tile
+// there is nothing to pair and it runs alone.
+//
+// TMEM: accumulator 256 columns | activations of tile 0, 128 | of tile 1, 128.
 // Warps: 0-15 epilogue (warp w: TMEM lane quarter w&3, feature quarter
 // w>>2), 16 producer (bulk copies), 17 MMA issue + TMEM owner.
 #include <cuda_bf16.h>
@@ -33,7 +46,11 @@ namespace {
 constexpr int QT = 128;                         // queries per tile
 constexpr int SLICE_BYTES = MLP_H * 16 * 2;     // one K slice: [256][16] bf16 = 8 KB
 constexpr int N_SLICES = MLP_H / 16;            // 16 per hidden layer
-constexpr int RING = 24;                        // slices in flight: hides L2 latency across layers
+constexpr int CHUNK = 4;                        // slices per copy, per wait and per release
+constexpr int CHUNK_BYTES = CHUNK * SLICE_BYTES;   // 32 KB
+constexpr int LAYER_CHUNKS = N_SLICES / CHUNK;  // 4
+constexpr int RING = 6;                         // chunks in flight: a layer and half of the next
+constexpr int X_BYTES = QT * MLP_IN * 4;        // a tile's inputs, 8 KB
 // packed member image (global):
 //   header 256 B: in_mean[16] in_inv_std[16] out_scale out_shift b4 (FP32)
 //   b1 b2 b3 w4 (FP32, w4 bf16-rounded) 4 KB
@@ -47,22 +64,25 @@ constexpr int MEMBER_BYTES = W3_OFF + N_SLICES * SLICE_BYTES;
 // shared memory
 constexpr int SM_CONST_BYTES = W2_OFF;                     // header + vectors + W1 image (one copy)
 constexpr int SM_RING_OFF = SM_CONST_BYTES;
-constexpr int SM_YSUM_OFF = SM_RING_OFF + RING * SLICE_BYTES;
-constexpr int SM_BAR_OFF = SM_YSUM_OFF + 3 * QT * 4;
-constexpr int N_BARS = 5 + 2 * RING;             // cready, full/empty ring, aready, dfull, ycomb, drain
+constexpr int SM_X_OFF = SM_RING_OFF + RING * CHUNK_BYTES;
+constexpr int SM_HB_OFF = SM_X_OFF + 2 * X_BYTES;
+constexpr int SM_YSUM_OFF = SM_HB_OFF + 3 * MLP_H * 4;
+constexpr int SM_BAR_OFF = SM_YSUM_OFF + 2 * 3 * QT * 4;
+constexpr int N_BARS = 12 + 2 * RING;   // cready, ring, aready 2, dfull, dfree, ycomb 2, x full 2, x empty 2, drain
 constexpr int SMEM_BYTES = SM_BAR_OFF + (N_BARS + 1) * 8;   // + the TMEM address slot
 constexpr int EPI_WARPS = 16;
 constexpr int PROD_WARP = 16;
 constexpr int MMA_WARP = 17;
 constexpr int THREADS = 18 * 32;
 constexpr int T_D = 0;       // accumulator: 256 FP32 columns
-constexpr int T_A = 256;     // activations: 128 columns of packed bf16 pairs
+constexpr int T_A = 256;     // activations: 128 columns of packed bf16 pairs per tile
+constexpr int T_A_TILE = 128;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 static_assert(MEMBER_BYTES % 16 == 0 && W1_OFF % 16 == 0, "bulk copy alignment");
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) |
-         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -71,10 +91,14 @@ __device__ __forceinline__ float tanh_approx(float x) {
   return y;
 }
 
-// silu(z) = z sigmoid(z) = 0.5 z (1 + tanh(z / 2))
-__device__ __forceinline__ float silu_fast(float z) {
-  const float h = 0.5f * z;
-  return fmaf(h, tanh_approx(h), h);
+// bf16 pair of silu(z + b) = h (1 + tanh h), h = (z + b) / 2, from the
+// accumulators and the halved biases: h = z / 2 + hb in one rounding is the
+// halved sum (a power of two), so a pair takes two packed FMAs, two tanh and
+// one conversion.
+__device__ __forceinline__ uint32_t silu_pair(uint32_t z0, uint32_t z1, float hb0, float hb1) {
+  const float2 h = __ffma2_rn(make_float2(__uint_as_float(z0), __uint_as_float(z1)), make_float2(0.5f, 0.5f), make_float2(hb0, hb1));
+  const float2 a = __ffma2_rn(h, make_float2(tanh_approx(h.x), tanh_approx(h.y)), h);
+  return pack_bf16(a.x, a.y);
 }
 
 struct InferParams {
@@ -83,25 +107,30 @@ struct InferParams {
   const float* x;
   int64_t batch;
   float* y;            // [members][batch]
-  int64_t tiles;
+  int tiles;
+  int per;             // tiles per turn: 2, or 1 where every CTA has one tile at most
 };
 
 __global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(InferParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const float* hdr = reinterpret_cast<const float*>(smem);
   const float* vec = reinterpret_cast<const float*>(smem + HDR_BYTES);   // b1 b2 b3 w4
+  float* half_b = reinterpret_cast<float*>(smem + SM_HB_OFF);            // b1 b2 b3, halved
   uint8_t* ring = smem + SM_RING_OFF;
-  float* ysum = reinterpret_cast<float*>(smem + SM_YSUM_OFF);
+  float* ysum = reinterpret_cast<float*>(smem + SM_YSUM_OFF);            // [2 tiles][3][QT]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM_BAR_OFF);
-  uint64_t* cready = bars;               // constants loaded
-  uint64_t* full = bars + 1;             // [RING]
-  uint64_t* empty = bars + 1 + RING;     // [RING]
-  uint64_t* aready = bars + 1 + 2 * RING;  // activations (or inputs) stored, all epilogue warps
-  uint64_t* dfull = bars + 2 + 2 * RING;   // layer accumulator complete
-  uint64_t* ycomb = bars + 3 + 2 * RING;   // partial dots of feature quarters 1-3 stored, 12 warps
-  uint64_t* drain = bars + 4 + 2 * RING;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5 + 2 * RING);
-  int64_t n_ring_copies = 0;
+  uint64_t* cready = bars;                 // constants loaded
+  uint64_t* full = bars + 1;               // [RING]
+  uint64_t* empty = bars + 1 + RING;       // [RING] chunk read for every tile of the turn
+  uint64_t* aready = bars + 1 + 2 * RING;  // [2] a tile's activations (or inputs) stored, all epilogue warps
+  uint64_t* dfull = aready + 2;            // accumulator complete
+  uint64_t* dfree = aready + 3;            // accumulator drained into registers, all epilogue warps
+  uint64_t* ycomb = aready + 4;            // [2] a tile's partial dots of feature quarters 1-3 stored, 12 warps
+  uint64_t* xfull = aready + 6;            // [2] a tile's inputs in shared memory
+  uint64_t* xempty = aready + 8;           // [2] and read, all epilogue warps
+  uint64_t* drain = aready + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aready + 11);
+  unsigned n_ring_copies = 0, n_x_copies[2] = {0, 0};
   int n_const_copies = 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -115,12 +144,19 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(InferParams p) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
-    mbar_init(aready, EPI_WARPS);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&aready[i], EPI_WARPS);
+      mbar_init(&ycomb[i], 12);
+      mbar_init(&xfull[i], 1);
+      mbar_init(&xempty[i], EPI_WARPS);
+    }
     mbar_init(dfull, 1);
-    mbar_init(ycomb, 12);
+    mbar_init(dfree, EPI_WARPS);
     mbar_init(drain, 1);
     fence_barrier_init();
   }
+  for (int i = threadIdx.x; i < 3 * MLP_H; i += THREADS)
+    half_b[i] = 0.5f * reinterpret_cast<const float*>(img + HDR_BYTES)[i];
   if (warp == MMA_WARP) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -129,20 +165,36 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(InferParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // turns of this CTA: tiles t0 .. t0 + per - 1, t0 = per (group + i groups)
+  const int t_first = group * p.per, t_step = groups * p.per;
 
   if (warp == PROD_WARP) {
     if (lane == 0) {
       mbar_arrive_expect_tx(cready, SM_CONST_BYTES);
       bulk_g2s(smem, img, SM_CONST_BYTES, cready);
       n_const_copies = 1;
-      int64_t g = 0;
-      for (int64_t t = group; t < p.tiles; t += groups) {
-        for (int sl = 0; sl < 2 * N_SLICES; ++sl, ++g) {
-          const int s = (int)(g % RING);
-          if (!mbar_wait(&empty[s], (uint32_t)(((g / RING) & 1) ^ 1), 51)) goto done;
-          mbar_arrive_expect_tx(&full[s], SLICE_BYTES);
-          bulk_g2s(ring + s * SLICE_BYTES, img + W2_OFF + sl * SLICE_BYTES, SLICE_BYTES, &full[s]);
-          n_ring_copies = g + 1;
+      int s = 0;
+      uint32_t ph = 0;
+      for (int t = t_first; t < p.tiles; t += t_step) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (k >= p.per || t + k >= p.tiles) continue;
+          if (!mbar_wait(&xempty[k], (n_x_copies[k] & 1u) ^ 1u, 51)) goto done;
+          const int64_t q = (int64_t)(t + k) * QT;
+          const uint32_t bytes = (uint32_t)imin<int64_t>(QT, p.batch - q) * (MLP_IN * 4);
+          mbar_arrive_expect_tx(&xfull[k], bytes);
+          bulk_g2s(smem + SM_X_OFF + k * X_BYTES, p.x + q * MLP_IN, bytes, &xfull[k]);
+          ++n_x_copies[k];
+        }
+        for (int c = 0; c < 2 * LAYER_CHUNKS; ++c) {
+          if (!mbar_wait(&empty[s], ph ^ 1u, 62)) goto done;
+          mbar_arrive_expect_tx(&full[s], CHUNK_BYTES);
+          bulk_g2s(ring + s * CHUNK_BYTES, img + W2_OFF + c * CHUNK_BYTES, CHUNK_BYTES, &full[s]);
+          ++n_ring_copies;
+          if (++s == RING) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
     }
@@ -152,28 +204,48 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(InferParams p) {
       const uint64_t w1d = smem_desc_kmajor(smem_u32(smem + W1_OFF), 128, 8 * 32);
       const uint64_t r0 = smem_desc_kmajor(smem_u32(ring), 128, 8 * 32);
       if (!mbar_wait(cready, 0, 52)) goto done;
-      int64_t g = 0;
-      int k = 0;   // layer phases completed (aready / dfull parity)
-      for (int64_t t = group; t < p.tiles; t += groups) {
-        // layer 1: inputs stored by the epilogue
-        if (!mbar_wait(aready, (uint32_t)(k & 1), 53)) goto done;
-        tc_fence_after();
-        mma_f16_ts(tmem + T_D, tmem + T_A, w1d, idesc, 0u);
-        mma_commit(dfull);
-        ++k;
-        for (int layer = 0; layer < 2; ++layer) {
-          if (!mbar_wait(aready, (uint32_t)(k & 1), 54)) goto done;
-          tc_fence_after();
-          for (int ks = 0; ks < N_SLICES; ++ks, ++g) {
-            const int s = (int)(g % RING);
-            if (!mbar_wait(&full[s], (uint32_t)((g / RING) & 1), 55)) goto done;
+      int s0 = 0;              // ring slot of the layer's first chunk
+      uint32_t ph0 = 0;        // and its phase
+      uint32_t step = 0;       // accumulations issued
+      uint32_t ka[2] = {0, 0}; // activations taken per tile slot
+      for (int t = t_first; t < p.tiles; t += t_step) {
+        const int n = t + 1 < p.tiles ? p.per : 1;   // tiles of this turn
+        for (int layer = 0; layer < 3; ++layer) {
+          for (int k = 0; k < n; ++k, ++step) {
+            if (!mbar_wait(&aready[k], ka[k] & 1u, 53)) goto done;
+            ++ka[k];
+            // the previous accumulation is in the epilogue's registers
+            if (step > 0 && !mbar_wait(dfree, (step - 1) & 1u, 54)) goto done;
             tc_fence_after();
-            mma_f16_ts(tmem + T_D, tmem + T_A + 8 * ks, r0 + (uint64_t)((s * SLICE_BYTES) >> 4), idesc,
-                           ks ? 1u : 0u);
-            mma_commit(&empty[s]);
+            const uint32_t a = tmem + T_A + (uint32_t)(k * T_A_TILE);
+            if (layer == 0) {
+              mma_f16_ts(tmem + T_D, a, w1d, idesc, 0u);
+            } else {
+              int s = s0;
+              uint32_t ph = ph0;
+#pragma unroll
+              for (int c = 0; c < LAYER_CHUNKS; ++c) {
+                if (k == 0) {
+                  if (!mbar_wait(&full[s], ph, 55)) goto done;
+                }
+                const uint64_t w = r0 + (uint64_t)((uint32_t)(s * CHUNK_BYTES) >> 4);
+#pragma unroll
+                for (int i = 0; i < CHUNK; ++i)
+                  mma_f16_ts(tmem + T_D, a + 8 * (CHUNK * c + i), w + (uint64_t)(i * (SLICE_BYTES >> 4)), idesc,
+                             c + i ? 1u : 0u);
+                if (k == n - 1) mma_commit(&empty[s]);
+                if (++s == RING) {
+                  s = 0;
+                  ph ^= 1u;
+                }
+              }
+              if (k == n - 1) {
+                s0 = s;
+                ph0 = ph;
+              }
+            }
+            mma_commit(dfull);
           }
-          mma_commit(dfull);
-          ++k;
         }
       }
     }
@@ -185,84 +257,104 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(InferParams p) {
     if (!mbar_wait(cready, 0, 56)) goto done;
     const float* mean = hdr;
     const float* inv_std = hdr + 16;
-    const float out_scale = hdr[32], out_shift = hdr[33], b4 = hdr[34];
-    int k = 0;
-    // this thread's 4 input features of a tile (features 4 fq .. 4 fq + 3);
-    // the next tile's are loaded while the current one runs
-    auto load_x = [&](int64_t tile) {
-      const int64_t qq = tile * QT + row;
-      if (tile < p.tiles && qq < p.batch) return __ldg(reinterpret_cast<const float4*>(p.x + qq * MLP_IN + 4 * fq));
-      return make_float4(mean[4 * fq], mean[4 * fq + 1], mean[4 * fq + 2], mean[4 * fq + 3]);
-    };
-    float4 xv = load_x(group);
-    for (int64_t t = group; t < p.tiles; t += groups) {
-      const int64_t q = t * QT + row;
-      {
-        const float4 v = xv;
-        xv = load_x(t + groups);
-        const int f = 4 * fq;
-        uint32_t pk[2];
-        pk[0] = pack_bf16((v.x - mean[f]) * inv_std[f], (v.y - mean[f + 1]) * inv_std[f + 1]);
-        pk[1] = pack_bf16((v.z - mean[f + 2]) * inv_std[f + 2], (v.w - mean[f + 3]) * inv_std[f + 3]);
-        tmem_st2(tmem + lane_off + T_A + 2 * fq, pk);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(aready);
+    // this thread's 4 input features of a tile (features 4 fq .. 4 fq + 3) into
+    // the tile slot's activations; `turn` is the tile's
+    auto put_inputs = [&](int tile, int k, uint32_t turn) -> bool {
+      const int f = 4 * fq;
+      if (!mbar_wait(&xfull[k], turn & 1u, 63)) return false;
+      float4 v = make_float4(mean[f], mean[f + 1], mean[f + 2], mean[f + 3]);
+      if ((int64_t)tile * QT + row < p.batch)
+        v = *reinterpret_cast<const float4*>(smem + SM_X_OFF + k * X_BYTES + (row * MLP_IN + f) * 4);
+      uint32_t pk[2];
+      pk[0] = pack_bf16((v.x - mean[f]) * inv_std[f], (v.y - mean[f + 1]) * inv_std[f + 1]);
+      pk[1] = pack_bf16((v.z - mean[f + 2]) * inv_std[f + 2], (v.w - mean[f + 3]) * inv_std[f + 3]);
+      tmem_st2(tmem + lane_off + T_A + k * T_A_TILE + 2 * fq, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&aready[k]);
+        mbar_arrive(&xempty[k]);
       }
-      float acc_y = 0.f;
+      return true;
+    };
+    for (int k = 0; k < p.per; ++k)
+      if (t_first + k < p.tiles && !put_inputs(t_first + k, k, 0)) goto done;
+    uint32_t step = 0, turn = 0;
+    for (int t = t_first; t < p.tiles; t += t_step, ++turn) {
+      const int n = t + 1 < p.tiles ? p.per : 1;
       for (int layer = 0; layer < 3; ++layer) {
-        if (!mbar_wait(dfull, (uint32_t)(k & 1), 57)) goto done;
-        tc_fence_after();
-        ++k;
-        const float* bias = vec + layer * MLP_H + 64 * fq;
-        const float* w4 = vec + 3 * MLP_H + 64 * fq;
+        const float* bias = half_b + layer * MLP_H + 64 * fq;
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-          uint32_t r[32];
-          tmem_ld32(tmem + lane_off + T_D + 64 * fq + 32 * c, r);
+        for (int k = 0; k < n; ++k, ++step) {
+          if (!mbar_wait(dfull, step & 1u, 57)) goto done;
+          tc_fence_after();
+          uint32_t r[2][32];
+          tmem_ld32(tmem + lane_off + T_D + 64 * fq, r[0]);
+          tmem_ld32(tmem + lane_off + T_D + 64 * fq + 32, r[1]);
           tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dfree);
           if (layer < 2) {
-            uint32_t pk[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float2 bb = *reinterpret_cast<const float2*>(bias + 32 * c + 2 * j);
-              pk[j] = pack_bf16(silu_fast(__uint_as_float(r[2 * j]) + bb.x), silu_fast(__uint_as_float(r[2 * j + 1]) + bb.y));
+            for (int c = 0; c < 8; ++c) {
+              uint32_t pk[4];
+#pragma unroll
+              for (int j = 0; j < 4; j += 2) {
+                const uint32_t* z = r[c >> 2] + 8 * (c & 3) + 2 * j;
+                const float4 bb = *reinterpret_cast<const float4*>(bias + 8 * c + 2 * j);
+                pk[j] = silu_pair(z[0], z[1], bb.x, bb.y);
+                pk[j + 1] = silu_pair(z[2], z[3], bb.z, bb.w);
+              }
+              tmem_st4(tmem + lane_off + T_A + k * T_A_TILE + 32 * fq + 4 * c, pk);
             }
-            tmem_st16(tmem + lane_off + T_A + 32 * fq + 16 * c, pk);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&aready[k]);
           } else {
+            const float* w4 = vec + 3 * MLP_H + 64 * fq;
+            float acc_y = 0.f;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float a = __bfloat162float(__float2bfloat16_rn(silu_fast(__uint_as_float(r[j]) + bias[32 * c + j])));
-              acc_y = fmaf(a, w4[32 * c + j], acc_y);
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int j = 0; j < 32; j += 4) {
+                const float4 bb = *reinterpret_cast<const float4*>(bias + 32 * c + j);
+                const float4 ww = *reinterpret_cast<const float4*>(w4 + 32 * c + j);
+                const uint32_t lo = silu_pair(r[c][j], r[c][j + 1], bb.x, bb.y);
+                const uint32_t hi = silu_pair(r[c][j + 2], r[c][j + 3], bb.z, bb.w);
+                acc_y = fmaf(__uint_as_float(lo << 16), ww.x, acc_y);
+                acc_y = fmaf(__uint_as_float(lo & 0xffff0000u), ww.y, acc_y);
+                acc_y = fmaf(__uint_as_float(hi << 16), ww.z, acc_y);
+                acc_y = fmaf(__uint_as_float(hi & 0xffff0000u), ww.w, acc_y);
+              }
+            // this tile slot's MMAs are done: the next turn's inputs
+            if (t + t_step + k < p.tiles && !put_inputs(t + t_step + k, k, turn + 1)) goto done;
+            // combine the four feature quarters of each query's dot product
+            float* ys = ysum + k * 3 * QT;
+            if (fq != 0) {
+              ys[(fq - 1) * QT + row] = acc_y;
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&ycomb[k]);
+            } else {
+              if (!mbar_wait(&ycomb[k], turn & 1u, 58)) goto done;
+              const float v = acc_y + ys[row] + ys[QT + row] + ys[2 * QT + row] + hdr[34];
+              const int64_t q = (int64_t)(t + k) * QT + row;
+              if (q < p.batch) p.y[(int64_t)member * p.batch + q] = fmaf(v, hdr[32], hdr[33]);
             }
           }
         }
-        if (layer < 2) {
-          tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(aready);
-        }
-      }
-      // combine the four feature quarters of each query's dot product
-      tc_fence_before();
-      if (fq != 0) {
-        ysum[(fq - 1) * QT + row] = acc_y;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(ycomb);
-      } else {
-        const int kt = (int)((t - group) / groups);
-        if (!mbar_wait(ycomb, (uint32_t)(kt & 1), 58)) goto done;
-        const float v = acc_y + ysum[row] + ysum[QT + row] + ysum[2 * QT + row] + b4;
-        if (q < p.batch) p.y[(int64_t)member * p.batch + q] = fmaf(v, out_scale, out_shift);
       }
     }
   }
 done:
   if (warp == PROD_WARP && lane == 0) {
-    for (int64_t i = imax<int64_t>(0, n_ring_copies - RING); i < n_ring_copies; ++i)
-      mbar_wait(&full[i % RING], (uint32_t)((i / RING) & 1), 59);
+    for (unsigned i = n_ring_copies > RING ? n_ring_copies - RING : 0u; i < n_ring_copies; ++i)
+      mbar_wait(&full[i % RING], (i / RING) & 1u, 59);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (n_x_copies[k]) mbar_wait(&xfull[k], (n_x_copies[k] - 1u) & 1u, 64);
     if (n_const_copies) mbar_wait(cready, 0, 60);
   }
   if (warp == MMA_WARP && lane == 0) {
@@ -371,9 +463,10 @@ int launch_infer(const void* packed, int members, const float* x, int64_t batch,
   p.x = x;
   p.batch = batch;
   p.y = y;
-  p.tiles = (batch + QT - 1) / QT;
+  p.tiles = (int)((batch + QT - 1) / QT);
   const int sms = sm_count();
-  int groups = (int)imax<int64_t>(1, imin<int64_t>(sms / members, p.tiles));
+  int groups = imax(1, imin(sms / members, p.tiles));
+  p.per = p.tiles > groups ? 2 : 1;
   cudaError_t e = cudaFuncSetAttribute(mlp_infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_status(e);
   TimerScope ts(K_MLP_INFER, (double)batch * members, s);
