@@ -383,6 +383,22 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// One lane of a converged warp, the same one each time.  MMAs are issued under
+// this and not under `lane == 0`: with elect.sync the compiler knows that one
+// thread runs the branch and keeps descriptors in uniform registers.  Under
+// `lane == 0` one thread issued an MMA every 118 cycles whatever its size (95
+// unrolled), under elect_one() every 9.7 at N = 16 and at the tensor core's
+// own rate, 32, at N = 64 (M = 128, K = 16, A in tensor memory).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T, kind::f16 (bf16 inputs, FP32 accumulate).
 __device__ __forceinline__ void mma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                             uint32_t idesc, uint32_t accumulate) {

@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_infer_kernel(InferParams p) {
       }
     }
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = idesc_bf16_f32(QT, MLP_H);
       const uint64_t w1d = smem_desc_kmajor(smem_u32(smem + W1_OFF), 128, 8 * 32);
       const uint64_t r0 = smem_desc_kmajor(smem_u32(ring), 128, 8 * 32);
@@ -357,7 +357,7 @@ done:
       if (n_x_copies[k]) mbar_wait(&xfull[k], (n_x_copies[k] - 1u) & 1u, 64);
     if (n_const_copies) mbar_wait(cready, 0, 60);
   }
-  if (warp == MMA_WARP && lane == 0) {
+  if (warp == MMA_WARP && elect_one()) {
     mma_commit(drain);
     mbar_wait(drain, 0, 61);
   }

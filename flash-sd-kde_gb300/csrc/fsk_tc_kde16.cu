@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
           if (!__all_sync(0xffffffffu, mbar_wait(&tempty[b * NQT + a], ((g >> 1) & 1u) ^ 1u, 5))) goto done;
           tc_fence_after();
           const uint64_t so = (uint64_t)(s * (KB_STAGE_BYTES >> 4));
-          if (lane == 0) {
+          if (elect_one()) {
             if (SINGLE)
               mma_s_tile_single(d0 + b * (uint32_t)(NQT * KNT), a_h, b_h0 + so, idesc);
             else
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
             ph ^= 1u;
           }
         }
-        if (lane == 0) mma_commit(qempty);
+        if (elect_one()) mma_commit(qempty);
         __syncwarp();
       }
     }
@@ -359,7 +359,7 @@ done:
       mbar_wait(&full[i % NS], (i / NS) & 1u, 7);
     if (n_query_copies > 0) mbar_wait(qready, (n_query_copies - 1) & 1u, 8);
   }
-  if ((warp == MMA_WARP || warp == MMA_WARP2) && lane == 0) {
+  if ((warp == MMA_WARP || warp == MMA_WARP2) && elect_one()) {
     mma_commit(drain);   // one arrival per issuing thread, when its MMAs have finished
     mbar_wait(drain, 0, 9);
   }

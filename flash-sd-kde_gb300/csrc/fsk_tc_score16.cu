@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
           const uint64_t b_h = dh0 + so;
           // three-part product, small terms first (the order of mma_s_tile)
           const uint64_t b_m = dm0 + so, b_l = dl0 + so;
-          if (lane == 0) {
+          if (elect_one()) {
             mma_f16_ts(d, a_h + 16u, b_m, idesc_s, 0u);                    // mid . mid
             mma_f16_ts(d, a_h, b_l, idesc_s, 1u);                          // hi . lo
             mma_f16_ts(d, a_h + 24u, b_h, idesc_s, 1u);                    // lo . hi
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
           const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
           const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT + part * 16);
           const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS + part * WN);
-          if (lane == 0) {
+          if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < NT / 16; ++ks) {
               // data columns 16 ks .. +15: column half ks/2; weights hi at +0, lo at +16
@@ -599,7 +599,7 @@ done:
       mbar_wait(&full[i % SNS], (uint32_t)((i / SNS) & 1), 32);
     if (n_query_copies > 0) mbar_wait(qready, (uint32_t)((n_query_copies - 1) & 1), 33);
   }
-  if ((warp == S_MMA_WARP || warp == S_MMA_WARP2 || warp >= W_MMA_WARP) && lane == 0) {
+  if ((warp == S_MMA_WARP || warp == S_MMA_WARP2 || warp >= W_MMA_WARP) && elect_one()) {
     mma_commit(drain);   // one arrival per issuing thread, when its MMAs have finished
     mbar_wait(drain, 0, 34);
   }
