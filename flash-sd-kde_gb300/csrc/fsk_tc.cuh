@@ -46,11 +46,13 @@ constexpr int MMA_WARP = EPI_WARPS + 1;   // owns TMEM, issues the MMAs of query
 constexpr int MMA_WARP2 = EPI_WARPS + 2;  // issues the MMAs of query tile 1
 constexpr int MMA_ISSUERS = 2;
 constexpr int THREADS = (EPI_WARPS + 3) * 32;
-constexpr int TMEM_COLS = 2 * NQT * KNT; // double-buffered accumulators
+constexpr int NACC = 3;                  // KDE: accumulators, taken in turn by the query tiles
+constexpr int T_KA = NACC * KNT;         // KDE: query operand in tensor memory, [NQT][hi 16 | mid 8 | lo 8]
+constexpr int TMEM_COLS = 512;
 constexpr int K_BAR_OFFSET = A_BYTES + NS * KB_STAGE_BYTES;
 // KDE: one 64-byte slot per epilogue thread for its query's FP32 row (read by
 // the exact recompute; each thread writes its own slot at the start of a unit)
-constexpr int K_QX_OFFSET = K_BAR_OFFSET + 256;
+constexpr int K_QX_OFFSET = K_BAR_OFFSET + 512;
 constexpr int SMEM_BYTES = K_QX_OFFSET + EPI_WARPS * 32 * FSK_D * 4;
 // A term is recomputed exactly when its 32-column chunk holds more than this
 // fraction of the running sum of its query (the chunk included).  With the
@@ -62,7 +64,9 @@ constexpr float NEAR_FRACTION = 1.0f / 8.0f;
 constexpr float PHI_LOG2_SCALE = 15.0f;   // score weights are phi * 2^15
 constexpr float FP16_TARGET = 8192.0f;  // largest operand magnitude aimed for
 
-static_assert(TMEM_COLS == 512, "TMEM budget");
+static_assert(T_KA + NQT * 32 <= TMEM_COLS, "TMEM budget");
+static_assert(NQT == 2 && NACC == 3, "the accumulator's predecessor and the depth of its barriers");
+static_assert((2 * NS + 8 * NQT + 2 + NQT + 1) * 8 + 4 <= 512, "barrier area");
 static_assert(KB_STAGE_BYTES % 16 == 0 && A_BYTES % 16 == 0, "bulk copy granularity");
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 

@@ -37,14 +37,21 @@
 //   warp 16 : producer - bulk (TMA) copies of query images per unit and of
 //             data-tile images (128 points) per stage into shared memory
 //             (mbarrier tx).
-//   warps 17, 18 : issue the MMAs of query tiles 0 and 1 (one lane each);
-//             warp 17 owns TMEM (512 columns).
+//   warps 17, 18 : copy the query operand of tiles 0 and 1 to tensor memory
+//             once per segment and issue their MMAs; warp 17 owns TMEM.
 //   warps 0-15: epilogue; warp w reads TMEM lanes 32*(w%4).. and columns
 //             64*((w/4)%2).. of query tile w/8.
 // A work unit (segment, see WorkLine) is 256 queries (two M=128 tiles) x a run
-// of data tiles; TMEM holds two accumulator buffers x two query tiles x 128
-// columns.  Each query's sum is kept as two column halves by two threads and
-// written as two rows of (value, error) pairs per segment.
+// of data tiles.  TMEM holds three accumulators of 128 columns, taken in turn
+// by the two query tiles, and the query operands (hi | mid | lo, 32 columns a
+// tile).  With both operands in shared memory an M=128, N=128, K=16 MMA takes
+// ~100 cycles (44 of them for A, whatever N is), with A in tensor memory 64:
+// four double-buffered accumulators and A in shared memory took 11.95 ms at
+// n = m = 262144, this 11.5 (2^20: 184.3, 177.7).  Now the exp pipe is busy
+// 62 % of the time, the tensor core 54 %, issue slots 55 %; the rest is the
+// latency of waits, TMEM loads and add chains that 16 warps of 96 registers
+// cannot hide.  Each query's sum is kept as two column halves by two threads
+// and written as two rows of (value, error) pairs per segment.
 #include <cuda_fp16.h>
 
 #include "fsk_kernels.cuh"
@@ -75,12 +82,16 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + K_BAR_OFFSET);
   uint64_t* full = bars;                 // [NS] data stage loaded
   uint64_t* empty = bars + NS;           // [NS] data stage consumed (MMAs + epilogue)
-  uint64_t* tfull = bars + 2 * NS;       // [2 buffers][NQT] accumulator written
-  uint64_t* tempty = bars + 2 * NS + 4;  // [2 buffers][NQT] accumulator drained
-  uint64_t* qready = bars + 2 * NS + 8;  // query images loaded
-  uint64_t* qempty = bars + 2 * NS + 9;  // query images no longer read by the MMAs
-  uint64_t* drain = bars + 2 * NS + 10;  // all MMAs of this CTA finished (exit path)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NS + 11);
+  // [NQT][4], by the tile's number modulo 4: one phase of a barrier must not
+  // pass before every waiter of the phase before has seen it, and an
+  // accumulator's three predecessors run up to two tiles ahead of it
+  uint64_t* tfull = bars + 2 * NS;       // accumulator written
+  uint64_t* tempty = tfull + 4 * NQT;    // accumulator drained
+  uint64_t* qready = tempty + 4 * NQT;   // query images loaded
+  uint64_t* qempty = qready + 1;         // query images copied to tensor memory
+  uint64_t* sdone = qready + 2;          // [NQT] a query tile's MMAs of the segment finished
+  uint64_t* drain = sdone + NQT;         // all MMAs of this CTA finished (exit path)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   uint32_t n_stage_copies = 0, n_query_copies = 0;   // producer: bulk copies issued
 
   const int warp = threadIdx.x >> 5;
@@ -91,11 +102,12 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], MMA_ISSUERS + EPI_WARPS);
     }
-    for (int i = 0; i < 2 * NQT; ++i) {
+    for (int i = 0; i < 4 * NQT; ++i) {
       mbar_init(&tfull[i], 1);
       mbar_init(&tempty[i], EPI_WARPS / NQT);
     }
     mbar_init(qready, 1);
+    for (int i = 0; i < NQT; ++i) mbar_init(&sdone[i], 1);
     mbar_init(qempty, MMA_ISSUERS);
     mbar_init(drain, MMA_ISSUERS);
     fence_barrier_init();
@@ -143,11 +155,14 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       }
     }
   } else if (warp == MMA_WARP || warp == MMA_WARP2) {
-    // Two issuing threads, one query tile each, with their own accumulator
-    // barriers: a tile's MMAs wait only for the 8 epilogue warps reading that
-    // tile.  The per-tile path is kept to the waits, the MMAs and the commits
-    // (descriptors of stage s = stage 0 + s * 1 KiB in the 16-byte address
-    // field).  The whole warp runs the loop; lane 0 issues and commits.
+    // Two issuing warps, one query tile each.  Accumulation u = 2 g + a (data
+    // tile g of this CTA's run, query tile a) goes to accumulator u % NACC, so
+    // the tiles take the accumulators in turn and a tile's MMAs wait only for
+    // the 8 warps reading the one before them there.  The query operand is
+    // copied to tensor memory once per segment.  u - NACC is tile g - 2 + a of
+    // the other query tile.  The per-tile path is kept to
+    // the waits, the MMAs and the commits (descriptors of stage s = stage 0 +
+    // s * KB_STAGE_BYTES in the 16-byte address field).
     {
       const uint32_t idesc = idesc_f16_f32(QT, KNT);
       const int a = (warp == MMA_WARP) ? 0 : 1;
@@ -159,36 +174,55 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       const uint64_t b_h0 = smem_desc_kmajor(bs0, 128, 8 * H_ROW_BYTES);
       const uint64_t b_m0 = smem_desc_kmajor(bs0 + KB_M_OFFSET, 128, 8 * L_ROW_BYTES);
       const uint64_t b_l0 = smem_desc_kmajor(bs0 + KB_L_OFFSET, 128, 8 * L_ROW_BYTES);
-      const uint32_t d0 = tmem_base + (uint32_t)(a * KNT);
-      uint32_t g = 0, k = 0, ph = 0;
+      const uint32_t ta = tmem_base + (uint32_t)(T_KA + a * 32);   // hi: features | bias; mid at +16, lo at +24
+      uint32_t k = 0, ph = 0;
       int s = 0;
+      int g = 0;            // data tile
+      int acc = a;          // u % NACC
       for (int done_tiles = 0;; ++k) {
         const int nt = next_segment(p.line, done_tiles).count;
         if (nt == 0) break;
         done_tiles += nt;
         if (!__all_sync(0xffffffffu, mbar_wait(qready, k & 1u, 3))) goto done;
-        for (int i = 0; i < nt; ++i, ++g) {
-          const uint32_t b = g & 1u;
+        // the previous segment's MMAs have read its operand
+        if (k > 0 && !__all_sync(0xffffffffu, mbar_wait(&sdone[a], (k - 1) & 1u, 10))) goto done;
+        tc_fence_after();
+        if (elect_one()) {
+          tmem_cp_128x256b(ta, a_h);
+          tmem_cp_128x256b(ta + 8u, a_h + (256 >> 4));
+          if (!SINGLE) {
+            tmem_cp_128x256b(ta + 16u, a_m);
+            tmem_cp_128x256b(ta + 24u, a_l);
+          }
+          mma_commit(qempty);
+        }
+        __syncwarp();
+        for (int i = 0; i < nt; ++i) {
           if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, 4))) goto done;
-          if (!__all_sync(0xffffffffu, mbar_wait(&tempty[b * NQT + a], ((g >> 1) & 1u) ^ 1u, 5))) goto done;
+          const int prev = g - 2 + a;
+          if (prev >= 0 && !__all_sync(0xffffffffu, mbar_wait(&tempty[(1 - a) * 4 + (prev & 3)], (uint32_t)(prev >> 2) & 1u, 5)))
+            goto done;
           tc_fence_after();
           const uint64_t so = (uint64_t)(s * (KB_STAGE_BYTES >> 4));
           if (elect_one()) {
+            const uint32_t d = tmem_base + (uint32_t)(acc * KNT);
             if (SINGLE)
-              mma_s_tile_single(d0 + b * (uint32_t)(NQT * KNT), a_h, b_h0 + so, idesc);
+              mma_s_tile_single(d, ta, b_h0 + so, idesc);
             else
-              mma_s_tile(d0 + b * (uint32_t)(NQT * KNT), a_h, a_m, a_l, b_h0 + so, b_m0 + so, b_l0 + so, idesc);
-            mma_commit(&tfull[b * NQT + a]);
+              mma_s_tile(d, ta, b_h0 + so, b_m0 + so, b_l0 + so, idesc);
+            mma_commit(&tfull[a * 4 + (g & 3)]);
             mma_commit(&empty[s]);
+            if (i == nt - 1) mma_commit(&sdone[a]);
           }
           __syncwarp();
+          ++g;
+          acc += NQT;
+          if (acc >= NACC) acc -= NACC;
           if (++s == NS) {
             s = 0;
             ph ^= 1u;
           }
         }
-        if (elect_one()) mma_commit(qempty);
-        __syncwarp();
       }
     }
   } else {
@@ -202,7 +236,8 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
     // slot float4 kk of thread t at [kk][t]: a warp's 16-byte accesses are contiguous
     float4* qslot = reinterpret_cast<float4*>(smem_raw + K_QX_OFFSET) + (warp * 32 + lane);
     constexpr int QS_STRIDE = EPI_WARPS * 32;
-    uint32_t g = 0;
+    int g = 0;     // data tile
+    int ab = qt;   // its accumulator, (2 g + qt) % NACC
     int s = 0;
     const int last_t = (int)p.line.n_tiles - 1;
     // valid columns of this thread's half of the last (possibly ragged) data
@@ -228,10 +263,9 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       const int last_i = last_t - sg.t0;
       const int nt = sg.count;
       for (int i = 0; i < nt; ++i, ++g) {
-        const uint32_t b = g & 1u;
         const int valid = i == last_i ? last_valid : KNT / 2;   // may be <= 0 on the last tile
         // (a timed-out wait ends the whole warp: it must stay converged)
-        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[b * NQT + qt], (g >> 1) & 1u, 6))) goto done;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[qt * 4 + (g & 3)], (uint32_t)(g >> 2) & 1u, 6))) goto done;
         tc_fence_after();
         const uint8_t* xrows = sB + s * KB_STAGE_BYTES + KB_X_OFFSET + half * (KNT / 2) * (FSK_D * 4);
         float tsum = 0.f;
@@ -239,13 +273,15 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         // accumulator buffer goes back to the MMA issuer as early as possible.
         uint32_t ra[32], rb[32];
         {
-          const uint32_t col = tmem_base + lane_off + b * (uint32_t)(NQT * KNT) + (uint32_t)(qt * KNT + half * (KNT / 2));
+          const uint32_t col = tmem_base + lane_off + (uint32_t)(ab * KNT + half * (KNT / 2));
           tmem_ld32(col, ra);
           tmem_ld32(col + 32u, rb);
           tmem_ld_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[b * NQT + qt]);
+          if (lane == 0) mbar_arrive(&tempty[qt * 4 + (g & 3)]);
+          ab += NQT;
+          if (ab >= NACC) ab -= NACC;
         }
         auto chunk = [&](const uint32_t (&r)[32], const int c) {
             float e[32];

@@ -25,26 +25,27 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uin
 
 // D = a2 for one 128-query tile x one data tile (smallest products first, so
 // the large hi.hi and bias terms meet last, then the bias K step).
-// a_h / b_h: H images (hi | bias), a_m / b_m: mid, a_l / b_l: lo images.
+// a: the query operand in tensor memory, hi features at +0, bias at +8, mid at
+// +16, lo at +24; b_h: H image (hi | bias), b_m: mid, b_l: lo image.
 // The six products whose error terms exceed ~2^-33, then the bias: seven MMAs.
-__device__ __forceinline__ void mma_s_tile(uint32_t d, uint64_t a_h, uint64_t a_m, uint64_t a_l, uint64_t b_h,
-                                           uint64_t b_m, uint64_t b_l, uint32_t idesc) {
+__device__ __forceinline__ void mma_s_tile(uint32_t d, uint32_t a, uint64_t b_h, uint64_t b_m, uint64_t b_l,
+                                           uint32_t idesc) {
   const uint64_t bias = 256 >> 4;   // bias K step: +256 B in the start-address field
-  mma_f16_ss(d, a_m, b_m, idesc, 0u);       // mid . mid
-  mma_f16_ss(d, a_h, b_l, idesc, 1u);       // hi . lo
-  mma_f16_ss(d, a_l, b_h, idesc, 1u);       // lo . hi
-  mma_f16_ss(d, a_h, b_m, idesc, 1u);       // hi . mid
-  mma_f16_ss(d, a_m, b_h, idesc, 1u);       // mid . hi
-  mma_f16_ss(d, a_h, b_h, idesc, 1u);       // hi . hi
-  mma_f16_ss(d, a_h + bias, b_h + bias, idesc, 1u);   // beta_j + alpha_i
+  mma_f16_ts(d, a + 16u, b_m, idesc, 0u);        // mid . mid
+  mma_f16_ts(d, a, b_l, idesc, 1u);              // hi . lo
+  mma_f16_ts(d, a + 24u, b_h, idesc, 1u);        // lo . hi
+  mma_f16_ts(d, a, b_m, idesc, 1u);              // hi . mid
+  mma_f16_ts(d, a + 16u, b_h, idesc, 1u);        // mid . hi
+  mma_f16_ts(d, a, b_h, idesc, 1u);              // hi . hi
+  mma_f16_ts(d, a + 8u, b_h + bias, idesc, 1u);  // beta_j + alpha_i
 }
 
 // Single-pass rung: hi.hi cross product and the bias K step (two MMAs); the
 // norms in the bias columns keep their three-part precision.
-__device__ __forceinline__ void mma_s_tile_single(uint32_t d, uint64_t a_h, uint64_t b_h, uint32_t idesc) {
+__device__ __forceinline__ void mma_s_tile_single(uint32_t d, uint32_t a, uint64_t b_h, uint32_t idesc) {
   const uint64_t bias = 256 >> 4;
-  mma_f16_ss(d, a_h, b_h, idesc, 0u);
-  mma_f16_ss(d, a_h + bias, b_h + bias, idesc, 1u);
+  mma_f16_ts(d, a, b_h, idesc, 0u);
+  mma_f16_ts(d, a + 8u, b_h + bias, idesc, 1u);
 }
 
 // sum_k (q_k - x_k)^2 from the original FP32 coordinates of data row r.
