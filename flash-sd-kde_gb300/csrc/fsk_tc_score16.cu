@@ -14,11 +14,9 @@
 //    operand images of the KDE kernel (fsk_tc_kde16.cu): seven tcgen05.mma
 //    per query tile, the query operand (hi | mid | lo rows) read from tensor
 //    memory, where the epilogue warps copy it at the start of each unit (an
-//    M=128, K=16 MMA with both operands in shared memory costs ~48 cycles,
-//    bound by the operand reads; with A in tensor memory it runs at the
-//    math rate when enough threads issue).  The +15 rides in the query's
-//    bias term, so 2^S = phi * 2^15 and the weights keep fp16 normal range
-//    down to phi ~ 2^-29.
+//    M=128, K=16 MMA with both operands in shared memory costs ~44 cycles
+//    more).  The +15 rides in the query's bias term, so 2^S = phi * 2^15 and
+//    the weights keep fp16 normal range down to phi ~ 2^-29.
 //  * Epilogue: tcgen05.ld, ex2.approx, pdf chunk sums, the exact near-pair
 //    recompute of the KDE kernel (the recomputed value also replaces the
 //    approximate one in the weights), then the weights are split into fp16
@@ -28,21 +26,29 @@
 //    (weights, M=128 x K=16 per step) read from tensor memory and the B
 //    operand ((x_j - mu) 2^ew as fp16 hi and lo rows, K-major over the data
 //    points) from the data stage, FP32 accumulation over a group of tiles
-//    (score_group), then added into compensated FP32 sums.  Four issuing threads,
-//    one per (query tile, weight part), each with its own accumulator: a
-//    single thread issues an M=128, K=16, N=32 MMA every ~46 cycles, four
-//    reach the tensor core's math rate.
+//    (score_group), then added into compensated FP32 sums.
 //
-// Pipeline (one persistent CTA per SM, 23 warps):
+// Pipeline (one persistent CTA per SM, 20 warps of 96 registers):
 //   warp 16 : producer (bulk copies of query images per unit, data stages).
-//   warps 17, 18 : issue S for query tiles 0 and 1 (one lane each), up to
-//             NBUF tiles ahead of W; warp 17 owns TMEM.
-//   warps 19-22 : issue the weighted-sum MMAs of (query tile, weight part)
-//             (0, hi), (0, lo), (1, hi), (1, lo).
+//   warp 17 : issues S for both query tiles, up to NBUF tiles ahead of W;
+//             owns TMEM.
+//   warps 18, 19 : issue the weighted-sum MMAs of query tiles 0 and 1.
 //   warps 0-15: epilogue; warp w: query tile w/8, data-column half (w/4)&1,
 //             TMEM lane quarter w&3.  The two column halves of a row keep
 //             separate pdf partials (two rows per segment) and
 //             read disjoint halves of the weighted-sum features.
+//
+// What bounds it: the epilogue's instructions.  Per tile a warp runs ~250 of
+// them for 32 columns; issue slots are 70 % busy, exp pipe 36 %, tensor core
+// 45 %.  So the tile loop is kept short: rare work (scaled sums, ragged and
+// diagonal columns in one block, near pairs, group read-out) is marked
+// unlikely and stays behind the straight path, and the weights are stored
+// before the sums, whose latency covers that of the stores.  n = 262144:
+// 24.1 ms with seven issuing warps of 80 registers and separate ragged and
+// diagonal blocks, 20.6 this way (2^20: 381, 328).  Tried and slower: eight
+// warps of 64 columns (28.6 ms), S and weights in separate columns with one
+// buffer each (25.9), the rare blocks as calls (21.6-22.3), the next tile's S
+// loaded ahead (25.0, spills).
 // TMEM: A operands [2 query tiles][hi 16 | mid 8 | lo 8]  (columns 0-63)
 //       | S / weights [NBUF buffers][2 query tiles][64]  (64-319)
 //       | W [2 group parities][2 query tiles][hi part 32 | lo part 16]  (320-511).
@@ -62,11 +68,10 @@ constexpr int SNS = 4;                                     // data stages
 constexpr int S_A_BYTES = SNQT * A_TILE_BYTES;             // 32 KB
 constexpr int S_EPI_WARPS = 8 * SNQT;
 constexpr int S_PRODUCER_WARP = S_EPI_WARPS;
-constexpr int S_MMA_WARP = S_EPI_WARPS + 1;     // issues the S MMAs of query tile 0, owns TMEM
-constexpr int S_MMA_WARP2 = S_EPI_WARPS + 2;    // issues the S MMAs of query tile 1
-constexpr int W_MMA_WARP = S_EPI_WARPS + 3;     // first of the W_ISSUERS weighted-sum issuers
-constexpr int W_ISSUERS = 2 * SNQT;             // (query tile, weight part hi / lo)
-constexpr int S_THREADS = (S_EPI_WARPS + 3 + W_ISSUERS) * 32;
+constexpr int S_MMA_WARP = S_EPI_WARPS + 1;     // issues the S MMAs, owns TMEM
+constexpr int W_MMA_WARP = S_EPI_WARPS + 2;     // first of the W_ISSUERS weighted-sum issuers
+constexpr int W_ISSUERS = SNQT;                 // one per query tile
+constexpr int S_THREADS = (S_EPI_WARPS + 2 + W_ISSUERS) * 32;
 constexpr int NBUF = 2;                                    // S / weight buffers in TMEM
 constexpr int WN = 2 * FSK_D;                              // W MMA N, hi weights: X_hi and X_lo rows
 constexpr int WN_LO = FSK_D;                               // W MMA N, lo weights: X_hi rows
@@ -142,7 +147,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
   // [NBUF][SNQT] weights stored.  One barrier per buffer and query tile: a
   // buffer's barrier cannot complete again before its weights are consumed.
   uint64_t* pready = tfull + NBUF * SNQT;
-  uint64_t* sfree = pready + NBUF * SNQT;         // [NBUF][SNQT] weights read by both W parts
+  uint64_t* sfree = pready + NBUF * SNQT;         // [NBUF][SNQT] weights read by the W MMAs
   uint64_t* wfull = sfree + NBUF * SNQT;          // [2 parities][SNQT] W group accumulated
   uint64_t* wempty = wfull + 2 * SNQT;            // [2 parities][SNQT] W group read
   uint64_t* aready = wempty + 2 * SNQT;           // [SNQT] unit's A operand in TMEM
@@ -166,16 +171,16 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
     for (int i = 0; i < NBUF * SNQT; ++i) {
       mbar_init(&tfull[i], 1);
       mbar_init(&pready[i], 8);
-      mbar_init(&sfree[i], 2);
+      mbar_init(&sfree[i], 1);
     }
     for (int i = 0; i < 2 * SNQT; ++i) {
-      mbar_init(&wfull[i], 2);
+      mbar_init(&wfull[i], 1);
       mbar_init(&wempty[i], 8);
     }
     for (int a = 0; a < SNQT; ++a) mbar_init(&aready[a], 8);
     mbar_init(qready, 1);
     mbar_init(qempty, S_EPI_WARPS);
-    mbar_init(drain, 2 + W_ISSUERS);
+    mbar_init(drain, 1 + W_ISSUERS);
     mbar_init(cready, S_EPI_WARPS);
     fence_barrier_init();
   }
@@ -223,17 +228,15 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         }
       }
     }
-  } else if (warp == S_MMA_WARP || warp == S_MMA_WARP2) {
-    // S(g) of one query tile for every tile, up to NBUF tiles ahead of W:
-    // buffer g % NBUF is reused once both W parts of tile g - NBUF have read
-    // its weights (sfree).  S and W are issued by different threads because
+  } else if (warp == S_MMA_WARP) {
+    // S(g) of both query tiles for every tile, up to NBUF tiles ahead of W:
+    // buffer g % NBUF is reused once the W MMAs of tile g - NBUF have read its
+    // weights (sfree).  S and W are issued by different threads because
     // tcgen05.commit tracks every earlier MMA of its thread.  The whole warp
-    // runs the loop (warp-uniform values stay in uniform registers); lane 0
+    // runs the loop (warp-uniform values stay in uniform registers), one lane
     // issues the MMAs and commits.
     {
-      const int a = warp == S_MMA_WARP ? 0 : 1;
       const uint32_t idesc_s = idesc_f16_f32(QT, NT);
-      const uint32_t a_h = tmem_base + (uint32_t)(T_A + a * 32);   // hi: features | bias; mid at +16, lo at +24
       // descriptors are advanced by adding (bytes >> 4) to the start-address
       // field (shared addresses stay below 2^18 B, so the field cannot carry)
       const uint32_t b0 = smem_u32(sB);
@@ -245,44 +248,39 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         const int count = segment_at(p.line, blockIdx.x, done_tiles).count;
         if (count == 0) break;
         done_tiles += count;
-        // the segment's A operand in TMEM
-        if (!__all_sync(0xffffffffu, mbar_wait(&aready[a], (uint32_t)(ku & 1), 23))) goto done;
-        ++ku;
         for (int i = 0; i < count; ++i, ++gs) {
           const int s = gs % SNS;
           const int b = gs % NBUF;
-          if (gs >= NBUF &&
-              !__all_sync(0xffffffffu, mbar_wait(&sfree[b * SNQT + a], (uint32_t)(((gs / NBUF) - 1) & 1), 25)))
-            goto done;
           if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)((gs / SNS) & 1), 24))) goto done;
-          tc_fence_after();
           const uint64_t so = (uint64_t)((s * S_STAGE_BYTES) >> 4);
-          const uint32_t d = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
-          const uint64_t b_h = dh0 + so;
-          // three-part product, small terms first (the order of mma_s_tile)
-          const uint64_t b_m = dm0 + so, b_l = dl0 + so;
-          if (elect_one()) {
-            mma_f16_ts(d, a_h + 16u, b_m, idesc_s, 0u);                    // mid . mid
-            mma_f16_ts(d, a_h, b_l, idesc_s, 1u);                          // hi . lo
-            mma_f16_ts(d, a_h + 24u, b_h, idesc_s, 1u);                    // lo . hi
-            mma_f16_ts(d, a_h, b_m, idesc_s, 1u);                          // hi . mid
-            mma_f16_ts(d, a_h + 16u, b_h, idesc_s, 1u);                    // mid . hi
-            mma_f16_ts(d, a_h, b_h, idesc_s, 1u);                          // hi . hi
-            mma_f16_ts(d, a_h + 8u, b_h + (uint64_t)(256 >> 4), idesc_s, 1u);   // bias . bias
-            mma_commit(&tfull[b * SNQT + a]);
+          const uint64_t b_h = dh0 + so, b_m = dm0 + so, b_l = dl0 + so;
+#pragma unroll
+          for (int a = 0; a < SNQT; ++a) {
+            // the segment's A operand in TMEM
+            if (i == 0 && !__all_sync(0xffffffffu, mbar_wait(&aready[a], (uint32_t)(ku & 1), 23))) goto done;
+            if (gs >= NBUF &&
+                !__all_sync(0xffffffffu, mbar_wait(&sfree[b * SNQT + a], (uint32_t)(((gs / NBUF) - 1) & 1), 25)))
+              goto done;
+            tc_fence_after();
+            const uint32_t a_h = tmem_base + (uint32_t)(T_A + a * 32);   // hi: features | bias; mid at +16, lo at +24
+            const uint32_t d = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
+            // three-part product, small terms first (the order of mma_s_tile)
+            if (elect_one()) {
+              mma_s_tile(d, a_h, b_h, b_m, b_l, idesc_s);
+              mma_commit(&tfull[b * SNQT + a]);
+            }
+            __syncwarp();
           }
-          __syncwarp();
         }
+        ++ku;
       }
     }
   } else if (warp >= W_MMA_WARP) {
-    // W(g) of one (query tile, weight part) once the epilogue warps of that
-    // query tile have stored tile g's weights (whole warp runs the loop, lane
-    // 0 issues).
+    // W(g) of one query tile once its epilogue warps have stored tile g's
+    // weights (whole warp runs the loop, one lane issues).
     {
-      const int wi = warp - W_MMA_WARP;
-      const int a = wi >> 1, part = wi & 1;   // part 0: hi weights x [X_hi | X_lo]; 1: lo weights x X_hi
-      const uint32_t idesc_w = idesc_f16_f32(QT, part ? WN_LO : WN);
+      const int a = warp - W_MMA_WARP;
+      const uint32_t idesc_hi = idesc_f16_f32(QT, WN), idesc_lo = idesc_f16_f32(QT, WN_LO);
       const uint64_t dx0 = smem_desc_kmajor(smem_u32(sB) + S_XTH_OFFSET, 128, 8 * XT_ROW_BYTES);
       int gw = 0, grp = 0;
       for (int done_tiles = 0;;) {
@@ -303,14 +301,17 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
           if (!__all_sync(0xffffffffu, mbar_wait(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
           tc_fence_after();
           const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
-          const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT + part * 16);
-          const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS + part * WN);
+          const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
+          const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS);
           if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < NT / 16; ++ks) {
               // data columns 16 ks .. +15: column half ks/2; weights hi at +0, lo at +16
               const uint32_t wa = ph + (uint32_t)(32 * (ks >> 1) + 8 * (ks & 1));
-              mma_f16_ts(d, wa, xd0 + (uint64_t)(ks * (256 >> 4)), idesc_w, (first && ks == 0) ? 0u : 1u);
+              const uint64_t xd = xd0 + (uint64_t)(ks * (256 >> 4));
+              const uint32_t add = ks > 0 || !first;
+              mma_f16_ts(d, wa, xd, idesc_hi, add);              // hi weights x [X_hi | X_lo]
+              mma_f16_ts(d + WN, wa + 16u, xd, idesc_lo, add);   // lo weights x X_hi
             }
             mma_commit(&sfree[b * SNQT + a]);
             mma_commit(&empty[s]);
@@ -391,6 +392,41 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       constexpr int EPI_T = S_EPI_WARPS * 32;
 #pragma unroll
       for (int k = 0; k < 4; ++k) wacc[k * EPI_T + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto read_group = [&]() -> bool {
+        const int par = grp & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait(&wfull[par * SNQT + qt], (uint32_t)((grp >> 1) & 1), 30))) return false;
+        tc_fence_after();
+        // this warp's 8 features: hi weights x X_hi, hi weights x X_lo, lo weights x X_hi
+        uint32_t wv[8], wl[8], wm[8];
+        const uint32_t wcol = tmem_base + lane_off + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + qt * W_TILE_COLS + half * 8);
+        tmem_ld8(wcol, wv);
+        tmem_ld8(wcol + FSK_D, wl);
+        tmem_ld8(wcol + WN, wm);
+        tmem_ld_wait();
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          wv[k] = __float_as_uint(__uint_as_float(wv[k]) + (__uint_as_float(wl[k]) + __uint_as_float(wm[k])));
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&wempty[par * SNQT + qt]);
+        {
+          float4 s0 = wacc[threadIdx.x], s1 = wacc[EPI_T + threadIdx.x];
+          float4 e0 = wacc[2 * EPI_T + threadIdx.x], e1 = wacc[3 * EPI_T + threadIdx.x];
+          Comp c;
+#define FSK_WADD(S, E, V) c = Comp{S, E}; c.add(__uint_as_float(V)); S = c.s; E = c.c;
+          FSK_WADD(s0.x, e0.x, wv[0]) FSK_WADD(s0.y, e0.y, wv[1])
+          FSK_WADD(s0.z, e0.z, wv[2]) FSK_WADD(s0.w, e0.w, wv[3])
+          FSK_WADD(s1.x, e1.x, wv[4]) FSK_WADD(s1.y, e1.y, wv[5])
+          FSK_WADD(s1.z, e1.z, wv[6]) FSK_WADD(s1.w, e1.w, wv[7])
+#undef FSK_WADD
+          wacc[threadIdx.x] = s0;
+          wacc[EPI_T + threadIdx.x] = s1;
+          wacc[2 * EPI_T + threadIdx.x] = e0;
+          wacc[3 * EPI_T + threadIdx.x] = e1;
+        }
+        ++grp;
+        return true;
+      };
       const int t0 = sg.t0;
       const int t1 = t0 + sg.count;
       bool pend = false;     // a W group ended at the previous tile and is not read yet
@@ -407,7 +443,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         tmem_ld32(my_cols, r);
         tmem_ld_wait();
         float e[32];
-        if (scaled) {
+        if (__builtin_expect(scaled, 0)) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) e[j] = __uint_as_float(r[j]) * out_mul;
         } else {
@@ -416,16 +452,25 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         }
 #pragma unroll
         for (int j = 0; j < 32; ++j) e[j] = ex2_approx(e[j]);
-        if (valid < NT) {
+        const bool diag = t * NT + half * 32 == diag_col;   // these 32 columns are this warp's 32 rows
+        if (__builtin_expect(diag || valid < NT, 0)) {
+          // columns past the data and the self pair
+          const int n_ok = imin(32, imax(0, valid - half * 32));
+          const uint32_t drop = ~(n_ok == 32 ? 0xffffffffu : (1u << n_ok) - 1u) | (diag ? 1u << lane : 0u);
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (half * 32 + j >= valid) e[j] = 0.f;
+            if (drop & (1u << j)) e[j] = 0.f;
         }
-        if (t * NT + half * 32 == diag_col) {
-          // this chunk's 32 columns are this warp's 32 rows: drop the self pair
+        // fp16 hi / lo weights for the W product, written over this warp's
+        // S columns (hi: 16 columns of packed pairs, then lo), eight pairs at
+        // a time to keep the register peak low
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j == lane) e[j] = 0.f;
+        for (int h8 = 0; h8 < 2; ++h8) {
+          uint32_t hi[8], lo[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) split_pack(e[16 * h8 + 2 * j], e[16 * h8 + 2 * j + 1], hi[j], lo[j]);
+          tmem_st8(my_cols + (uint32_t)(8 * h8), hi);
+          tmem_st8(my_cols + (uint32_t)(16 + 8 * h8), lo);
         }
         float2 pa = make_float2(e[0], e[1]), pb = make_float2(e[2], e[3]);
 #pragma unroll
@@ -436,7 +481,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         pa = __fadd2_rn(pa, pb);
         const float cs = pa.x + pa.y;
         const bool trig = cs > (phi_scale + acc.s + cs) * SCORE_NEAR_FRACTION;   // phi_scale: the self pair
-        if (__any_sync(0xffffffffu, trig)) {
+        if (__builtin_expect(__any_sync(0xffffffffu, trig), 0)) {
           // The chunk's largest weight is recomputed exactly (argmax on keys
           // = value bits with the column in the low 5 bits, as in the KDE
           // kernel).  With A the keyed approximation, the pdf gets ex - A
@@ -488,17 +533,6 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
           __syncwarp();
         }
         acc.add(cs);
-        // fp16 hi / lo weights for the W product, written over this warp's
-        // S columns (hi: 16 columns of packed pairs, then lo), eight pairs at
-        // a time to keep the register peak low
-#pragma unroll
-        for (int h8 = 0; h8 < 2; ++h8) {
-          uint32_t hi[8], lo[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) split_pack(e[16 * h8 + 2 * j], e[16 * h8 + 2 * j + 1], hi[j], lo[j]);
-          tmem_st8(my_cols + (uint32_t)(8 * h8), hi);
-          tmem_st8(my_cols + (uint32_t)(16 + 8 * h8), lo);
-        }
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -508,47 +542,11 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         }
         // read a W group that ended at the previous tile (its MMAs were
         // issued after that tile's weights, so by now they are usually done)
-        const bool last = --left == 0 || t == t1 - 1;
-        if (last) left = p.group;
-        for (int pass = 0; pass < 2; ++pass) {
-          const bool do_read = pass == 0 ? pend : (last && t == t1 - 1);
-          if (!do_read) continue;
-          const int par = grp & 1;
-          if (!__all_sync(0xffffffffu, mbar_wait(&wfull[par * SNQT + qt], (uint32_t)((grp >> 1) & 1), 30))) goto done;
-          tc_fence_after();
-          // this warp's 8 features: hi weights x X_hi, hi weights x X_lo, lo weights x X_hi
-          uint32_t wv[8], wl[8], wm[8];
-          const uint32_t wcol = tmem_base + lane_off + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + qt * W_TILE_COLS + half * 8);
-          tmem_ld8(wcol, wv);
-          tmem_ld8(wcol + FSK_D, wl);
-          tmem_ld8(wcol + WN, wm);
-          tmem_ld_wait();
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            wv[k] = __float_as_uint(__uint_as_float(wv[k]) + (__uint_as_float(wl[k]) + __uint_as_float(wm[k])));
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&wempty[par * SNQT + qt]);
-          {
-            float4 s0 = wacc[threadIdx.x], s1 = wacc[EPI_T + threadIdx.x];
-            float4 e0 = wacc[2 * EPI_T + threadIdx.x], e1 = wacc[3 * EPI_T + threadIdx.x];
-            Comp c;
-#define FSK_WADD(S, E, V) c = Comp{S, E}; c.add(__uint_as_float(V)); S = c.s; E = c.c;
-            FSK_WADD(s0.x, e0.x, wv[0]) FSK_WADD(s0.y, e0.y, wv[1])
-            FSK_WADD(s0.z, e0.z, wv[2]) FSK_WADD(s0.w, e0.w, wv[3])
-            FSK_WADD(s1.x, e1.x, wv[4]) FSK_WADD(s1.y, e1.y, wv[5])
-            FSK_WADD(s1.z, e1.z, wv[6]) FSK_WADD(s1.w, e1.w, wv[7])
-#undef FSK_WADD
-            wacc[threadIdx.x] = s0;
-            wacc[EPI_T + threadIdx.x] = s1;
-            wacc[2 * EPI_T + threadIdx.x] = e0;
-            wacc[3 * EPI_T + threadIdx.x] = e1;
-          }
-          ++grp;
-          if (pass == 0) pend = false;
-        }
-        if (last && t != t1 - 1) pend = true;
+        if (__builtin_expect(pend, 0) && !read_group()) goto done;
+        pend = --left == 0;
+        if (pend) left = p.group;
       }
+      if (!read_group()) goto done;   // the segment's last group
       // Combine the two column halves' corrections of this row for the 8
       // features this warp outputs.  Buffers alternate by unit parity; the
       // previous parity is cleared once every warp has passed this unit's
@@ -599,7 +597,7 @@ done:
       mbar_wait(&full[i % SNS], (uint32_t)((i / SNS) & 1), 32);
     if (n_query_copies > 0) mbar_wait(qready, (uint32_t)((n_query_copies - 1) & 1), 33);
   }
-  if ((warp == S_MMA_WARP || warp == S_MMA_WARP2 || warp >= W_MMA_WARP) && elect_one()) {
+  if (warp >= S_MMA_WARP && elect_one()) {
     mma_commit(drain);   // one arrival per issuing thread, when its MMAs have finished
     mbar_wait(drain, 0, 34);
   }
