@@ -87,35 +87,42 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_rows_kernel(const double* 
   if (skip != nullptr && *skip != 0) return;
   constexpr int ROWS = RED_THREADS / RL;
   const int r = threadIdx.x % ROWS, l = threadIdx.x / ROWS;
-  const int64_t i = (int64_t)blockIdx.x * ROWS + r;
-  double s = 0.0;
-  if (i < m) {
+  for (int64_t i0 = (int64_t)blockIdx.x * ROWS; i0 < m; i0 += (int64_t)gridDim.x * ROWS) {
+    const int64_t i = i0 + r;
+    double s = 0.0;
+    if (i < m) {
 #pragma unroll 4
-    for (int k = l; k < splits; k += RL) s += partials[(int64_t)k * m + i];
-  }
-  if (RL > 1) {
-    __shared__ double sh[RL][ROWS];
-    sh[l][r] = s;
-    __syncthreads();
-    if (l > 0 || i >= m) return;
+      for (int k = l; k < splits; k += RL) s += partials[(int64_t)k * m + i];
+    }
+    if (RL > 1) {
+      __shared__ double sh[RL][ROWS];
+      __syncthreads();   // the rows before are out
+      sh[l][r] = s;
+      __syncthreads();
+      if (l > 0 || i >= m) continue;
 #pragma unroll
-    for (int j = 1; j < RL; ++j) s += sh[j][r];
+      for (int j = 1; j < RL; ++j) s += sh[j][r];
+    }
+    if (i >= m) continue;
+    double v = s * scale;
+    if (log_out) v = log(v + eps);
+    out[i] = (float)v;
   }
-  if (i >= m) return;
-  double v = s * scale;
-  if (log_out) v = log(v + eps);
-  out[i] = (float)v;
 }
 
 void launch_reduce_rows(const double* partials, int splits, int64_t m, double scale, double eps,
                         bool log_out, float* out, const int* skip, cudaStream_t s) {
-  // one thread per row while the chain is short
+  // one thread per row while the chain is short; where the launch may turn out
+  // to have nothing to do, no more blocks than fit at once (32768 that return
+  // at once take 19 us)
+  const int rows = splits <= 4 ? RED_THREADS : RED_THREADS / RED_LANES;
+  int64_t blocks = (m + rows - 1) / rows;
+  if (skip != nullptr) blocks = imin<int64_t>(blocks, 8LL * sm_count());
   if (splits <= 4)
-    reduce_rows_kernel<1><<<(unsigned)((m + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
-        partials, splits, m, scale, eps, log_out ? 1 : 0, out, skip);
+    reduce_rows_kernel<1><<<(unsigned)blocks, RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out, skip);
   else
-    reduce_rows_kernel<RED_LANES><<<(unsigned)((m + RED_THREADS / RED_LANES - 1) / (RED_THREADS / RED_LANES)),
-                                    RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out, skip);
+    reduce_rows_kernel<RED_LANES><<<(unsigned)blocks, RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out,
+                                                                           skip);
   count_launch();
 }
 
