@@ -61,10 +61,27 @@ __global__ void reduce_rows_logexact_kernel(const double* __restrict__ partials,
   finish_or_list(i, m, s, scale, tiny, out, count, list);
 }
 
-// data parts per query group: enough work items to fill the grid
-__device__ __forceinline__ int ls_parts(int64_t groups, int grid) {
-  const int64_t want = (grid + groups - 1) / groups;
-  return (int)(want < 1 ? 1 : (want > FSK_LS_PARTS ? FSK_LS_PARTS : want));
+// Data parts per query group: a work item per resident block, more than 8 parts
+// only of at least 4 tiles per warp, as far as the partial rows' FSK_LS_PARTS * m
+// entries go (a row is `stride` slots long, the listed queries in whole
+// groups).  With 8 parts at most a short list left blocks idle: 2000 of 100003
+// queries against 262147 points took 1.1 ms here, 0.5 this way; twice the
+// items cost more in the combination than they balance.
+struct LsSplit {
+  int parts;
+  int64_t stride;
+};
+__device__ __forceinline__ LsSplit ls_split(int64_t count, int64_t m, int64_t n, int grid) {
+  const int64_t groups = (count + LS_QG - 1) / LS_QG;
+  LsSplit w;
+  w.stride = groups * LS_QG < m ? groups * LS_QG : m;
+  int64_t parts = (grid + groups - 1) / groups;
+  const int64_t tiles = (n + LS_TN - 1) / LS_TN;
+  const int64_t most = tiles / (4 * LS_WARPS) > 8 ? tiles / (4 * LS_WARPS) : 8;
+  if (parts > most) parts = most;
+  if (parts > FSK_LS_PARTS * m / w.stride) parts = FSK_LS_PARTS * m / w.stride;
+  w.parts = parts < 1 ? 1 : (int)parts;
+  return w;
 }
 
 // Running state of a lane's two queries (x and y halves), packed so that
@@ -115,7 +132,8 @@ __global__ void __launch_bounds__(LS_THREADS) logspace_kde16_kernel(
   const int64_t count = *count_ptr;
   if (count == 0) return;
   const int64_t groups = (count + LS_QG - 1) / LS_QG;
-  const int parts = ls_parts(groups, (int)gridDim.x);
+  const LsSplit w = ls_split(count, m, n, (int)gridDim.x);
+  const int parts = w.parts;
   const int64_t items = groups * parts;
   const int64_t n_tiles = (n + LS_TN - 1) / LS_TN;
   const int64_t tpp = (n_tiles + parts - 1) / parts;
@@ -184,8 +202,8 @@ __global__ void __launch_bounds__(LS_THREADS) logspace_kde16_kernel(
       }
       const int64_t slot = grp * LS_QG + qs;
       if (slot < count) {
-        pd[(int64_t)part * m + slot] = dm;
-        ps[(int64_t)part * m + slot] = sum;
+        pd[(int64_t)part * w.stride + slot] = dm;
+        ps[(int64_t)part * w.stride + slot] = sum;
       }
     }
     __syncthreads();
@@ -194,20 +212,21 @@ __global__ void __launch_bounds__(LS_THREADS) logspace_kde16_kernel(
 
 // out[list[slot]] = log(S) - dmin / (2 h^2) + log(scale) over the parts
 __global__ void logspace_combine_kernel(const uint32_t* __restrict__ count_ptr, const uint32_t* __restrict__ list,
-                                        const float* __restrict__ pd, const double* __restrict__ ps, int64_t m,
+                                        const float* __restrict__ pd, const double* __restrict__ ps, int64_t m, int64_t n,
                                         int ls_grid, double c2d, double c1d, double log_scale,
                                         float* __restrict__ out) {
   const int64_t count = *count_ptr;
   if (count == 0) return;
-  const int parts = ls_parts((count + LS_QG - 1) / LS_QG, ls_grid);
+  const LsSplit w = ls_split(count, m, n, ls_grid);
+  const int parts = w.parts;
   for (int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; slot < count;
        slot += (int64_t)gridDim.x * blockDim.x) {
     float dm = pd[slot];
-    for (int p = 1; p < parts; ++p) dm = fminf(dm, pd[(int64_t)p * m + slot]);
+    for (int p = 1; p < parts; ++p) dm = fminf(dm, pd[(int64_t)p * w.stride + slot]);
     double sum = 0.0;
     for (int p = 0; p < parts; ++p) {
-      const float d = pd[(int64_t)p * m + slot];
-      if (d < __int_as_float(0x7f800000)) sum += ps[(int64_t)p * m + slot] * exp2(-c2d * ((double)d - (double)dm));
+      const float d = pd[(int64_t)p * w.stride + slot];
+      if (d < __int_as_float(0x7f800000)) sum += ps[(int64_t)p * w.stride + slot] * exp2(-c2d * ((double)d - (double)dm));
     }
     const int64_t q = list[slot];
     if (in_bounds(q, m, 55)) out[q] = (float)(log(sum) - c1d * (double)dm + log_scale);
@@ -240,7 +259,7 @@ static void launch_listed(const float* q, int64_t m, const float* x, int64_t n, 
                                                                b.pd, b.ps, m);
     count_launch();
   }
-  logspace_combine_kernel<<<2 * sm_count(), 256, 0, s>>>(b.count, b.list, b.pd, b.ps, m, grid, c2d, c1d, log(scale),
+  logspace_combine_kernel<<<2 * sm_count(), 256, 0, s>>>(b.count, b.list, b.pd, b.ps, m, n, grid, c2d, c1d, log(scale),
                                                           out);
   count_launch();
 }
