@@ -42,10 +42,8 @@ constexpr int KB_X_OFFSET = KB_L_OFFSET + KNT * L_ROW_BYTES;  // 16 KB
 constexpr int KB_STAGE_BYTES = KB_X_OFFSET + KNT * FSK_D * 4; // 24 KB
 constexpr int EPI_WARPS = 8 * NQT;      // KDE: (lane quarter, column half) per query tile
 constexpr int PRODUCER_WARP = EPI_WARPS;
-constexpr int MMA_WARP = EPI_WARPS + 1;   // owns TMEM, issues the MMAs of query tile 0
-constexpr int MMA_WARP2 = EPI_WARPS + 2;  // issues the MMAs of query tile 1
-constexpr int MMA_ISSUERS = 2;
-constexpr int THREADS = (EPI_WARPS + 3) * 32;
+constexpr int MMA_WARP = EPI_WARPS + 1;   // owns TMEM, issues the MMAs
+constexpr int THREADS = (EPI_WARPS + 2) * 32;
 constexpr int NACC = 3;                  // KDE: accumulators, taken in turn by the query tiles
 constexpr int T_KA = NACC * KNT;         // KDE: query operand in tensor memory, [NQT][hi 16 | mid 8 | lo 8]
 constexpr int TMEM_COLS = 512;
@@ -66,7 +64,7 @@ constexpr float FP16_TARGET = 8192.0f;  // largest operand magnitude aimed for
 
 static_assert(T_KA + NQT * 32 <= TMEM_COLS, "TMEM budget");
 static_assert(NQT == 2 && NACC == 3, "the accumulator's predecessor and the depth of its barriers");
-static_assert((2 * NS + 8 * NQT + 2 + NQT + 1) * 8 + 4 <= 512, "barrier area");
+static_assert((2 * NS + 8 * NQT + 4) * 8 + 4 <= 512, "barrier area");
 static_assert(KB_STAGE_BYTES % 16 == 0 && A_BYTES % 16 == 0, "bulk copy granularity");
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 

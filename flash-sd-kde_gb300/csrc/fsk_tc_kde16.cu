@@ -33,12 +33,12 @@
 //    terms carry the ~2^-25 relative error of the accumulation, which
 //    averages out.
 //
-// Pipeline (one persistent CTA per SM, 19 warps):
+// Pipeline (one persistent CTA per SM, 18 warps):
 //   warp 16 : producer - bulk (TMA) copies of query images per unit and of
 //             data-tile images (128 points) per stage into shared memory
 //             (mbarrier tx).
-//   warps 17, 18 : copy the query operand of tiles 0 and 1 to tensor memory
-//             once per segment and issue their MMAs; warp 17 owns TMEM.
+//   warp 17 : copies the query operands to tensor memory once per segment
+//             and issues all MMAs (one lane); owns TMEM.
 //   warps 0-15: epilogue; warp w reads TMEM lanes 32*(w%4).. and columns
 //             64*((w/4)%2).. of query tile w/8.
 // A work unit (segment, see WorkLine) is 256 queries (two M=128 tiles) x a run
@@ -47,7 +47,7 @@
 // tile).  With both operands in shared memory an M=128, N=128, K=16 MMA takes
 // ~100 cycles (44 of them for A, whatever N is), with A in tensor memory 64:
 // four double-buffered accumulators and A in shared memory took 11.95 ms at
-// n = m = 262144, this 11.5 (2^20: 184.3, 177.7).  Now the exp pipe is busy
+// n = m = 262144, this 11.35 (2^20: 184.3, 176.4).  The exp pipe is then busy
 // 62 % of the time, the tensor core 54 %, issue slots 55 %; the rest is the
 // latency of waits, TMEM loads and add chains that 16 warps of 96 registers
 // cannot hide.  Each query's sum is kept as two column halves by two threads
@@ -89,8 +89,8 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
   uint64_t* tempty = tfull + 4 * NQT;    // accumulator drained
   uint64_t* qready = tempty + 4 * NQT;   // query images loaded
   uint64_t* qempty = qready + 1;         // query images copied to tensor memory
-  uint64_t* sdone = qready + 2;          // [NQT] a query tile's MMAs of the segment finished
-  uint64_t* drain = sdone + NQT;         // all MMAs of this CTA finished (exit path)
+  uint64_t* sdone = qready + 2;          // the MMAs of the segment finished
+  uint64_t* drain = sdone + 1;           // all MMAs of this CTA finished (exit path)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   uint32_t n_stage_copies = 0, n_query_copies = 0;   // producer: bulk copies issued
 
@@ -100,16 +100,16 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < NS; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], MMA_ISSUERS + EPI_WARPS);
+      mbar_init(&empty[s], 1 + EPI_WARPS);
     }
     for (int i = 0; i < 4 * NQT; ++i) {
       mbar_init(&tfull[i], 1);
       mbar_init(&tempty[i], EPI_WARPS / NQT);
     }
     mbar_init(qready, 1);
-    for (int i = 0; i < NQT; ++i) mbar_init(&sdone[i], 1);
-    mbar_init(qempty, MMA_ISSUERS);
-    mbar_init(drain, MMA_ISSUERS);
+    mbar_init(sdone, 1);
+    mbar_init(qempty, 1);
+    mbar_init(drain, 1);
     fence_barrier_init();
   }
   if (warp == MMA_WARP) {
@@ -154,19 +154,19 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         }
       }
     }
-  } else if (warp == MMA_WARP || warp == MMA_WARP2) {
-    // Two issuing warps, one query tile each.  Accumulation u = 2 g + a (data
-    // tile g of this CTA's run, query tile a) goes to accumulator u % NACC, so
-    // the tiles take the accumulators in turn and a tile's MMAs wait only for
-    // the 8 warps reading the one before them there.  The query operand is
-    // copied to tensor memory once per segment.  u - NACC is tile g - 2 + a of
-    // the other query tile.  The per-tile path is kept to
-    // the waits, the MMAs and the commits (descriptors of stage s = stage 0 +
-    // s * KB_STAGE_BYTES in the 16-byte address field).
+  } else if (warp == MMA_WARP) {
+    // Accumulation u = 2 g + a (data tile g of this CTA's run, query tile a)
+    // goes to accumulator u % NACC, so the query tiles take the accumulators
+    // in turn and a tile's MMAs wait only for the 8 warps reading the one
+    // before them there: u - NACC, tile g - 2 + a of the other query tile.  The
+    // query operand is copied to tensor memory once per segment.  The per-tile
+    // path is kept to the waits, the MMAs and the commits (descriptors of
+    // stage s = stage 0 + s * KB_STAGE_BYTES in the 16-byte address field).
+    // One warp issues for both query tiles: a second one's polling took issue
+    // slots from the epilogue (11.5 against 11.35 ms at n = m = 262144).
     {
       const uint32_t idesc = idesc_f16_f32(QT, KNT);
-      const int a = (warp == MMA_WARP) ? 0 : 1;
-      const uint32_t as = smem_u32(sA + a * A_TILE_BYTES);
+      const uint32_t as = smem_u32(sA);
       const uint64_t a_h = smem_desc_kmajor(as, 128, 8 * H_ROW_BYTES);
       const uint64_t a_m = smem_desc_kmajor(as + A_M_OFFSET, 128, 8 * L_ROW_BYTES);
       const uint64_t a_l = smem_desc_kmajor(as + A_L_OFFSET, 128, 8 * L_ROW_BYTES);
@@ -174,50 +174,56 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       const uint64_t b_h0 = smem_desc_kmajor(bs0, 128, 8 * H_ROW_BYTES);
       const uint64_t b_m0 = smem_desc_kmajor(bs0 + KB_M_OFFSET, 128, 8 * L_ROW_BYTES);
       const uint64_t b_l0 = smem_desc_kmajor(bs0 + KB_L_OFFSET, 128, 8 * L_ROW_BYTES);
-      const uint32_t ta = tmem_base + (uint32_t)(T_KA + a * 32);   // hi: features | bias; mid at +16, lo at +24
+      const uint32_t ta = tmem_base + (uint32_t)T_KA;   // per query tile, hi: features | bias; mid at +16, lo at +24
       uint32_t k = 0, ph = 0;
       int s = 0;
       int g = 0;            // data tile
-      int acc = a;          // u % NACC
+      int acc = 0;          // u % NACC
       for (int done_tiles = 0;; ++k) {
         const int nt = next_segment(p.line, done_tiles).count;
         if (nt == 0) break;
         done_tiles += nt;
         if (!__all_sync(0xffffffffu, mbar_wait(qready, k & 1u, 3))) goto done;
         // the previous segment's MMAs have read its operand
-        if (k > 0 && !__all_sync(0xffffffffu, mbar_wait(&sdone[a], (k - 1) & 1u, 10))) goto done;
+        if (k > 0 && !__all_sync(0xffffffffu, mbar_wait(sdone, (k - 1) & 1u, 10))) goto done;
         tc_fence_after();
         if (elect_one()) {
-          tmem_cp_128x256b(ta, a_h);
-          tmem_cp_128x256b(ta + 8u, a_h + (256 >> 4));
-          if (!SINGLE) {
-            tmem_cp_128x256b(ta + 16u, a_m);
-            tmem_cp_128x256b(ta + 24u, a_l);
+#pragma unroll
+          for (int a = 0; a < NQT; ++a) {
+            const uint64_t at = (uint64_t)(a * A_TILE_BYTES >> 4);
+            tmem_cp_128x256b(ta + 32u * a, a_h + at);
+            tmem_cp_128x256b(ta + 32u * a + 8u, a_h + at + (256 >> 4));
+            if (!SINGLE) {
+              tmem_cp_128x256b(ta + 32u * a + 16u, a_m + at);
+              tmem_cp_128x256b(ta + 32u * a + 24u, a_l + at);
+            }
           }
           mma_commit(qempty);
         }
         __syncwarp();
         for (int i = 0; i < nt; ++i) {
           if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, 4))) goto done;
-          const int prev = g - 2 + a;
-          if (prev >= 0 && !__all_sync(0xffffffffu, mbar_wait(&tempty[(1 - a) * 4 + (prev & 3)], (uint32_t)(prev >> 2) & 1u, 5)))
-            goto done;
-          tc_fence_after();
           const uint64_t so = (uint64_t)(s * (KB_STAGE_BYTES >> 4));
-          if (elect_one()) {
-            const uint32_t d = tmem_base + (uint32_t)(acc * KNT);
-            if (SINGLE)
-              mma_s_tile_single(d, ta, b_h0 + so, idesc);
-            else
-              mma_s_tile(d, ta, b_h0 + so, b_m0 + so, b_l0 + so, idesc);
-            mma_commit(&tfull[a * 4 + (g & 3)]);
-            mma_commit(&empty[s]);
-            if (i == nt - 1) mma_commit(&sdone[a]);
+#pragma unroll
+          for (int a = 0; a < NQT; ++a) {
+            const int prev = g - 2 + a;
+            if (prev >= 0 && !__all_sync(0xffffffffu, mbar_wait(&tempty[(1 - a) * 4 + (prev & 3)], (uint32_t)(prev >> 2) & 1u, 5)))
+              goto done;
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t d = tmem_base + (uint32_t)(acc * KNT);
+              if (SINGLE)
+                mma_s_tile_single(d, ta + 32u * a, b_h0 + so, idesc);
+              else
+                mma_s_tile(d, ta + 32u * a, b_h0 + so, b_m0 + so, b_l0 + so, idesc);
+              mma_commit(&tfull[a * 4 + (g & 3)]);
+              if (a == NQT - 1) mma_commit(&empty[s]);
+              if (a == NQT - 1 && i == nt - 1) mma_commit(sdone);
+            }
+            __syncwarp();
+            if (++acc == NACC) acc = 0;
           }
-          __syncwarp();
           ++g;
-          acc += NQT;
-          if (acc >= NACC) acc -= NACC;
           if (++s == NS) {
             s = 0;
             ph ^= 1u;
@@ -395,7 +401,7 @@ done:
       mbar_wait(&full[i % NS], (i / NS) & 1u, 7);
     if (n_query_copies > 0) mbar_wait(qready, (n_query_copies - 1) & 1u, 8);
   }
-  if ((warp == MMA_WARP || warp == MMA_WARP2) && elect_one()) {
+  if (warp == MMA_WARP && elect_one()) {
     mma_commit(drain);   // one arrival per issuing thread, when its MMAs have finished
     mbar_wait(drain, 0, 9);
   }
