@@ -28,11 +28,11 @@
 //    points) from the data stage, FP32 accumulation over a group of tiles
 //    (score_group), then added into compensated FP32 sums.
 //
-// Pipeline (one persistent CTA per SM, 20 warps of 96 registers):
+// Pipeline (one persistent CTA per SM, 19 warps of 96 registers):
 //   warp 16 : producer (bulk copies of query images per unit, data stages).
 //   warp 17 : issues S for both query tiles, up to NBUF tiles ahead of W;
 //             owns TMEM.
-//   warps 18, 19 : issue the weighted-sum MMAs of query tiles 0 and 1.
+//   warp 18 : issues the weighted-sum MMAs of both query tiles.
 //   warps 0-15: epilogue; warp w: query tile w/8, data-column half (w/4)&1,
 //             TMEM lane quarter w&3.  The two column halves of a row keep
 //             separate pdf partials (two rows per segment) and
@@ -45,7 +45,9 @@
 // unlikely and stays behind the straight path, and the weights are stored
 // before the sums, whose latency covers that of the stores.  n = 262144:
 // 24.1 ms with seven issuing warps of 80 registers and separate ragged and
-// diagonal blocks, 20.6 this way (2^20: 381, 328).  Tried and slower: eight
+// diagonal blocks, 20.6 this way, 20.0 with one weighted-sum issuer instead
+// of one per query tile (its polling took issue slots) and five data stages
+// (2^20: 381, 328, 318).  Tried and slower: one warp for all MMAs (29.9), eight
 // warps of 64 columns (28.6 ms), S and weights in separate columns with one
 // buffer each (25.9), the rare blocks as calls (21.6-22.3), the next tile's S
 // loaded ahead (25.0, spills).
@@ -64,14 +66,13 @@ namespace tc {
 namespace {
 
 constexpr int SNQT = 2;                                    // query tiles per unit (256 queries)
-constexpr int SNS = 4;                                     // data stages
+constexpr int SNS = 5;                                     // data stages
 constexpr int S_A_BYTES = SNQT * A_TILE_BYTES;             // 32 KB
 constexpr int S_EPI_WARPS = 8 * SNQT;
 constexpr int S_PRODUCER_WARP = S_EPI_WARPS;
 constexpr int S_MMA_WARP = S_EPI_WARPS + 1;     // issues the S MMAs, owns TMEM
-constexpr int W_MMA_WARP = S_EPI_WARPS + 2;     // first of the W_ISSUERS weighted-sum issuers
-constexpr int W_ISSUERS = SNQT;                 // one per query tile
-constexpr int S_THREADS = (S_EPI_WARPS + 2 + W_ISSUERS) * 32;
+constexpr int W_MMA_WARP = S_EPI_WARPS + 2;     // issues the weighted-sum MMAs
+constexpr int S_THREADS = (S_EPI_WARPS + 3) * 32;
 constexpr int NBUF = 2;                                    // S / weight buffers in TMEM
 constexpr int WN = 2 * FSK_D;                              // W MMA N, hi weights: X_hi and X_lo rows
 constexpr int WN_LO = FSK_D;                               // W MMA N, lo weights: X_hi rows
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < SNS; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], W_ISSUERS + S_EPI_WARPS);   // the W threads' commits + every epilogue warp
+      mbar_init(&empty[s], SNQT + S_EPI_WARPS);   // W commits of both query tiles + every epilogue warp
     }
     for (int i = 0; i < NBUF * SNQT; ++i) {
       mbar_init(&tfull[i], 1);
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
     for (int a = 0; a < SNQT; ++a) mbar_init(&aready[a], 8);
     mbar_init(qready, 1);
     mbar_init(qempty, S_EPI_WARPS);
-    mbar_init(drain, 1 + W_ISSUERS);
+    mbar_init(drain, 2);   // the S and the W issuer
     mbar_init(cready, S_EPI_WARPS);
     fence_barrier_init();
   }
@@ -275,11 +276,10 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         ++ku;
       }
     }
-  } else if (warp >= W_MMA_WARP) {
-    // W(g) of one query tile once its epilogue warps have stored tile g's
-    // weights (whole warp runs the loop, one lane issues).
+  } else if (warp == W_MMA_WARP) {
+    // W(g) of both query tiles in turn, each once its epilogue warps have
+    // stored tile g's weights (whole warp runs the loop, one lane issues).
     {
-      const int a = warp - W_MMA_WARP;
       const uint32_t idesc_hi = idesc_f16_f32(QT, WN), idesc_lo = idesc_f16_f32(QT, WN_LO);
       const uint64_t dx0 = smem_desc_kmajor(smem_u32(sB) + S_XTH_OFFSET, 128, 8 * XT_ROW_BYTES);
       int gw = 0, grp = 0;
@@ -295,29 +295,32 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
           if (first) left = p.group;
           const bool last = --left == 0 || i == count - 1;
           const int par = grp & 1;
-          if (first &&
-              !__all_sync(0xffffffffu, mbar_wait(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
-            goto done;
-          if (!__all_sync(0xffffffffu, mbar_wait(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
-          tc_fence_after();
-          const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
-          const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
-          const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS);
-          if (elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < NT / 16; ++ks) {
-              // data columns 16 ks .. +15: column half ks/2; weights hi at +0, lo at +16
-              const uint32_t wa = ph + (uint32_t)(32 * (ks >> 1) + 8 * (ks & 1));
-              const uint64_t xd = xd0 + (uint64_t)(ks * (256 >> 4));
-              const uint32_t add = ks > 0 || !first;
-              mma_f16_ts(d, wa, xd, idesc_hi, add);              // hi weights x [X_hi | X_lo]
-              mma_f16_ts(d + WN, wa + 16u, xd, idesc_lo, add);   // lo weights x X_hi
+          for (int a = 0; a < SNQT; ++a) {
+            if (first &&
+                !__all_sync(0xffffffffu, mbar_wait(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
+              goto done;
+            if (!__all_sync(0xffffffffu, mbar_wait(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
+            tc_fence_after();
+            const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
+            const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
+            const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS);
+            if (elect_one()) {
+#pragma unroll
+              for (int ks = 0; ks < NT / 16; ++ks) {
+                // data columns 16 ks .. +15: column half ks/2; weights hi at +0, lo at +16
+                const uint32_t wa = ph + (uint32_t)(32 * (ks >> 1) + 8 * (ks & 1));
+                const uint64_t xd = xd0 + (uint64_t)(ks * (256 >> 4));
+                const uint32_t add = ks > 0 || !first;
+                mma_f16_ts(d, wa, xd, idesc_hi, add);              // hi weights x [X_hi | X_lo]
+                mma_f16_ts(d + WN, wa + 16u, xd, idesc_lo, add);   // lo weights x X_hi
+              }
+              mma_commit(&sfree[b * SNQT + a]);
+              mma_commit(&empty[s]);
+              if (last) mma_commit(&wfull[par * SNQT + a]);
             }
-            mma_commit(&sfree[b * SNQT + a]);
-            mma_commit(&empty[s]);
-            if (last) mma_commit(&wfull[par * SNQT + a]);
+            __syncwarp();
           }
-          __syncwarp();
           if (last) ++grp;
         }
       }
