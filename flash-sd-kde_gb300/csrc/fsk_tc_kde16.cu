@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         const Segment sg = next_segment(p.line, done_tiles);
         if (sg.count == 0) break;
         done_tiles += sg.count;
-        if (!__all_sync(0xffffffffu, mbar_wait(qempty, (k & 1u) ^ 1u, 1))) goto done;
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(qempty, (k & 1u) ^ 1u, 1))) goto done;
         if (lane == 0) {
           mbar_arrive_expect_tx(qready, A_BYTES);
           bulk_g2s(sA, p.qimg + sg.qb * (int64_t)A_BYTES, A_BYTES, qready);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         ++k;
         const uint8_t* src = p.ximg + sg.t0 * (int64_t)KB_STAGE_BYTES;
         for (int i = 0; i < sg.count; ++i, src += KB_STAGE_BYTES) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1u, 2))) goto done;
+          if (!__all_sync(0xffffffffu, mbar_wait_cold(&empty[s], ph ^ 1u, 2))) goto done;
           if (lane == 0) {
             mbar_arrive_expect_tx(&full[s], KB_STAGE_BYTES);
             bulk_g2s(sB + s * KB_STAGE_BYTES, src, KB_STAGE_BYTES, &full[s]);
@@ -183,9 +183,9 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         const int nt = next_segment(p.line, done_tiles).count;
         if (nt == 0) break;
         done_tiles += nt;
-        if (!__all_sync(0xffffffffu, mbar_wait(qready, k & 1u, 3))) goto done;
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(qready, k & 1u, 3))) goto done;
         // the previous segment's MMAs have read its operand
-        if (k > 0 && !__all_sync(0xffffffffu, mbar_wait(sdone, (k - 1) & 1u, 10))) goto done;
+        if (k > 0 && !__all_sync(0xffffffffu, mbar_wait_cold(sdone, (k - 1) & 1u, 10))) goto done;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -202,12 +202,12 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
         }
         __syncwarp();
         for (int i = 0; i < nt; ++i) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, 4))) goto done;
+          if (!__all_sync(0xffffffffu, mbar_wait_cold(&full[s], ph, 4))) goto done;
           const uint64_t so = (uint64_t)(s * (KB_STAGE_BYTES >> 4));
 #pragma unroll
           for (int a = 0; a < NQT; ++a) {
             const int prev = g - 2 + a;
-            if (prev >= 0 && !__all_sync(0xffffffffu, mbar_wait(&tempty[(1 - a) * 4 + (prev & 3)], (uint32_t)(prev >> 2) & 1u, 5)))
+            if (prev >= 0 && !__all_sync(0xffffffffu, mbar_wait_cold(&tempty[(1 - a) * 4 + (prev & 3)], (uint32_t)(prev >> 2) & 1u, 5)))
               goto done;
             tc_fence_after();
             if (elect_one()) {
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       for (int i = 0; i < nt; ++i, ++g) {
         const int valid = i == last_i ? last_valid : KNT / 2;   // may be <= 0 on the last tile
         // (a timed-out wait ends the whole warp: it must stay converged)
-        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[qt * 4 + (g & 3)], (uint32_t)(g >> 2) & 1u, 6))) goto done;
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(&tfull[qt * 4 + (g & 3)], (uint32_t)(g >> 2) & 1u, 6))) goto done;
         tc_fence_after();
         const uint8_t* xrows = sB + s * KB_STAGE_BYTES + KB_X_OFFSET + half * (KNT / 2) * (FSK_D * 4);
         float tsum = 0.f;
@@ -398,12 +398,12 @@ done:
   // MMAs finish before shared and tensor memory are released.
   if (warp == PRODUCER_WARP && lane == 0) {
     for (uint32_t i = n_stage_copies > (uint32_t)NS ? n_stage_copies - NS : 0u; i < n_stage_copies; ++i)
-      mbar_wait(&full[i % NS], (i / NS) & 1u, 7);
-    if (n_query_copies > 0) mbar_wait(qready, (n_query_copies - 1) & 1u, 8);
+      mbar_wait_cold(&full[i % NS], (i / NS) & 1u, 7);
+    if (n_query_copies > 0) mbar_wait_cold(qready, (n_query_copies - 1) & 1u, 8);
   }
   if (warp == MMA_WARP && elect_one()) {
     mma_commit(drain);   // one arrival per issuing thread, when its MMAs have finished
-    mbar_wait(drain, 0, 9);
+    mbar_wait_cold(drain, 0, 9);
   }
   tc_fence_before();
   __syncthreads();

@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         const Segment sg = segment_at(p.line, blockIdx.x, done_tiles);
         if (sg.count == 0) break;
         done_tiles += sg.count;
-        if (!__all_sync(0xffffffffu, mbar_wait(qempty, (uint32_t)((k & 1) ^ 1), 21))) goto done;
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(qempty, (uint32_t)((k & 1) ^ 1), 21))) goto done;
         if (lane == 0) {
           mbar_arrive_expect_tx(qready, S_A_BYTES + S_QX_BYTES);
           bulk_g2s(sA, p.qimg + sg.qb * (int64_t)S_A_BYTES, S_A_BYTES, qready);
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         ++k;
         const uint8_t* src = p.ximg + sg.t0 * (int64_t)S_STAGE_BYTES;
         for (int i = 0; i < sg.count; ++i, src += S_STAGE_BYTES) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty[st], ph ^ 1u, 22))) goto done;
+          if (!__all_sync(0xffffffffu, mbar_wait_cold(&empty[st], ph ^ 1u, 22))) goto done;
           if (lane == 0) {
             mbar_arrive_expect_tx(&full[st], S_STAGE_BYTES);
             bulk_g2s(sB + st * S_STAGE_BYTES, src, S_STAGE_BYTES, &full[st]);
@@ -252,15 +252,15 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         for (int i = 0; i < count; ++i, ++gs) {
           const int s = gs % SNS;
           const int b = gs % NBUF;
-          if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)((gs / SNS) & 1), 24))) goto done;
+          if (!__all_sync(0xffffffffu, mbar_wait_cold(&full[s], (uint32_t)((gs / SNS) & 1), 24))) goto done;
           const uint64_t so = (uint64_t)((s * S_STAGE_BYTES) >> 4);
           const uint64_t b_h = dh0 + so, b_m = dm0 + so, b_l = dl0 + so;
 #pragma unroll
           for (int a = 0; a < SNQT; ++a) {
             // the segment's A operand in TMEM
-            if (i == 0 && !__all_sync(0xffffffffu, mbar_wait(&aready[a], (uint32_t)(ku & 1), 23))) goto done;
+            if (i == 0 && !__all_sync(0xffffffffu, mbar_wait_cold(&aready[a], (uint32_t)(ku & 1), 23))) goto done;
             if (gs >= NBUF &&
-                !__all_sync(0xffffffffu, mbar_wait(&sfree[b * SNQT + a], (uint32_t)(((gs / NBUF) - 1) & 1), 25)))
+                !__all_sync(0xffffffffu, mbar_wait_cold(&sfree[b * SNQT + a], (uint32_t)(((gs / NBUF) - 1) & 1), 25)))
               goto done;
             tc_fence_after();
             const uint32_t a_h = tmem_base + (uint32_t)(T_A + a * 32);   // hi: features | bias; mid at +16, lo at +24
@@ -298,9 +298,9 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
 #pragma unroll
           for (int a = 0; a < SNQT; ++a) {
             if (first &&
-                !__all_sync(0xffffffffu, mbar_wait(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
+                !__all_sync(0xffffffffu, mbar_wait_cold(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
               goto done;
-            if (!__all_sync(0xffffffffu, mbar_wait(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
+            if (!__all_sync(0xffffffffu, mbar_wait_cold(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
             tc_fence_after();
             const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
             const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       // The unit's query images: this row's A operand to TMEM (column half 0
       // copies the hi row, half 1 the mid and lo rows).  The S MMAs of the previous
       // unit have all completed: this warp consumed their accumulators.
-      if (!__all_sync(0xffffffffu, mbar_wait(qready, (uint32_t)(k_unit & 1), 36))) goto done;
+      if (!__all_sync(0xffffffffu, mbar_wait_cold(qready, (uint32_t)(k_unit & 1), 36))) goto done;
       {
         const uint8_t* tile = sA + qt * A_TILE_BYTES;
         const uint32_t ta = tmem_base + lane_off + (uint32_t)(T_A + qt * 32);
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       for (int k = 0; k < 4; ++k) wacc[k * EPI_T + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
       auto read_group = [&]() -> bool {
         const int par = grp & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(&wfull[par * SNQT + qt], (uint32_t)((grp >> 1) & 1), 30))) return false;
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(&wfull[par * SNQT + qt], (uint32_t)((grp >> 1) & 1), 30))) return false;
         tc_fence_after();
         // this warp's 8 features: hi weights x X_hi, hi weights x X_lo, lo weights x X_hi
         uint32_t wv[8], wl[8], wm[8];
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       for (int t = t0; t < t1; ++t, ++g, s = (s + 1 == SNS) ? 0 : s + 1) {
         const int b = g % NBUF;
         const int valid = t == last_t ? last_valid : NT;
-        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[b * SNQT + qt], (uint32_t)((g / NBUF) & 1), 28))) goto done;
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(&tfull[b * SNQT + qt], (uint32_t)((g / NBUF) & 1), 28))) goto done;
         tc_fence_after();
         const uint8_t* stage = sB + s * S_STAGE_BYTES;
         // this warp's 32 S columns; its weights go back into the same columns
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         mbar_arrive(cready);
         mbar_arrive(qempty);   // done with this unit's query images and rows in shared memory
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(cready, (uint32_t)(k_unit & 1), 35))) goto done;
+      if (!__all_sync(0xffffffffu, mbar_wait_cold(cready, (uint32_t)(k_unit & 1), 35))) goto done;
       {
         float* wc_next = wcorr + ((k_unit + 1) & 1) * WC_PAR + half * WC_HALF + wc_row;
 #pragma unroll
@@ -597,12 +597,12 @@ done:
   // MMAs finish before shared and tensor memory are released.
   if (warp == S_PRODUCER_WARP && lane == 0) {
     for (int64_t i = imax<int64_t>(0, n_stage_copies - SNS); i < n_stage_copies; ++i)
-      mbar_wait(&full[i % SNS], (uint32_t)((i / SNS) & 1), 32);
-    if (n_query_copies > 0) mbar_wait(qready, (uint32_t)((n_query_copies - 1) & 1), 33);
+      mbar_wait_cold(&full[i % SNS], (uint32_t)((i / SNS) & 1), 32);
+    if (n_query_copies > 0) mbar_wait_cold(qready, (uint32_t)((n_query_copies - 1) & 1), 33);
   }
   if (warp >= S_MMA_WARP && elect_one()) {
     mma_commit(drain);   // one arrival per issuing thread, when its MMAs have finished
-    mbar_wait(drain, 0, 34);
+    mbar_wait_cold(drain, 0, 34);
   }
   tc_fence_before();
   __syncthreads();
