@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(LS_THREADS) logspace_kde16_kernel(
   const int64_t count = *count_ptr;
   if (count == 0) return;
   const int64_t groups = (count + LS_QG - 1) / LS_QG;
-  const LsSplit w = ls_split(count, m, n, (int)gridDim.x);
-  const int parts = w.parts;
+  const LsSplit split = ls_split(count, m, n, (int)gridDim.x);
+  const int parts = split.parts;
   const int64_t items = groups * parts;
   const int64_t n_tiles = (n + LS_TN - 1) / LS_TN;
   const int64_t tpp = (n_tiles + parts - 1) / parts;
@@ -202,8 +202,8 @@ __global__ void __launch_bounds__(LS_THREADS) logspace_kde16_kernel(
       }
       const int64_t slot = grp * LS_QG + qs;
       if (slot < count) {
-        pd[(int64_t)part * w.stride + slot] = dm;
-        ps[(int64_t)part * w.stride + slot] = sum;
+        pd[(int64_t)part * split.stride + slot] = dm;
+        ps[(int64_t)part * split.stride + slot] = sum;
       }
     }
     __syncthreads();
@@ -217,16 +217,16 @@ __global__ void logspace_combine_kernel(const uint32_t* __restrict__ count_ptr, 
                                         float* __restrict__ out) {
   const int64_t count = *count_ptr;
   if (count == 0) return;
-  const LsSplit w = ls_split(count, m, n, ls_grid);
-  const int parts = w.parts;
+  const LsSplit split = ls_split(count, m, n, ls_grid);
+  const int parts = split.parts;
   for (int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; slot < count;
        slot += (int64_t)gridDim.x * blockDim.x) {
     float dm = pd[slot];
-    for (int p = 1; p < parts; ++p) dm = fminf(dm, pd[(int64_t)p * w.stride + slot]);
+    for (int p = 1; p < parts; ++p) dm = fminf(dm, pd[(int64_t)p * split.stride + slot]);
     double sum = 0.0;
     for (int p = 0; p < parts; ++p) {
-      const float d = pd[(int64_t)p * w.stride + slot];
-      if (d < __int_as_float(0x7f800000)) sum += ps[(int64_t)p * w.stride + slot] * exp2(-c2d * ((double)d - (double)dm));
+      const float d = pd[(int64_t)p * split.stride + slot];
+      if (d < __int_as_float(0x7f800000)) sum += ps[(int64_t)p * split.stride + slot] * exp2(-c2d * ((double)d - (double)dm));
     }
     const int64_t q = list[slot];
     if (in_bounds(q, m, 55)) out[q] = (float)(log(sum) - c1d * (double)dm + log_scale);

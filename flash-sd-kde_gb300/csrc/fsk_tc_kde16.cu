@@ -47,7 +47,7 @@
 // tile).  With both operands in shared memory an M=128, N=128, K=16 MMA takes
 // ~100 cycles (44 of them for A, whatever N is), with A in tensor memory 64:
 // four double-buffered accumulators and A in shared memory took 11.95 ms at
-// n = m = 262144, this 11.35 (2^20: 184.3, 176.4).  The exp pipe is then busy
+// n = m = 262144, this 11.24 (2^20: 184.3, 173).  The exp pipe is then busy
 // 62 % of the time, the tensor core 54 %, issue slots 55 %; the rest is the
 // latency of waits, TMEM loads and add chains that 16 warps of 96 registers
 // cannot hide.  Each query's sum is kept as two column halves by two threads

@@ -47,7 +47,8 @@
 // 24.1 ms with seven issuing warps of 80 registers and separate ragged and
 // diagonal blocks, 20.6 this way, 20.0 with one weighted-sum issuer instead
 // of one per query tile (its polling took issue slots) and five data stages
-// (2^20: 381, 328, 318).  Tried and slower: one warp for all MMAs (29.9), eight
+// (2^20: 381, 328, 318), 19.8 (316) with the waits' slow path out of line.
+// Tried and slower: one warp for all MMAs (29.9), eight
 // warps of 64 columns (28.6 ms), S and weights in separate columns with one
 // buffer each (25.9), the rare blocks as calls (21.6-22.3), the next tile's S
 // loaded ahead (25.0, spills).
