@@ -378,18 +378,24 @@ __global__ void __launch_bounds__(Q_THREADS) cell_query_kernel(const float* __re
     const float y = exp2f(-p);
     acc.add(fmaf(y, -e * 0.69314718055994531f, y) * s);
   };
+  // from the query to cell c's interval, in h: 0 inside it, so that a query
+  // far outside the data stops at the first cell on either side (visited at
+  // 1e5 h the moments' polynomial overflows; its weight there is 0)
+  auto gap = [&](int c) {
+    const float below = fmaf((float)c, st.w, st.lo) - qv, above = qv - fmaf((float)(c + 1), st.w, st.lo);
+    return fmaxf(0.f, fmaxf(below, above)) * inv_h;
+  };
   int right = own, left = own - 1;
   bool go_r = right < st.cells, go_l = left >= 0;
-  if (fabsf(qv) == __int_as_float(0x7f800000)) go_r = go_l = false;   // no mass at infinity
   while (go_r || go_l) {
     if (go_r) {
-      const float g = fmaxf(0.f, fmaf((float)right, st.w, st.lo) - qv) * inv_h;
+      const float g = gap(right);
       if (g * g * 0.72134752f > limit) go_r = false;
       else visit(right);
       if (++right >= st.cells) go_r = false;
     }
     if (go_l) {
-      const float g = fmaxf(0.f, qv - fmaf((float)(left + 1), st.w, st.lo)) * inv_h;
+      const float g = gap(left);
       if (g * g * 0.72134752f > limit) go_l = false;
       else visit(left);
       if (--left < 0) go_l = false;

@@ -1,0 +1,55 @@
+"""The range of the 1-D cell expansions: queries far outside the data, bandwidths,
+scales and sizes at the ends of what the FP32 tables hold, against the pair
+kernel (the same queries in chunks below the dispatch size) or the exact value.
+
+Where both sums are formed they are compared at 1e-5, the pair kernel's own
+exponent rounding in the far tail."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+PAIRS = 1 << 30
+FLT_MAX = 3.4028234663852886e38
+
+
+def _gen(seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return g
+
+
+def _mixture(n, seed):
+    g = _gen(seed)
+    x = torch.randn(n, generator=g, device="cuda")
+    u = torch.rand(n, generator=g, device="cuda")
+    return torch.where(u < 0.3, x * 0.3 - 2.0, torch.where(u < 0.7, x * 0.5 + 0.5, x * 0.8 + 3.0))
+
+
+def _pairs(q, x, h, **kw):
+    from fsk import ops
+
+    step = max(1, (PAIRS - 1) // x.numel())
+    return torch.cat([ops.kde1d_sum(q[i:i + step], x, h, **kw) for i in range(0, q.numel(), step)])
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_queries_far_from_the_data(cuda_dev, seed):
+    from fsk import ops
+
+    x = _mixture(1 << 20, seed)
+    lo, hi = float(x.min()), float(x.max())
+    h = 0.9 * float(x.std()) * x.numel() ** -0.2 * (1.0, 0.3, 4.0)[seed % 3]
+    steps = torch.tensor([0.0, 15.0, 20.0, 100.0, 1e3, 1e4, 1e5, 1e6, 1e9], dtype=torch.float64)
+    ends = torch.tensor([1e4, 1e5, 1e6, 1e9, 1e19, 3e19, 1e20, FLT_MAX, float("inf")], dtype=torch.float64)
+    q = torch.cat([hi + steps * h, lo - steps * h, ends, -ends, torch.linspace(lo, hi, 1100).double()])
+    q = q.float().to(cuda_dev)
+    assert x.numel() * q.numel() >= PAIRS
+    forms = [{}, {"atomic": True}, {"log_eps": 1e-12}, {"log_eps": 0.0}, {"out_scale": -2.0}]
+    for kw in forms:
+        got, want = ops.kde1d_sum(q, x, h, **kw), _pairs(q, x, h, **kw)
+        same = got == want   # zeros and infinities of the logarithm
+        near = (got - want).abs() <= 1e-5 * (want.abs() + ("log_eps" in kw))
+        assert (same | near).all(), (kw, q[~same], got[~same], want[~same])
+    ops.device_status(cuda_dev)
+    got = ops.kde1d_sum(q, x, h)
+    assert (got[1:9] == 0).all() and (got[10:18] == 0).all() and (got[18:36] == 0).all()
