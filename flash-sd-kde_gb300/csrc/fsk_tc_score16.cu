@@ -614,14 +614,18 @@ done:
 }  // namespace
 
 // Data tiles per W accumulation.  The tensor core's FP32 accumulation over a
-// group is the largest error of the weighted sums (debiased points against
-// FP64 at n = 6258: 3.2e-7 with one group of 16 tiles, 6e-8 with groups of 1
-// or 2), each group's read-out costs about half a tile.  Small problems, bound
-// by launches and not by tiles, take short groups; 14 below and 16 above 1024
-// tiles per CTA.
+// group is the largest error of the weighted sums and grows with its length
+// (debiased points against FP64, rows sorted by a feature: ~4e-8 per tile of
+// the group); each group's read-out costs about half a tile.  Small problems,
+// bound by launches and not by tiles, take short groups.  The lengths are
+// those of equal splits of every query block (2 or 3 tiles at n = 8000 to
+// 10000, 10 at 19500, 13 to 16 above) at the sizes where those were shortest:
+// with tiles / 8 here the error was up to twice as large between them.
 static int score_group(const TcPlan& pl) {
-  const int64_t tiles = pl.q_blocks * pl.n_tiles / pl.line.grid;
-  return tiles >= 1024 ? 16 : (int)imin<int64_t>(14, imax<int64_t>(1, tiles / 8));
+  const int64_t tiles = pl.q_blocks * pl.n_tiles / pl.line.grid;   // per CTA
+  if (tiles >= 16384) return 16;
+  if (tiles >= 1024) return 15;
+  return (int)imin<int64_t>(13, imax<int64_t>(1, tiles / 15));
 }
 
 TcPlan plan_score16(int64_t n) {
