@@ -48,16 +48,19 @@ __device__ __forceinline__ void load_row(const float* __restrict__ p, bool vec, 
   }
 }
 
-// Per-block column sums as (value, error) pairs: thread t adds feature t % 16
-// of the rows t / 16, t / 16 + 16, ... of the block's share.
-__global__ void __launch_bounds__(PT) tc_mean_kernel(const float* __restrict__ x, int64_t n,
+// Per-block column sums of x * down as (value, error) pairs: thread t adds
+// feature t % 16 of the rows t / 16, t / 16 + 16, ... of the block's share.
+// down: a power of two below 1 / (2 n), so that no partial sum overflows where
+// a column holds values near the largest float.
+__global__ void __launch_bounds__(PT) tc_mean_kernel(const float* __restrict__ x, int64_t n, float down,
                                                      float2* __restrict__ part) {
   pdl_launch_dependents();
   constexpr int L = PT / FSK_D;
   const int k = threadIdx.x % FSK_D, l = threadIdx.x / FSK_D;
   Comp a{0.f, 0.f};
 #pragma unroll 4
-  for (int64_t r = (int64_t)blockIdx.x * L + l; r < n; r += (int64_t)gridDim.x * L) a.add(x[r * FSK_D + k]);
+  for (int64_t r = (int64_t)blockIdx.x * L + l; r < n; r += (int64_t)gridDim.x * L)
+    a.add(x[r * FSK_D + k] * down);
   __shared__ float2 sh[PT];
   sh[threadIdx.x] = make_float2(a.s, a.c);
   __syncthreads();
@@ -72,7 +75,7 @@ __global__ void __launch_bounds__(PT) tc_mean_kernel(const float* __restrict__ x
 // The mean from the per-block sums into shared memory (every block, same
 // order, same bits).  Any centre would do: it is subtracted exactly as
 // rounded here and added back by the reductions.
-__device__ __forceinline__ void block_mean(const float2* __restrict__ part, int blocks, int64_t n,
+__device__ __forceinline__ void block_mean(const float2* __restrict__ part, int blocks, int64_t n, float down,
                                            float (&mu)[FSK_D], float2 (&sh)[PT]) {
   constexpr int L = PT / FSK_D;
   const int k = threadIdx.x % FSK_D, l = threadIdx.x / FSK_D;
@@ -84,9 +87,9 @@ __device__ __forceinline__ void block_mean(const float2* __restrict__ part, int 
   if (threadIdx.x < FSK_D) {
 #pragma unroll
     for (int j = 1; j < L; ++j) s = df_add(s, sh[j * FSK_D + threadIdx.x]);
-    const float nf = (float)n;
-    const float q = s.x / nf;
-    mu[threadIdx.x] = q + (fmaf(-q, nf, s.x) + s.y) / nf;
+    const float n2 = (float)n * (2.f * down);   // half the mean, which cannot round to infinity
+    const float q = s.x / n2;
+    mu[threadIdx.x] = 2.f * (q + (fmaf(-q, n2, s.x) + s.y) / n2);
   }
   __syncthreads();
 }
@@ -97,12 +100,13 @@ __device__ __forceinline__ void block_mean(const float2* __restrict__ part, int 
 // whose queries are the data).
 __global__ void __launch_bounds__(PT) tc_stats_kernel(const float* __restrict__ x, int64_t n,
                                                       const float* __restrict__ q, int64_t m, int vec, int data_blocks,
-                                                      int mean_blocks, float c2, float alpha_off, PrepBufs b) {
+                                                      int mean_blocks, float down, float c2, float alpha_off,
+                                                      PrepBufs b) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ float mu[FSK_D];
   __shared__ float2 sh[PT];
-  block_mean(b.mean_part, mean_blocks, n, mu, sh);
+  block_mean(b.mean_part, mean_blocks, n, down, mu, sh);
   if (blockIdx.x == 0 && threadIdx.x < FSK_D) b.mu[threadIdx.x] = mu[threadIdx.x];
   const bool data = (int)blockIdx.x < data_blocks;
   const float* pts = data ? x : q;
@@ -339,11 +343,12 @@ int launch_prep(const float* x, int64_t n, const float* q, int64_t m, double h, 
   const float c2 = (float)(FSK_LOG2E / (2.0 * h * h));
   const int vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(q)) & 15) == 0;
   const int mean_blocks = blocks_for(n, MEAN_MAX_BLOCKS);
-  tc_mean_kernel<<<mean_blocks, PT, 0, s>>>(x, n, b.mean_part);
+  const float down = ldexpf(1.f, -2 - (int)log2((double)n));
+  tc_mean_kernel<<<mean_blocks, PT, 0, s>>>(x, n, down, b.mean_part);
   count_launch();
   const int data_stats = blocks_for(n, STATS_MAX_BLOCKS);
   const int stats_blocks = data_stats + (SCORE ? 0 : blocks_for(m, STATS_MAX_BLOCKS));
-  launch_pdl(tc_stats_kernel, stats_blocks, PT, 0, s, x, n, q, m, vec, data_stats, mean_blocks, c2, alpha_off, b);
+  launch_pdl(tc_stats_kernel, stats_blocks, PT, 0, s, x, n, q, m, vec, data_stats, mean_blocks, down, c2, alpha_off, b);
   count_launch();
   ImageArgs a;
   a.x = x;
