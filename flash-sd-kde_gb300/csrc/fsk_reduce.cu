@@ -161,7 +161,8 @@ void launch_reduce_tc_rows(const tc::TcPartials& p, int64_t m, double scale, dou
 // the shift were bound by the FP64 unit (26 + 18 us at n = 65536).
 __global__ void __launch_bounds__(RED_THREADS) reduce_score_tc_kernel(tc::ScPartials p, int64_t n,
                                                                       const float* __restrict__ x, ScoreOut o,
-                                                                      float eps_hi, float eps_lo, double inv_h2) {
+                                                                      float eps_hi, float eps_lo, int eps_wide,
+                                                                      double eps64, double inv_h2) {
   constexpr int QB = 256;   // rows per query block
   pdl_wait();
   const int64_t e = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x;
@@ -195,12 +196,26 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_score_tc_kernel(tc::ScPart
   mp.y = fmaf(mk, ps.y, mp.y);
   const float2 wt = df_add(df_add(ws, mp), make_float2(xi, 0.f));
   const float2 pdf = df_add(ps, make_float2(1.0f, 0.f));
+  // beyond the pairs' range (eps, or a weighted sum past the largest float): FP64
+  const bool wide = eps_wide != 0 || !(fabsf(wt.x) < __int_as_float(0x7f800000));
+  float w = wt.x;
+  double off = 0.0;   // W / (pdf + eps) - x
+  if (__builtin_expect(wide, 0)) {
+    const double p64 = (double)ps.x + (double)ps.y, c64 = (double)ws.x + (double)ws.y;
+    w = (float)(c64 + (double)mk * p64 + (double)xi);
+    off = (c64 + ((double)mk - (double)xi) * p64) / (p64 + 1.0 + eps64) - (double)xi / (1.0 + (p64 + 1.0) / eps64);
+  }
   if (o.w) {
     const int64_t at = i * o.ws_row + k * o.ws_col;
-    if (in_bounds(at, n * FSK_D, 53)) o.w[at] = wt.x;
+    if (in_bounds(at, n * FSK_D, 53)) o.w[at] = w;
   }
   if (o.pdf && k == 0) o.pdf[i] = pdf.x;
   if (o.debiased) {
+    if (__builtin_expect(wide, 0)) {
+      o.debiased[e] = (float)(0.5 * off + (double)xi);
+      if (o.score) o.score[e] = (float)(off * inv_h2);
+      return;
+    }
     // m = W / (pdf + eps) as a quotient and its remainder over the divisor (pdf >= 1)
     const float2 d = df_add(pdf, make_float2(eps_hi, eps_lo));
     const float q = wt.x / d.x;
@@ -218,7 +233,7 @@ void launch_reduce_score_tc(const tc::ScPartials& p, int64_t n, const float* x, 
                             cudaStream_t s) {
   const float eps_hi = (float)eps, eps_lo = (float)(eps - (double)eps_hi);
   launch_pdl(reduce_score_tc_kernel, (int)((n * FSK_D + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s, p, n, x, o,
-             eps_hi, eps_lo, 1.0 / (h * h));
+             eps_hi, eps_lo, eps < 1e30 ? 0 : 1, eps, 1.0 / (h * h));
   count_launch();
 }
 

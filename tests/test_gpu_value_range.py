@@ -33,3 +33,33 @@ def test_constant_column_of_large_values(cuda_dev, value, n, m):
     rest = [k for k in range(16) if k != 5]
     assert torch.equal(pdf2, pdf)
     assert torch.equal(w2[:, rest], w[:, rest]) and torch.equal(deb2[:, rest], deb[:, rest])
+
+
+@pytest.mark.parametrize("eps", [1e29, 1e31, 1e38, 1e39, 1e300, float("inf")])
+def test_shift_with_a_large_eps(cuda_dev, eps):
+    """W / (pdf + eps) vanishes: half of each point, and the score -x / h^2."""
+    from fsk import ops
+
+    x, h = _rows(700, 3), 0.8
+    deb, pdf, w, score = ops.sdshift16(x, h, eps, return_debug=True)
+    one_call = ops.sdkde16(x, x[:100], h, eps=eps, return_debiased=True)[1]
+    ops.device_status(cuda_dev)
+    assert torch.equal(deb, 0.5 * x) and torch.equal(one_call, 0.5 * x)
+    want = -x.double() / (h * h)
+    assert ((score - want).abs() <= 2.0 ** -24 * want.abs()).all()
+    plain = ops.empscore16(x, h)
+    assert torch.equal(pdf, plain[0]) and torch.equal(w, plain[1])
+
+
+def test_weighted_sums_past_the_largest_float(cuda_dev):
+    """300 points at 1e37: their weighted sum 3e39 is infinite in FP32 and their
+    mean is not.  Sums within the 2e-6 of the score tests."""
+    from fsk import ops
+
+    x = torch.full((300, 16), 1e37, device=cuda_dev)
+    x[:, 3] = 2.0
+    deb, pdf, w, score = ops.sdshift16(x, 0.5, 0.0, return_debug=True)
+    ops.device_status(cuda_dev)
+    assert torch.equal(deb, x) and (score == 0).all()
+    assert ((pdf - 300).abs() <= 2e-6 * 300).all() and ((w[:, 3] - 600).abs() <= 2e-6 * 600).all()
+    assert torch.isposinf(w[:, 0]).all()
