@@ -471,7 +471,7 @@ int fsk_kde1d(const float* queries, int64_t m, const float* data, int64_t n, dou
   // sums cancel and stay with the pair kernel); their flag tells the pair
   // kernel on the device whether it is still needed.
   const int* skip = nullptr;
-  if (!laplace && cell1d_applies(m, n)) {
+  if (!laplace && cell1d_applies(m, n) && cell1d_holds(bandwidth)) {
     st = launch_cell1d(queries, m, data, n, bandwidth, out_scale, out_eps, log_out, c, out, &skip, s);
     if (st) return st;
   }

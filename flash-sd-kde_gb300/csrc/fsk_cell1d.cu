@@ -464,6 +464,11 @@ CellConsts cell_consts(double h) {
 // turns out too spread for the tables pays ~12 us for the attempt.
 bool cell1d_applies(int64_t m, int64_t n) { return n >= 4096 && (double)m * (double)n >= 1073741824.0; }
 
+// Bandwidths whose squares the FP32 tables hold: a visited cell's d^2 reaches
+// (16 h)^2, its rounding error and c2 = log2(e) / 2 h^2 have to stay normal.
+// Others take the pair kernel alone.
+bool cell1d_holds(double h) { return h >= 1e-15 && h <= 1e18; }
+
 void take_cell1d(WsCarver& c) { take_cells(c); }
 
 int launch_cell1d(const float* q, int64_t m, const float* x, int64_t n, double h, double scale, double eps,

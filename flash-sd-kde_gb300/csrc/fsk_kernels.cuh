@@ -45,6 +45,7 @@ void launch_kde1d_score(const float* q, int64_t m, const float* x, int64_t n, do
 // flag, 0 when the data is too spread for them and the direct kernels (given
 // the flag) have to run.
 bool cell1d_applies(int64_t m, int64_t n);
+bool cell1d_holds(double h);
 void take_cell1d(WsCarver& c);
 int launch_cell1d(const float* q, int64_t m, const float* x, int64_t n, double h, double scale, double eps,
                   bool log_out, WsCarver& c, float* out, const int** taken, cudaStream_t s);

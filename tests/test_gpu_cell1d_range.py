@@ -53,3 +53,21 @@ def test_queries_far_from_the_data(cuda_dev, seed):
     ops.device_status(cuda_dev)
     got = ops.kde1d_sum(q, x, h)
     assert (got[1:9] == 0).all() and (got[10:18] == 0).all() and (got[18:36] == 0).all()
+
+
+@pytest.mark.parametrize("h", [1e-300, 1e-160, 1e-40, 1e-30, 1e-22, 1e-16, 2e-15, 1e-10, 1e10, 9e17, 2e18, 1e20, 1e28, 1e29,
+                               1e30, 1e37, 3e38, 1e39, 1e160, 1e300])
+@pytest.mark.parametrize("unit", ["one", "h"])
+def test_bandwidths_of_any_size(cuda_dev, h, unit):
+    """Data of spread 1 and of spread h: finite where the pair kernel is, and equal."""
+    from fsk import ops
+
+    s = 1.0 if unit == "one" else min(max(h, 1e-37), 1e37)
+    x = (_mixture(1 << 18, 3).double() * s).float()
+    q = (torch.linspace(-12, 12, 4200, dtype=torch.float64, device="cuda") * s).float()
+    for kw in ({}, {"log_eps": 1e-12}):
+        got, want = ops.kde1d_sum(q, x, h, **kw), _pairs(q, x, h, **kw)
+        assert torch.equal(got.isnan(), want.isnan())
+        ok = (got == want) | ((got - want).abs() <= 1e-5 * (want.abs() + ("log_eps" in kw))) | want.isnan()
+        assert ok.all(), (kw, q[~ok], got[~ok], want[~ok])
+    ops.device_status(cuda_dev)
