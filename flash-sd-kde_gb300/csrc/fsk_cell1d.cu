@@ -491,7 +491,8 @@ int launch_cell1d(const float* q, int64_t m, const float* x, int64_t n, double h
   launch_pdl(cell_local_kernel, CELLS_MAX / 2, LOCAL_THREADS, 0, s, b, (float)log2((double)n), k);
   count_launch();
   float2 scale2 = make_float2(0.f, 0.f);
-  if (!log_out && fabs(scale) > 1e-30 && fabs(scale) < 1e30) {
+  // (a sum is at most n: no product beyond FP32, whose error would be infinite)
+  if (!log_out && fabs(scale) > 1e-30 && fabs(scale) * (double)n < 1e38) {
     scale2.x = (float)scale;
     scale2.y = (float)(scale - (double)scale2.x);
   }

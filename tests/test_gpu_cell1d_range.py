@@ -71,3 +71,18 @@ def test_bandwidths_of_any_size(cuda_dev, h, unit):
         ok = (got == want) | ((got - want).abs() <= 1e-5 * (want.abs() + ("log_eps" in kw))) | want.isnan()
         assert ok.all(), (kw, q[~ok], got[~ok], want[~ok])
     ops.device_status(cuda_dev)
+
+
+def test_densities_past_the_largest_float(cuda_dev):
+    """4e8 points at one place times 9e29 is infinite, not NaN; times 8e29 it is 3.2e38."""
+    from fsk import ops
+
+    n = 400_000_000
+    x = torch.full((n,), 1.5, device=cuda_dev)
+    q = torch.tensor([1.5, 1.5, 40.0], device=cuda_dev)
+    got = ops.kde1d_sum(q, x, 1.0, out_scale=9e29)
+    assert torch.isposinf(got[:2]).all() and float(got[2]) == 0.0
+    assert torch.isneginf(ops.kde1d_sum(q, x, 1.0, out_scale=-9e29)[:2]).all()
+    fits = ops.kde1d_sum(q, x, 1.0, out_scale=8e29)
+    ops.device_status(cuda_dev)
+    assert (fits[:2].double() / 3.2e38 - 1).abs().max() <= 5e-7
