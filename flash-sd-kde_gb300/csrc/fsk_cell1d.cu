@@ -462,7 +462,10 @@ CellConsts cell_consts(double h) {
 // Where the expansions are tried: at 2^30 pairs (131 us of pair sums) their
 // seven launches take ~40 us, half of that per point and query.  Data that
 // turns out too spread for the tables pays ~12 us for the attempt.
-bool cell1d_applies(int64_t m, int64_t n) { return n >= 4096 && (double)m * (double)n >= 1073741824.0; }
+// n <= 2^31: a point adds up to 1.5 x 2^31 to the signed 64-bit moments.
+bool cell1d_applies(int64_t m, int64_t n) {
+  return n >= 4096 && n <= (int64_t(1) << 31) && (double)m * (double)n >= 1073741824.0;
+}
 
 // Bandwidths whose squares the FP32 tables hold: a visited cell's d^2 reaches
 // (16 h)^2, its rounding error and c2 = log2(e) / 2 h^2 have to stay normal.

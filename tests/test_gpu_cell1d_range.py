@@ -86,3 +86,17 @@ def test_densities_past_the_largest_float(cuda_dev):
     fits = ops.kde1d_sum(q, x, 1.0, out_scale=8e29)
     ops.device_status(cuda_dev)
     assert (fits[:2].double() / 3.2e38 - 1).abs().max() <= 5e-7
+
+
+def test_more_than_2p32_points(cuda_dev):
+    """The sum of 2^32 + 2^26 equal points at their place (the 64-bit fixed-point
+    moments hold 2^31)."""
+    from fsk import ops
+
+    n = (1 << 32) + (1 << 26)
+    x = torch.full((n,), 0.5, device=cuda_dev)
+    q = torch.tensor([0.5, 1.5], device=cuda_dev)
+    got = ops.kde1d_sum(q, x, 1.0).double()
+    ops.device_status(cuda_dev)
+    want = n * torch.exp(torch.tensor([0.0, -0.5], dtype=torch.float64, device=cuda_dev))
+    assert ((got - want).abs() <= 5e-7 * want).all()
