@@ -47,9 +47,12 @@ struct SvBufs {
 };
 }  // namespace
 
+// Order-preserving key; positive NaNs come last.  As a xor and not as a choice
+// between ~u and u | sign bit: the latter can be compiled to a negation of the
+// float, which does not keep a NaN's bits (its key came out as 0x7FFFFFFF, -0).
 __device__ __forceinline__ uint32_t sortable_key(float f) {
-  uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+  const uint32_t u = __float_as_uint(f);
+  return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
 }
 __device__ __forceinline__ float key_to_float(uint32_t k) {
   uint32_t u = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
