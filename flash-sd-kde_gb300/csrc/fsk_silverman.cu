@@ -66,22 +66,25 @@ __device__ __forceinline__ int64_t target_rank(int64_t n, int t) {
 }
 
 // Digit of one statistic from its 256-bin histogram, by one warp holding 8 bins
-// per lane: the bin where the running count passes the rank.
-__device__ __forceinline__ SvPick pick_digit(uint4 u, uint4 v, SvPick p) {
+// per lane: the bin where the running count passes the rank.  RANK: the type of
+// ranks and running counts, 64 bits for the first digit of more than 2^32 rows
+// (a rank inside one bin fits 32).
+template <typename RANK>
+__device__ __forceinline__ SvPick pick_digit(uint4 u, uint4 v, uint32_t prefix, RANK rank) {
   const int lane = threadIdx.x & 31;
   const unsigned int c[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-  unsigned int total = 0;
+  RANK total = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) total += c[i];
-  unsigned int below = total;   // inclusive scan over lanes
+  RANK below = total;   // inclusive scan over lanes
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const unsigned int w = __shfl_up_sync(0xffffffffu, below, o);
+    const RANK w = __shfl_up_sync(0xffffffffu, below, o);
     if (lane >= o) below += w;
   }
   below -= total;
-  const bool mine = p.rank >= below && p.rank - below < total;
-  unsigned int left = p.rank - below;
+  const bool mine = rank >= below && rank - below < total;
+  RANK left = rank - below;
   int bin = 0;
 #pragma unroll
   for (int i = 0; i < 7; ++i) {
@@ -94,7 +97,7 @@ __device__ __forceinline__ SvPick pick_digit(uint4 u, uint4 v, SvPick p) {
   const unsigned int who = __ballot_sync(0xffffffffu, mine);
   const int src = who ? __ffs(who) - 1 : 31;
   const uint32_t digit = (uint32_t)__shfl_sync(0xffffffffu, 8 * lane + bin, src);
-  return SvPick{(p.prefix << 8) | digit, __shfl_sync(0xffffffffu, left, src)};
+  return SvPick{(prefix << 8) | digit, (uint32_t)__shfl_sync(0xffffffffu, left, src)};
 }
 
 // The selections after `digits` digits of columns [c0, c0 + dc) into shared
@@ -122,7 +125,10 @@ __device__ __forceinline__ void block_picks(const SvBufs& b, int64_t n, int d, i
     }
 #pragma unroll
     for (int i = 0; i < U; ++i) {
-      p[i] = pick_digit(u[i], v[i], p[i]);
+      if (q == 0 && n > 0xffffffffll)
+        p[i] = pick_digit<uint64_t>(u[i], v[i], 0u, (uint64_t)target_rank(n, min(s0 + i, stats - 1) % SV_TARGETS));
+      else
+        p[i] = pick_digit<uint32_t>(u[i], v[i], p[i].prefix, p[i].rank);
       if (lane == 0 && s0 + i < stats) {
         pick[s0 + i] = p[i];
         if (keep) b.pick[(int64_t)q * d * SV_TARGETS + c0 * SV_TARGETS + s0 + i] = p[i];

@@ -37,3 +37,24 @@ def test_nan_values(cuda_dev, n, d, share):
     ops.device_status(cuda_dev)
     assert math.isnan(got) == math.isnan(want), (got, want)
     assert math.isnan(want) or abs(got - want) <= 1e-12 * abs(want), (got, want)
+
+
+def test_more_than_2p32_rows(cuda_dev):
+    """Ranks beyond 32 bits: 6e9 rows, 5860000 copies of the values v |v|, v = -512
+    .. 511.  std 512^2 / sqrt 5 is above IQR / 1.34, so the quartiles decide."""
+    from fsk import ops
+
+    copies = 5_860_000
+    v = torch.arange(-512, 512, device=cuda_dev, dtype=torch.float32)
+    v = v * v.abs()
+    x = v.repeat(copies).view(-1, 1)
+    n = x.shape[0]
+    assert 0.75 * (n - 1) > 1 << 32
+    got = float(ops.silverman(x))
+    ops.device_status(cuda_dev)
+    del x
+    w = v.double()
+    q25 = float(torch.lerp(w[255], w[256], 0.75))   # 0.25 (n - 1) = 256 copies - 0.25
+    q75 = float(torch.lerp(w[767], w[768], 0.25))
+    want = 0.9 * (q75 - q25) / 1.34 * n ** -0.2
+    assert abs(got - want) <= 1e-12 * want
