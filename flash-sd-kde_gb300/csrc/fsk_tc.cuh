@@ -133,22 +133,24 @@ struct Segment {
   int qb, t0, count;   // query block, first data tile, tiles
 };
 
-// The segment of CTA b that begins after `done` of its tiles; count = 0 at the
-// end.  (`done` is the only state a role keeps across its tile loop, where
-// the epilogue warps have no registers to spare.)
-__host__ __device__ inline Segment segment_at(const WorkLine& w, int b, int done) {
+// Segment k of CTA b: its whole query blocks, then the one or two that its
+// share of the line (at most n_tiles tiles) falls into; count = 0 at the end.
+// (k is the only state a role keeps across its tile loop, where the epilogue
+// warps have no registers to spare, and stays small: a count of tiles would
+// pass 2^31 at 1e8 points and queries.)
+__host__ __device__ inline Segment segment_at(const WorkLine& w, int b, int k) {
   Segment g;
-  const int n_tiles = (int)w.n_tiles, k = done / n_tiles;
   if (k < w.whole) {
     g.qb = b + k * w.grid;
     g.t0 = 0;
-    g.count = n_tiles;
+    g.count = (int)w.n_tiles;
   } else {
-    const int64_t L = w.begin(b) + (done - w.whole * n_tiles);
-    const int64_t r = L / n_tiles;
+    const int64_t L0 = w.begin(b), L1 = w.begin((int64_t)b + 1);
+    const int64_t r = L0 / w.n_tiles + (k - w.whole);   // query block of the line
+    const int64_t L = imax<int64_t>(L0, r * w.n_tiles);
     g.qb = (int)r + w.whole * w.grid;
-    g.t0 = (int)(L - r * n_tiles);
-    g.count = (int)imin<int64_t>(n_tiles - g.t0, w.begin((int64_t)b + 1) - L);
+    g.t0 = (int)(L - r * w.n_tiles);
+    g.count = (int)imax<int64_t>(0, imin<int64_t>((r + 1) * w.n_tiles, L1) - L);
   }
   return g;
 }

@@ -63,8 +63,8 @@ namespace tc {
 
 // Out of line: inlined into the three roles it costs the epilogue 8 bytes of
 // spills per tile (192 against 186 ms at n = m = 2^20).
-static __device__ __noinline__ Segment next_segment(const WorkLine& w, int done) {
-  return segment_at(w, blockIdx.x, done);
+static __device__ __noinline__ Segment next_segment(const WorkLine& w, int k) {
+  return segment_at(w, blockIdx.x, k);
 }
 
 // SINGLE: the single-pass precision rung (FSK_PREC_FP16_SINGLE) - only the
@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
   uint64_t* sdone = qready + 2;          // the MMAs of the segment finished
   uint64_t* drain = sdone + 1;           // all MMAs of this CTA finished (exit path)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
-  uint32_t n_stage_copies = 0, n_query_copies = 0;   // producer: bulk copies issued
+  uint32_t n_stage_copies = 0;   // producer: bulk copies issued
+  uint32_t n_query_copies = 0;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -129,10 +130,10 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       uint32_t& k = n_query_copies;
       int s = 0;
       uint32_t ph = 0;
-      for (int done_tiles = 0;;) {
-        const Segment sg = next_segment(p.line, done_tiles);
+      for (int k_seg = 0;; ++k_seg) {
+        const Segment sg = next_segment(p.line, k_seg);
         if (sg.count == 0) break;
-        done_tiles += sg.count;
+        if (g >= 1u << 30) g = 2 * NS + g % (2 * NS);   // stage and phase of the last copies are kept
         if (!__all_sync(0xffffffffu, mbar_wait_cold(qempty, (k & 1u) ^ 1u, 1))) goto done;
         if (lane == 0) {
           mbar_arrive_expect_tx(qready, A_BYTES);
@@ -175,17 +176,17 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       const uint64_t b_m0 = smem_desc_kmajor(bs0 + KB_M_OFFSET, 128, 8 * L_ROW_BYTES);
       const uint64_t b_l0 = smem_desc_kmajor(bs0 + KB_L_OFFSET, 128, 8 * L_ROW_BYTES);
       const uint32_t ta = tmem_base + (uint32_t)T_KA;   // per query tile, hi: features | bias; mid at +16, lo at +24
-      uint32_t k = 0, ph = 0;
+      uint32_t ph = 0;
       int s = 0;
       int g = 0;            // data tile
       int acc = 0;          // u % NACC
-      for (int done_tiles = 0;; ++k) {
-        const int nt = next_segment(p.line, done_tiles).count;
+      for (int k = 0;; ++k) {
+        const int nt = next_segment(p.line, k).count;
         if (nt == 0) break;
-        done_tiles += nt;
-        if (!__all_sync(0xffffffffu, mbar_wait_cold(qready, k & 1u, 3))) goto done;
+        if (g >= 1 << 30) g = 8 + (g & 7);   // its low bits count; a segment has fewer than 2^30 tiles
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(qready, (uint32_t)k & 1u, 3))) goto done;
         // the previous segment's MMAs have read its operand
-        if (k > 0 && !__all_sync(0xffffffffu, mbar_wait_cold(sdone, (k - 1) & 1u, 10))) goto done;
+        if (k > 0 && !__all_sync(0xffffffffu, mbar_wait_cold(sdone, (uint32_t)(k - 1) & 1u, 10))) goto done;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -242,17 +243,16 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
     // slot float4 kk of thread t at [kk][t]: a warp's 16-byte accesses are contiguous
     float4* qslot = reinterpret_cast<float4*>(smem_raw + K_QX_OFFSET) + (warp * 32 + lane);
     constexpr int QS_STRIDE = EPI_WARPS * 32;
-    int g = 0;     // data tile
+    uint32_t g = 0;   // data tile
     int ab = qt;   // its accumulator, (2 g + qt) % NACC
     int s = 0;
     const int last_t = (int)p.line.n_tiles - 1;
     // valid columns of this thread's half of the last (possibly ragged) data
     // tile; every other tile has KNT / 2
     const int last_valid = (int)imin<int64_t>(KNT / 2, p.n - ((int64_t)last_t * KNT + half * (KNT / 2)));
-    for (int done_tiles = 0;;) {
-      const Segment sg = next_segment(p.line, done_tiles);
+    for (int k_seg = 0;; ++k_seg) {
+      const Segment sg = next_segment(p.line, k_seg);
       if (sg.count == 0) break;
-      done_tiles += sg.count;
       const int qrow = qt * QT + quarter * 32 + lane;                   // row in the query block
       const int64_t gi = (int64_t)sg.qb * (NQT * QT) + qrow;            // padded query index
       // this query's FP32 row into the thread's own shared-memory slot (read
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(THREADS, 1) kde16_tc_kernel(TcParams p) {
       for (int i = 0; i < nt; ++i, ++g) {
         const int valid = i == last_i ? last_valid : KNT / 2;   // may be <= 0 on the last tile
         // (a timed-out wait ends the whole warp: it must stay converged)
-        if (!__all_sync(0xffffffffu, mbar_wait_cold(&tfull[qt * 4 + (g & 3)], (uint32_t)(g >> 2) & 1u, 6))) goto done;
+        if (!__all_sync(0xffffffffu, mbar_wait_cold(&tfull[qt * 4 + (g & 3)], (g >> 2) & 1u, 6))) goto done;
         tc_fence_after();
         const uint8_t* xrows = sB + s * KB_STAGE_BYTES + KB_X_OFFSET + half * (KNT / 2) * (FSK_D * 4);
         float tsum = 0.f;
@@ -397,8 +397,8 @@ done:
   // Exit path (also after a timed-out wait): let this CTA's bulk copies and
   // MMAs finish before shared and tensor memory are released.
   if (warp == PRODUCER_WARP && lane == 0) {
-    for (uint32_t i = n_stage_copies > (uint32_t)NS ? n_stage_copies - NS : 0u; i < n_stage_copies; ++i)
-      mbar_wait_cold(&full[i % NS], (i / NS) & 1u, 7);
+    for (uint32_t i = n_stage_copies > NS ? n_stage_copies - NS : 0u; i < n_stage_copies; ++i)
+      mbar_wait_cold(&full[i % NS], (uint32_t)(i / NS) & 1u, 7);
     if (n_query_copies > 0) mbar_wait_cold(qready, (n_query_copies - 1) & 1u, 8);
   }
   if (warp == MMA_WARP && elect_one()) {

@@ -204,10 +204,9 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       int64_t& k = n_query_copies;
       int st = 0;
       uint32_t ph = 0;
-      for (int done_tiles = 0;;) {
-        const Segment sg = segment_at(p.line, blockIdx.x, done_tiles);
+      for (int k_seg = 0;; ++k_seg) {
+        const Segment sg = segment_at(p.line, blockIdx.x, k_seg);
         if (sg.count == 0) break;
-        done_tiles += sg.count;
         if (!__all_sync(0xffffffffu, mbar_wait_cold(qempty, (uint32_t)((k & 1) ^ 1), 21))) goto done;
         if (lane == 0) {
           mbar_arrive_expect_tx(qready, S_A_BYTES + S_QX_BYTES);
@@ -245,27 +244,26 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       const uint64_t dh0 = smem_desc_kmajor(b0, 128, 8 * H_ROW_BYTES);
       const uint64_t dm0 = smem_desc_kmajor(b0 + B_M_OFFSET, 128, 8 * L_ROW_BYTES);
       const uint64_t dl0 = smem_desc_kmajor(b0 + B_L_OFFSET, 128, 8 * L_ROW_BYTES);
-      int gs = 0, ku = 0;
-      for (int done_tiles = 0;;) {
-        const int count = segment_at(p.line, blockIdx.x, done_tiles).count;
+      uint32_t gs = 0;     // data tile (modulo 2^32: only its low bits are used)
+      int s = 0;           // its stage
+      uint32_t sph = 0;    // and that one's phase
+      for (int ku = 0;; ++ku) {
+        const int count = segment_at(p.line, blockIdx.x, ku).count;
         if (count == 0) break;
-        done_tiles += count;
         for (int i = 0; i < count; ++i, ++gs) {
-          const int s = gs % SNS;
-          const int b = gs % NBUF;
-          if (!__all_sync(0xffffffffu, mbar_wait_cold(&full[s], (uint32_t)((gs / SNS) & 1), 24))) goto done;
+          const uint32_t b = gs % NBUF;
+          if (!__all_sync(0xffffffffu, mbar_wait_cold(&full[s], sph, 24))) goto done;
           const uint64_t so = (uint64_t)((s * S_STAGE_BYTES) >> 4);
           const uint64_t b_h = dh0 + so, b_m = dm0 + so, b_l = dl0 + so;
 #pragma unroll
           for (int a = 0; a < SNQT; ++a) {
             // the segment's A operand in TMEM
             if (i == 0 && !__all_sync(0xffffffffu, mbar_wait_cold(&aready[a], (uint32_t)(ku & 1), 23))) goto done;
-            if (gs >= NBUF &&
-                !__all_sync(0xffffffffu, mbar_wait_cold(&sfree[b * SNQT + a], (uint32_t)(((gs / NBUF) - 1) & 1), 25)))
-              goto done;
+            // (before the first tiles: a phase that has passed)
+            if (!__all_sync(0xffffffffu, mbar_wait_cold(&sfree[b * SNQT + a], ((gs / NBUF) & 1u) ^ 1u, 25))) goto done;
             tc_fence_after();
             const uint32_t a_h = tmem_base + (uint32_t)(T_A + a * 32);   // hi: features | bias; mid at +16, lo at +24
-            const uint32_t d = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
+            const uint32_t d = tmem_base + T_S + b * (SNQT * NT) + (uint32_t)(a * NT);
             // three-part product, small terms first (the order of mma_s_tile)
             if (elect_one()) {
               mma_s_tile(d, a_h, b_h, b_m, b_l, idesc_s);
@@ -273,8 +271,11 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
             }
             __syncwarp();
           }
+          if (++s == SNS) {
+            s = 0;
+            sph ^= 1u;
+          }
         }
-        ++ku;
       }
     }
   } else if (warp == W_MMA_WARP) {
@@ -283,29 +284,28 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
     {
       const uint32_t idesc_hi = idesc_f16_f32(QT, WN), idesc_lo = idesc_f16_f32(QT, WN_LO);
       const uint64_t dx0 = smem_desc_kmajor(smem_u32(sB) + S_XTH_OFFSET, 128, 8 * XT_ROW_BYTES);
-      int gw = 0, grp = 0;
-      for (int done_tiles = 0;;) {
-        const int count = segment_at(p.line, blockIdx.x, done_tiles).count;
+      uint32_t gw = 0, grp = 0;   // data tile and group (modulo 2^32)
+      int s = 0;                  // the tile's stage
+      for (int k_seg = 0;; ++k_seg) {
+        const int count = segment_at(p.line, blockIdx.x, k_seg).count;
         if (count == 0) break;
-        done_tiles += count;
         int left = 0;   // tiles left in the group
-        for (int i = 0; i < count; ++i, ++gw) {
-          const int b = gw % NBUF;
-          const int s = gw % SNS;
+        for (int i = 0; i < count; ++i, ++gw, s = (s + 1 == SNS) ? 0 : s + 1) {
+          const uint32_t b = gw % NBUF;
           const bool first = left == 0;
           if (first) left = p.group;
           const bool last = --left == 0 || i == count - 1;
-          const int par = grp & 1;
+          const uint32_t par = grp & 1u;
 #pragma unroll
           for (int a = 0; a < SNQT; ++a) {
             if (first &&
-                !__all_sync(0xffffffffu, mbar_wait_cold(&wempty[par * SNQT + a], (uint32_t)(((grp >> 1) & 1) ^ 1), 26)))
+                !__all_sync(0xffffffffu, mbar_wait_cold(&wempty[par * SNQT + a], ((grp >> 1) & 1u) ^ 1u, 26)))
               goto done;
-            if (!__all_sync(0xffffffffu, mbar_wait_cold(&pready[b * SNQT + a], (uint32_t)((gw / NBUF) & 1), 27))) goto done;
+            if (!__all_sync(0xffffffffu, mbar_wait_cold(&pready[b * SNQT + a], (gw / NBUF) & 1u, 27))) goto done;
             tc_fence_after();
             const uint64_t xd0 = dx0 + (uint64_t)((s * S_STAGE_BYTES) >> 4);
-            const uint32_t ph = tmem_base + (uint32_t)(T_S + b * (SNQT * NT) + a * NT);
-            const uint32_t d = tmem_base + (uint32_t)(T_W + par * (SNQT * W_TILE_COLS) + a * W_TILE_COLS);
+            const uint32_t ph = tmem_base + T_S + b * (SNQT * NT) + (uint32_t)(a * NT);
+            const uint32_t d = tmem_base + T_W + par * (SNQT * W_TILE_COLS) + (uint32_t)(a * W_TILE_COLS);
             if (elect_one()) {
 #pragma unroll
               for (int ks = 0; ks < NT / 16; ++ks) {
@@ -348,15 +348,14 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
       for (int k = 0; k < FSK_D; k += 4)
         *reinterpret_cast<float4*>(wcorr + par * WC_PAR + half * WC_HALF + wc_row + k) =
             make_float4(0.f, 0.f, 0.f, 0.f);
-    int g = 0, grp = 0, k_unit = 0;
+    uint32_t g = 0, grp = 0;   // data tile and W group (modulo 2^32)
     int s = 0;   // data stage of tile g (g % SNS, advanced per tile)
     // valid columns of the last (possibly ragged) data tile; every other tile has NT
     const int last_t = (int)p.line.n_tiles - 1;
     const int last_valid = (int)(p.n - (int64_t)last_t * NT);
-    for (int done_tiles = 0;; ++k_unit) {
-      const Segment sg = segment_at(p.line, blockIdx.x, done_tiles);
+    for (int k_unit = 0;; ++k_unit) {
+      const Segment sg = segment_at(p.line, blockIdx.x, k_unit);
       if (sg.count == 0) break;
-      done_tiles += sg.count;
       const int qb = sg.qb;
       const int gi = qb * (SNQT * QT) + qt * QT + row;
       const int diag_col = qb * (SNQT * QT) + qt * QT + quarter * 32;   // this warp's rows
