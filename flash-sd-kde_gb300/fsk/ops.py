@@ -236,6 +236,16 @@ def _sdshift16(x: torch.Tensor, h: float, eps: float, dev: torch.device, symmetr
     return (deb, pdf, w.t() if feature_major else w, score) if return_debug else deb
 
 
+def _sdkde16_flags(precision: str = "tensor", log_eps: float | None = None, log_exact: bool = False,
+                   atomic: bool = False, **_) -> int:
+    flags = (L.FSK_PREC_IEEE if precision == "ieee" else 0) | (L.FSK_ATOMIC if atomic else 0)
+    if log_exact:
+        flags |= L.FSK_OUT_LOG_EXACT
+    if log_exact or log_eps is not None:
+        flags |= L.FSK_OUT_LOG
+    return flags
+
+
 def sdkde16(
     data: torch.Tensor,
     queries: torch.Tensor,
@@ -265,14 +275,9 @@ def sdkde16(
         raise ValueError("data and queries must contain at least one sample.")
     if precision not in ("tensor", "ieee"):
         raise ValueError(f"unknown precision {precision!r}")
-    flags = (L.FSK_PREC_IEEE if precision == "ieee" else 0) | (L.FSK_ATOMIC if atomic else 0)
-    if log_exact:
-        if log_eps:
-            raise ValueError("log_exact takes no log_eps (the log is taken without a floor).")
-        log_eps = 0.0
-        flags |= L.FSK_OUT_LOG_EXACT
-    if log_eps is not None:
-        flags |= L.FSK_OUT_LOG
+    if log_exact and log_eps:
+        raise ValueError("log_exact takes no log_eps (the log is taken without a floor).")
+    flags = _sdkde16_flags(precision, log_eps, log_exact, atomic)
     if out_scale is None:
         out_scale = 1.0 / ((2.0 * math.pi) ** 8 * h ** 16 * n)
     lib = L.load()
@@ -301,9 +306,8 @@ class SDKDEGraph:
         self.data = as_matrix(data, dev).clone()
         self.queries = as_matrix(queries, dev).clone()
         self.out = torch.empty(self.queries.shape[0], dtype=torch.float32, device=dev)
-        flags = L.FSK_PREC_IEEE if kw.get("precision") == "ieee" else 0
         self.workspace = _workspace(L.load().fsk_sdkde16_workspace_bytes(self.data.shape[0], self.queries.shape[0],
-                                                                         flags), dev)
+                                                                         _sdkde16_flags(**kw)), dev)
         self._call = lambda: sdkde16(self.data, self.queries, bandwidth, out=self.out, workspace=self.workspace,
                                      **kw)
         side = torch.cuda.Stream(dev)
