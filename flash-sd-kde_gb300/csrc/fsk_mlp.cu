@@ -364,8 +364,8 @@ TrainBufs carve_train(WsCarver& c, int members, int64_t batch) {
   for (int l = 0; l < 3; ++l) {
     t.z[l] = c.take<float>(act);
     t.a[l] = c.take<__nv_bfloat16>(act);
-    t.dz[l] = c.take<float>(act);
   }
+  for (int l = 0; l < 2; ++l) t.dz[l] = c.take<float>(act);
   return t;
 }
 
@@ -404,7 +404,7 @@ void launch_backward(const float* params, int members, int64_t batch, const Trai
   const int64_t act = batch * MLP_H;
   const int row_blocks = (int)imin<int64_t>(512, (batch + 63) / 64);
   output_bwd_kernel<<<dim3((unsigned)row_blocks, (unsigned)members), MLP_H, 0, s>>>(params, t.a[2], t.z[2], dy,
-                                                                                     batch, members, t.dz[2], grads);
+                                                                                     batch, members, t.dz[0], grads);
   count_launch();
   const int64_t w_off[3] = {OFF_W1, OFF_W2, OFF_W3}, b_off[3] = {OFF_B1, OFF_B2, OFF_B3};
   const int64_t wq_off[3] = {WQ_W1, WQ_W2, WQ_W3};
@@ -412,7 +412,7 @@ void launch_backward(const float* params, int members, int64_t batch, const Trai
   for (int l = 2; l >= 0; --l) {
     // weight gradient: dW_l[o][k] = sum_b dz[b][o] a_{l-1}[b][k], split over the batch
     GemmArgs g{};
-    g.A = t.dz[l];
+    g.A = t.dz[l & 1];
     g.lda = MLP_H;
     g.sA = act;
     g.B = l == 0 ? t.a0 : t.a[l - 1];
@@ -432,7 +432,7 @@ void launch_backward(const float* params, int members, int64_t batch, const Trai
     gemm<true, true, EPI_ATOMIC, 128, float>(g, MLP_H, members, s);
     // data gradient into the layer below: dz_{l-1} = (dz W_l) * silu'(z_{l-1})
     GemmArgs d{};
-    d.A = t.dz[l];
+    d.A = t.dz[l & 1];
     d.lda = d.ldb = d.ldc = MLP_H;
     d.sA = act;
     d.B = t.w + wq_off[l];
@@ -440,7 +440,7 @@ void launch_backward(const float* params, int members, int64_t batch, const Trai
     d.M = (int)batch;
     d.K = d.k_chunk = MLP_H;
     d.splits = 1;
-    d.C = t.dz[l - 1];
+    d.C = t.dz[(l - 1) & 1];
     d.sC = act;
     d.Zprev = t.z[l - 1];
     gemm<false, true, EPI_DGRAD, 128, float>(d, MLP_H, members, s);

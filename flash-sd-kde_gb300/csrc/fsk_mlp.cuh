@@ -28,7 +28,7 @@ struct TrainBufs {
   __nv_bfloat16* w;      // [members][W1 | W2 | W3] bf16 weights of the current call
   float* z[3];           // [members][batch][256] pre-activations
   __nv_bfloat16* a[3];   // [members][batch][256] activations
-  float* dz[3];          // [members][batch][256] gradients of the pre-activations
+  float* dz[2];          // [members][batch][256] gradients of the pre-activations, layer l in dz[l & 1]
 };
 
 TrainBufs carve_train(WsCarver& c, int members, int64_t batch);

@@ -10,10 +10,13 @@ using namespace fsk;
 namespace {
 constexpr int MAX_MEMBERS = 8;
 bool bad_members(int m) { return m < 1 || m > MAX_MEMBERS; }
+// 26 bytes per activation, the inputs and the bf16 weights; never below the 28
+// that the interface has asked for from the first, so that sizes which were
+// valid stay so.
 size_t train_bytes(int members, int64_t batch) {
   WsCarver c(nullptr, 0);
   mlp::carve_train(c, members, batch);
-  return align_up(c.used, 256);
+  return align_up(imax<size_t>(c.used, (size_t)28 * members * batch * mlp::MLP_H), 256);
 }
 }  // namespace
 
