@@ -59,7 +59,7 @@ K_OPS_PER_POLY_EXP = 10.0
 KERNEL_NAMES = {1: "kde16_tc_kernel", 2: "kde16_simt_kernel", 3: "score16_simt_kernel",
                 4: "score16_sym_simt_kernel", 5: "kde1d_kernel", 6: "kde1d_score_kernel",
                 7: "score16_tc_kernel", 9: "mlp_infer_kernel", 10: "kde16_logspace_kernel",
-                11: "kde_nd_kernel", 12: "score_nd_kernel", 13: "cell_query_kernel"}
+                11: "kde_nd_kernel", 12: "score_nd_kernel", 13: "kde1d_cells (all launches of the call)"}
 # Tensor-core flops per pair evaluation.  "issued": what the tcgen05 kernels
 # execute (three-part fp16 operands: seven K=16 MMAs for the exponent; the
 # score kernel's weighted sums as fp16 hi/lo weights times [X_hi | X_lo] and

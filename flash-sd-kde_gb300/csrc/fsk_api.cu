@@ -471,14 +471,20 @@ int fsk_kde1d(const float* queries, int64_t m, const float* data, int64_t n, dou
   // sums cancel and stay with the pair kernel); their flag tells the pair
   // kernel on the device whether it is still needed.
   const int* skip = nullptr;
+  auto pairs = [&]() {
+    if (atomic) launch_zero(part, m, s);
+    launch_kde1d(queries, m, data, n, bandwidth, laplace, splits, atomic ? nullptr : part, atomic ? part : nullptr, skip,
+                 s);
+    launch_reduce_rows(part, atomic ? 1 : splits, m, out_scale, out_eps, log_out, out, skip, s);
+  };
   if (!laplace && cell1d_applies(m, n) && cell1d_holds(bandwidth)) {
+    TimerScope ts(K_KDE1D_CELL, (double)m * (double)n, s);   // whichever path the device takes
     st = launch_cell1d(queries, m, data, n, bandwidth, out_scale, out_eps, log_out, c, out, &skip, s);
     if (st) return st;
+    pairs();
+  } else {
+    pairs();
   }
-  if (atomic) launch_zero(part, m, s);
-  launch_kde1d(queries, m, data, n, bandwidth, laplace, splits, atomic ? nullptr : part, atomic ? part : nullptr, skip,
-               s);
-  launch_reduce_rows(part, atomic ? 1 : splits, m, out_scale, out_eps, log_out, out, skip, s);
   return cuda_status(cudaGetLastError());
 }
 

@@ -499,12 +499,9 @@ int launch_cell1d(const float* q, int64_t m, const float* x, int64_t n, double h
     scale2.x = (float)scale;
     scale2.y = (float)(scale - (double)scale2.x);
   }
-  {
-    TimerScope ts(K_KDE1D_CELL, (double)m * (double)n, s);
-    e = launch_pdl(cell_query_kernel, (int)((m + Q_THREADS - 1) / Q_THREADS), Q_THREADS, 0, s, q, m,
-                   (float)log2((double)n), k.inv_h, k.c2, k.c2_lo, scale, eps, log_out ? 1 : 0, scale2, b, out);
-    count_launch();
-  }
+  e = launch_pdl(cell_query_kernel, (int)((m + Q_THREADS - 1) / Q_THREADS), Q_THREADS, 0, s, q, m, (float)log2((double)n),
+                 k.inv_h, k.c2, k.c2_lo, scale, eps, log_out ? 1 : 0, scale2, b, out);
+  count_launch();
   return cuda_status(e);
 }
 

@@ -77,7 +77,7 @@ enum KernelId {
   K_KDE16_LOGSPACE = 10,   // shifted recompute of underflowing queries (work not known on the host)
   K_KDE_ND = 11,
   K_SCORE_ND = 12,
-  K_KDE1D_CELL = 13,   // 1-D KDE by cell expansions (work unit: the pairs it stands for)
+  K_KDE1D_CELL = 13,   // 1-D KDE where cell expansions are tried, all launches (work unit: the pairs it stands for)
 };
 
 // Host-side NVTX range around one C-ABI entry point, so profilers (ncu

@@ -319,7 +319,8 @@ FSK_API int fsk_diag_pipe_rates(double* rates_out, void* stream);
 /* Kernel ids: 1 tensor-core 16-D KDE, 2 CUDA-core 16-D KDE, 3 CUDA-core
  * ordered score, 4 CUDA-core symmetric score, 5 1-D KDE, 6 1-D KDE score,
  * 7 tensor-core score, 9 surrogate inference (unit: one query x member),
- * 13 1-D KDE by cell expansions (unit: the pairs it stands for). */
+ * 13 1-D KDE where cell expansions are tried: all launches of the call, pair
+ * kernel included where the data is too spread (unit: the pairs it stands for). */
 /* When enabled, each hot-path kernel launch is bracketed by CUDA events on
  * its own stream. */
 FSK_API void fsk_timer_enable(int on);
