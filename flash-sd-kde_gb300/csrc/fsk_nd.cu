@@ -70,7 +70,10 @@ __global__ void __launch_bounds__(ND_THREADS, DP == 16 ? 7 : 4) kde_nd_kernel(co
   const int64_t n_tiles = (n + ND_TN - 1) / ND_TN;
   const int64_t t0 = (int64_t)blockIdx.y * tps;
   const int64_t t1 = min(n_tiles, t0 + tps);
-  // the next tile's values are loaded while the present one is summed
+  // the next tile's values are loaded while the present one is summed, except
+  // at DP = 32, whose registers leave no room for it (d = 24, 30000 x 30000:
+  // 1927 us without, 1939 with; d = 8 1159 and 1149, d = 64 5.98 and 4.99 ms)
+  constexpr bool AHEAD = DP != 32;
   constexpr int ITEMS = ND_TN * DP / ND_THREADS;
   float next[ITEMS];
   auto fetch = [&](int64_t tile) {
@@ -82,15 +85,17 @@ __global__ void __launch_bounds__(ND_THREADS, DP == 16 ? 7 : 4) kde_nd_kernel(co
       next[i] = (r < valid && k < d) ? x[(j0 + r) * d + k] : 0.f;
     }
   };
-  if (t0 < t1) fetch(t0);
+  if (AHEAD && t0 < t1) fetch(t0);
   for (int64_t t = t0; t < t1; ++t) {
     const int64_t j0 = t * ND_TN;
     const int valid = (int)imin<int64_t>(ND_TN, n - j0);
     __syncthreads();
+    if (!AHEAD) stage_rows<DP>(xs, x, j0, valid, d);
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) xs[(threadIdx.x + i * ND_THREADS) / DP][(threadIdx.x + i * ND_THREADS) % DP] = next[i];
+    for (int i = 0; AHEAD && i < ITEMS; ++i)
+      xs[(threadIdx.x + i * ND_THREADS) / DP][(threadIdx.x + i * ND_THREADS) % DP] = next[i];
     __syncthreads();
-    if (t + 1 < t1) fetch(t + 1);
+    if (AHEAD && t + 1 < t1) fetch(t + 1);
     if constexpr (QPT == 2) {
       // both queries in every f32x2 instruction: the roundings of the scalar
       // code below, half the issue slots
@@ -250,32 +255,39 @@ __global__ void debias_nd_kernel(const float* __restrict__ x, int64_t n, int d, 
 }
 
 // Splits of the data for ~16 blocks per SM; with the kernel's blocks per SM
-// given, down to a quarter of that where the waves then cost at least 3 %
-// less (Laplace, d = 32, 20000 points at 5000 queries: 105 splits are 3.45
-// waves of 6 tiles, 30 are one of 21: 291 -> 256 us, d = 64 677 -> 570; where
-// the model sees no difference the count stays).
-int nd_splits(int64_t row_blocks, int64_t n, int resident) {
+// given, down to a quarter of that where whole waves are then cheaper (a wave
+// costs its tiles and a quarter for a block's start).  Laplace, d = 32, 20000
+// points at 5000 queries: 105 splits are 3.45 waves of 6 tiles, 30 are one of
+// 21, 275 -> 250 us.  With two queries per thread (d <= 32) the FP32 pipe is
+// full in a part of a wave as well, so there only the starts of short blocks
+// count (d = 8, 5000 x 50000: 13 tiles a block in 2.4 waves 328 us, 32 in one
+// 353; d = 64, 30000 x 30000: 4.98 -> 4.86 ms by waves).
+int nd_splits(int64_t row_blocks, int64_t n, int resident, bool short_only) {
   const int64_t n_tiles = (n + ND_TN - 1) / ND_TN;
   const int64_t target = 4LL * sm_count() * 4;
   int64_t most = (target + row_blocks - 1) / row_blocks;
   most = imax<int64_t>(1, imin<int64_t>(most, imax<int64_t>(1, n_tiles / 4)));
   most = imin<int64_t>(most, 65535);
-  const int64_t slots = resident * (int64_t)sm_count();
-  auto cost = [&](int64_t sp) {   // waves x (tiles, and a quarter for a block's start)
-    const int64_t tps = (n_tiles + sp - 1) / sp, blocks = row_blocks * ((n_tiles + tps - 1) / tps);
-    return (double)((blocks + slots - 1) / slots) * (4.0 * (double)tps + 1.0);
-  };
-  int64_t best = most;
-  if (resident > 0) {
-    double least = 0.97 * cost(most);
-    for (int64_t sp = most; sp >= 1 && sp >= most / 4; --sp)
-      if (cost(sp) < least) {
-        best = sp;
-        least = cost(sp);
+  int64_t best = (n_tiles + most - 1) / most;   // tiles per split
+  if (resident > 0 && !(short_only && best >= 12)) {
+    const int64_t slots = resident * (int64_t)sm_count();
+    auto cost = [&](int64_t tps) {
+      const int64_t blocks = row_blocks * ((n_tiles + tps - 1) / tps);
+      return (double)((blocks + slots - 1) / slots) * (4.0 * (double)tps + 1.0);
+    };
+    double least = 0.97 * cost(best);
+    // the shortest splits that fit each number of waves
+    for (int64_t waves = 1, splits = 0; splits < most; ++waves) {
+      splits = imin<int64_t>(most, waves * slots / row_blocks);
+      if (splits < 1 || splits < most / 4) continue;
+      const int64_t tps = (n_tiles + splits - 1) / splits;
+      if (cost(tps) < least) {
+        best = tps;
+        least = cost(tps);
       }
+    }
   }
-  const int64_t tps = (n_tiles + best - 1) / best;
-  return (int)((n_tiles + tps - 1) / tps);   // non-empty splits only
+  return (int)((n_tiles + best - 1) / best);   // non-empty splits only
 }
 
 template <int DP, int QPT>
@@ -308,11 +320,14 @@ void launch_score_nd_dp(const float* x, int64_t n, int d, const float* mu, doubl
 
 int kde_nd_splits(int64_t m, int64_t n, int d) {
   const int qpt = d <= 32 ? 2 : 1;
-  // blocks per SM by the registers of launch_kde_nd's kernels
-  return nd_splits((m + ND_THREADS * qpt - 1) / (ND_THREADS * qpt), n, d <= 16 ? 7 : 4);
+  // blocks per SM by the registers of launch_kde_nd's kernels.  17 to 31 keep
+  // the splits: there a block's start is cheap and fewer blocks balance worse
+  // (d = 20, 10000 x 10000: 233 us, 239 in one wave; d = 32 273 and 248).
+  const int resident = d <= 16 ? 7 : (d < 32 ? 0 : 4);
+  return nd_splits((m + ND_THREADS * qpt - 1) / (ND_THREADS * qpt), n, resident, qpt == 2);
 }
 
-int score_nd_splits(int64_t n) { return nd_splits((n + ND_THREADS - 1) / ND_THREADS, n, 0); }
+int score_nd_splits(int64_t n) { return nd_splits((n + ND_THREADS - 1) / ND_THREADS, n, 0, false); }
 
 void launch_kde_nd(const float* q, int64_t m, const float* x, int64_t n, int d, double h, bool laplace, int splits,
                    double* partials, cudaStream_t s) {
