@@ -112,13 +112,15 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_rows_kernel(const double* 
 
 void launch_reduce_rows(const double* partials, int splits, int64_t m, double scale, double eps,
                         bool log_out, float* out, const int* skip, cudaStream_t s) {
-  // one thread per row while the chain is short; where the launch may turn out
-  // to have nothing to do, no more blocks than fit at once (32768 that return
-  // at once take 19 us)
-  const int rows = splits <= 4 ? RED_THREADS : RED_THREADS / RED_LANES;
+  // one thread per row while the chain is short, or the rows alone fill the
+  // GPU (100000 rows x 6 splits: 4 us more with 8 threads per row); where the
+  // launch may turn out to have nothing to do, no more blocks than fit at once
+  // (32768 that return at once take 19 us)
+  const bool single = splits <= 4 || (splits <= 32 && m >= 65536);
+  const int rows = single ? RED_THREADS : RED_THREADS / RED_LANES;
   int64_t blocks = (m + rows - 1) / rows;
   if (skip != nullptr) blocks = imin<int64_t>(blocks, 8LL * sm_count());
-  if (splits <= 4)
+  if (single)
     reduce_rows_kernel<1><<<(unsigned)blocks, RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out, skip);
   else
     reduce_rows_kernel<RED_LANES><<<(unsigned)blocks, RED_THREADS, 0, s>>>(partials, splits, m, scale, eps, log_out ? 1 : 0, out,
