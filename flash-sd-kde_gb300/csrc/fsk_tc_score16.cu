@@ -485,13 +485,16 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
         const float cs = pa.x + pa.y;
         const bool trig = cs > (phi_scale + acc.s + cs) * SCORE_NEAR_FRACTION;   // phi_scale: the self pair
         if (__builtin_expect(__any_sync(0xffffffffu, trig), 0)) {
-          // The chunk's largest weight is recomputed exactly (argmax on keys
-          // = value bits with the column in the low 5 bits, as in the KDE
-          // kernel).  With A the keyed approximation, the pdf gets ex - A
-          // (corr) and the weighted sum (ex - A)(x_j - mu) (shared-memory
-          // corrections), so both see the same weight e_j - A + ex.
+          // The chunk's largest weight A is recomputed exactly (argmax on keys =
+          // value bits with the column in the low 5 bits; A is then taken from the
+          // column, since the key is up to 31 ulps off the value in the sum).  The
+          // pdf gets ex - A (corr) and the weighted sum (ex - A)(x_j - mu)
+          // (shared-memory corrections).
           if (trig) {
-            // four interleaved max chains keep the register peak low
+            // (an opaque copy for the compiler: 2932 us at n = 100000 with it, 2985
+            // without)
+#pragma unroll
+            for (int k = 0; k < 32; ++k) asm volatile("" : "+f"(e[k]));
             uint32_t k0 = 0u, k1 = 0u, k2 = 0u, k3 = 0u;
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
@@ -500,8 +503,13 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
               k2 = max(k2, (__float_as_uint(e[j + 2]) & ~31u) | (uint32_t)(j + 2));
               k3 = max(k3, (__float_as_uint(e[j + 3]) & ~31u) | (uint32_t)(j + 3));
             }
-            const uint32_t kmax = max(max(k0, k1), max(k2, k3));
-            const int j = (int)(kmax & 31u);
+            const int j = (int)(max(max(k0, k1), max(k2, k3)) & 31u);
+            // column j of e, which is not needed after this: halves until one is left
+#pragma unroll
+            for (int w = 16; w > 0; w >>= 1)
+#pragma unroll
+              for (int k = 0; k < w; ++k) e[k] = (j & w) ? e[k + w] : e[k];
+            const float top = e[0];
             const int col = half * 32 + j;
             const float4* xr = reinterpret_cast<const float4*>(stage + S_X_OFFSET + col * (FSK_D * 4));
             // exact squared distance, four features at a time
@@ -519,7 +527,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) score16_tc_kernel(ScParams p) {
             const float dist = (d0 + d1) + (d2 + d3);
             float ex = exp2_neg_scaled(dist, p.c2, p.c2_lo) * phi_scale;
             if (col >= valid || t * NT + col == gi) ex = 0.f;
-            const float delta = ex - __uint_as_float(kmax);
+            const float delta = ex - top;
             corr += delta;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
