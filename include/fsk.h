@@ -95,7 +95,8 @@ enum fsk_status {
  * log(that) - dmin / (2 h^2) + log(out_scale) in FP64. */
 #define FSK_OUT_LOG_EXACT 0x20
 /* Reduce splits with FP64 atomics instead of the ordered partial buffer
- * (kde_backend="atomic" / emp_score_backend="symmetric_atomic"). */
+ * (kde_backend="atomic" / emp_score_backend="symmetric_atomic").  No effect on
+ * 1-D calls that the cell expansions serve (fsk_kde1d), which have no splits. */
 #define FSK_ATOMIC 0x8
 /* fsk_empscore16: write weighted_sum as a (16, n) buffer, the layout of the
  * reference's flash backend (kernels/flash_sd_kde/empirical.py:180,223). */
