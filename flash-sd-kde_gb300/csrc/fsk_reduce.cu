@@ -198,8 +198,10 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_score_tc_kernel(tc::ScPart
   mp.y = fmaf(mk, ps.y, mp.y);
   const float2 wt = df_add(df_add(ws, mp), make_float2(xi, 0.f));
   const float2 pdf = df_add(ps, make_float2(1.0f, 0.f));
-  // beyond the pairs' range (eps, or a weighted sum past the largest float): FP64
-  const bool wide = eps_wide != 0 || !(fabsf(wt.x) < __int_as_float(0x7f800000));
+  // beyond the pairs' range (eps, a weighted sum past the largest float, a point
+  // whose double is): FP64
+  constexpr float LARGE = 8.5e37f;   // 2^126
+  const bool wide = eps_wide != 0 || !(fabsf(wt.x) < LARGE) || !(fabsf(xi) < LARGE);
   float w = wt.x;
   double off = 0.0;   // W / (pdf + eps) - x
   if (__builtin_expect(wide, 0)) {

@@ -63,3 +63,19 @@ def test_weighted_sums_past_the_largest_float(cuda_dev):
     assert torch.equal(deb, x) and (score == 0).all()
     assert ((pdf - 300).abs() <= 2e-6 * 300).all() and ((w[:, 3] - 600).abs() <= 2e-6 * 600).all()
     assert torch.isposinf(w[:, 0]).all()
+
+
+@pytest.mark.parametrize("value", [-FLT_MAX, 3e38, 1e38, -1e36])
+@pytest.mark.parametrize("h", [1e-3, 0.9, 500.0])
+def test_shift_of_points_near_the_largest_float(cuda_dev, value, h):
+    """A constant column stays where it is, with few neighbours (the weighted sum is
+    the point itself) and with many."""
+    from fsk import ops
+
+    x = _rows(300, 4)
+    x[:, 9] = value
+    deb = ops.sdshift16(x, h, 0.0)
+    deb2, _, _, score = ops.sdshift16(x, h, 1e-12, return_debug=True)
+    ops.device_status(cuda_dev)
+    assert torch.equal(deb[:, 9], x[:, 9]) and torch.equal(deb2[:, 9], x[:, 9])
+    assert torch.isfinite(deb).all() and torch.isfinite(score).all()
