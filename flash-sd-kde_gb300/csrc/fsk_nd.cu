@@ -50,7 +50,7 @@ __device__ __forceinline__ void stage_rows(float (*xs)[DP], const float* __restr
 
 // Bound by the FP32 pipe: 93 % of its measured rate at 100000 x 100000, d = 32
 // (10^10 pairs in 21.5 ms).
-template <int DP, int QPT, bool LAPLACE>
+template <int DP, int QPT, bool LAPLACE, bool AHEAD>
 __global__ void __launch_bounds__(ND_THREADS, DP == 16 ? 7 : 4) kde_nd_kernel(const float* __restrict__ q, int64_t m,
                                                             const float* __restrict__ x, int64_t n, int d, float c2,
                                                             float c2_lo, float c1, float lap0, int64_t tps,
@@ -70,10 +70,7 @@ __global__ void __launch_bounds__(ND_THREADS, DP == 16 ? 7 : 4) kde_nd_kernel(co
   const int64_t n_tiles = (n + ND_TN - 1) / ND_TN;
   const int64_t t0 = (int64_t)blockIdx.y * tps;
   const int64_t t1 = min(n_tiles, t0 + tps);
-  // the next tile's values are loaded while the present one is summed, except
-  // at DP = 32, whose registers leave no room for it (d = 24, 30000 x 30000:
-  // 1927 us without, 1939 with; d = 8 1159 and 1149, d = 64 5.98 and 4.99 ms)
-  constexpr bool AHEAD = DP != 32;
+  // AHEAD: the next tile's values are loaded while the present one is summed
   constexpr int ITEMS = ND_TN * DP / ND_THREADS;
   float next[ITEMS];
   auto fetch = [&](int64_t tile) {
@@ -290,7 +287,7 @@ int nd_splits(int64_t row_blocks, int64_t n, int resident, bool short_only) {
   return (int)((n_tiles + best - 1) / best);   // non-empty splits only
 }
 
-template <int DP, int QPT>
+template <int DP, int QPT, bool AHEAD>
 void launch_kde_nd_dp(const float* q, int64_t m, const float* x, int64_t n, int d, double h, bool laplace,
                       int splits, double* partials, cudaStream_t s) {
   const int64_t n_tiles = (n + ND_TN - 1) / ND_TN;
@@ -301,9 +298,9 @@ void launch_kde_nd_dp(const float* q, int64_t m, const float* x, int64_t n, int 
   const float c1 = (float)(1.0 / (2.0 * h * h));
   const float lap0 = 1.0f + 0.5f * (float)d;
   if (laplace)
-    kde_nd_kernel<DP, QPT, true><<<grid, ND_THREADS, 0, s>>>(q, m, x, n, d, c2, c2_lo, c1, lap0, tps, partials);
+    kde_nd_kernel<DP, QPT, true, AHEAD><<<grid, ND_THREADS, 0, s>>>(q, m, x, n, d, c2, c2_lo, c1, lap0, tps, partials);
   else
-    kde_nd_kernel<DP, QPT, false><<<grid, ND_THREADS, 0, s>>>(q, m, x, n, d, c2, c2_lo, c1, lap0, tps, partials);
+    kde_nd_kernel<DP, QPT, false, AHEAD><<<grid, ND_THREADS, 0, s>>>(q, m, x, n, d, c2, c2_lo, c1, lap0, tps, partials);
 }
 
 template <int DP>
@@ -332,10 +329,16 @@ int score_nd_splits(int64_t n) { return nd_splits((n + ND_THREADS - 1) / ND_THRE
 void launch_kde_nd(const float* q, int64_t m, const float* x, int64_t n, int d, double h, bool laplace, int splits,
                    double* partials, cudaStream_t s) {
   TimerScope ts(K_KDE_ND, (double)m * (double)n, s);
-  if (d <= 16) launch_kde_nd_dp<16, 2>(q, m, x, n, d, h, laplace, splits, partials, s);
-  else if (d <= 32) launch_kde_nd_dp<32, 2>(q, m, x, n, d, h, laplace, splits, partials, s);
-  else if (d <= 48) launch_kde_nd_dp<48, 1>(q, m, x, n, d, h, laplace, splits, partials, s);
-  else launch_kde_nd_dp<64, 1>(q, m, x, n, d, h, laplace, splits, partials, s);
+  // Loading ahead: 30000 x 30000 without and with it, d = 8 1159 and 1149 us, d =
+  // 64 5.98 and 4.99 ms, but d = 24 1927 and 1939, d = 32 1978 and 1985, where the
+  // registers leave no room for it; there it pays in short blocks of full rows
+  // only (d = 32, 20000 x 5000, 21 tiles a block: 254 and 250).
+  const bool short_rows = d == 32 && (int64_t)splits * 64 * ND_TN > n;
+  if (d <= 16) launch_kde_nd_dp<16, 2, true>(q, m, x, n, d, h, laplace, splits, partials, s);
+  else if (d <= 32 && short_rows) launch_kde_nd_dp<32, 2, true>(q, m, x, n, d, h, laplace, splits, partials, s);
+  else if (d <= 32) launch_kde_nd_dp<32, 2, false>(q, m, x, n, d, h, laplace, splits, partials, s);
+  else if (d <= 48) launch_kde_nd_dp<48, 1, true>(q, m, x, n, d, h, laplace, splits, partials, s);
+  else launch_kde_nd_dp<64, 1, true>(q, m, x, n, d, h, laplace, splits, partials, s);
   count_launch();
 }
 
