@@ -459,9 +459,16 @@ CellConsts cell_consts(double h) {
 }
 }  // namespace
 
-// Where the expansions are tried: at 2^30 pairs (131 us of pair sums) their
-// seven launches take ~40 us, half of that per point and query.  Data that
-// turns out too spread for the tables pays ~12 us for the attempt.
+// Where the expansions are tried.  Both sides, us per call (pair sums /
+// expansions / data too spread, which pays for the attempt):
+//   0.10e9 pairs: 4096 x 25000 41 / 43 / 49, 100000 x 1000 41 / 36 / 51
+//   0.34e9:       4096 x 80000 76 / 47 / 84, 100000 x 3500 78 / 38 / 86
+//   0.70e9:       4096 x 170000 117 / 47 / 125
+//   1.07e9:       4095 x 262144 154 / 45 / 162, 4096 x 262144 154 / 47 / 162
+//   4.3e9:        4095 x 1048576 544 / 54 / 554
+// The expansions win from ~1.5e8 pairs on; the line at 2^30 keeps what spread
+// data loses (3 to 10 us) at 5 % or less.  The limit of 4096 points has no
+// reason in time (2000 x 2000000: 518 / 64 / 531; 500 x 1000000: 85 / 77 / 97).
 // n <= 2^31: a point adds up to 1.5 x 2^31 to the signed 64-bit moments.
 bool cell1d_applies(int64_t m, int64_t n) {
   return n >= 4096 && n <= (int64_t(1) << 31) && (double)m * (double)n >= 1073741824.0;

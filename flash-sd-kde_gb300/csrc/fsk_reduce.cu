@@ -1,7 +1,8 @@
-// fsk_reduce.cu - O(n) FP64 kernels: column means for centering, the fixed-
-// order cross-split reduction of partial sums with the FP64 normalisation
-// (and optional log), the empirical-score reduction, and the SD-KDE debias
-// shift.  The split reduction replaces kernels/reduce_partials.py:6-58 (which
+// fsk_reduce.cu - O(n) kernels: column means for centering, the fixed-order
+// cross-split reduction of partial sums with the FP64 normalisation (and
+// optional log), the empirical-score reduction, and the SD-KDE debias shift.
+// The CUDA-core kernels' partials are FP64, the tensor-core kernels' FP32
+// (value, error) pairs, added as double-float (~48 bits).  The split reduction replaces kernels/reduce_partials.py:6-58 (which
 // sums splits in FP32); normalisation follows flash_sd_kde/kde.py:93-94,
 // :119-122; the debias shift follows flash_sd_kde/kde.py:319-322.
 #include "fsk_kernels.cuh"

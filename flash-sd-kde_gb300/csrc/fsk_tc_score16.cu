@@ -7,7 +7,8 @@
 // the accumulators of kernels/flash_sd_kde/empirical.py:72-131 and
 // kernels/emp_score_16d_ordered_splitk.py:20-95 (both tl.dot products with
 // allow_tf32), as (value, error) partials per segment (see WorkLine); the weighted sum is kept
-// centred (sum_j phi_ij (x_j - mu)) and mu * pdf_sum is added back in FP64.
+// centred (sum_j phi_ij (x_j - mu)) and mu * pdf_sum is added back by the
+// reduction, in double-float.
 //
 // How (per 256-query x 64-point tile):
 //  * S = the log2-domain exponent a2 + 15, three-part fp16 product of the

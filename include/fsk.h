@@ -208,6 +208,9 @@ FSK_API int fsk_debias16(const float* data, int64_t n, const float* pdf_sum,
                  float* debiased, float* score, void* stream);
 
 /* ---- 1-D Gaussian KDE and KDE score ------------------------------------ */
+/* fsk_kde1d without FSK_LAPLACE, for 4096 <= n <= 2^31 and m n >= 2^30: cell
+ * expansions where the data spans less than 447 bandwidths and is finite (decided
+ * on the device), pair sums otherwise. */
 FSK_API size_t fsk_kde1d_workspace_bytes(int64_t m, int64_t n, int flags);
 FSK_API int fsk_kde1d(const float* queries, int64_t m, const float* data, int64_t n,
               double bandwidth, int flags, double out_scale, double out_eps,
