@@ -91,10 +91,10 @@ struct TcScales {
 // Query blocks x data tiles over `grid` CTAs, in segments: a segment is a run
 // of data tiles of one query block, one accumulation and one row of partial
 // sums.  CTA b first takes the `whole` query blocks b, b + grid, ... from
-// their first to their last tile; all CTAs then walk the data in step, so a
-// tile comes from DRAM once for all of them (ranges that start anywhere made
-// the score kernel 5 % slower at n = 2^20, where the 268 MB data image exceeds
-// the L2).  The remaining rest < grid blocks form one line of rest * n_tiles
+// their first to their last tile; all CTAs then walk the data roughly in step,
+// and a wave of 152 blocks reads the score's 268 MB data image at n = 2^20, which
+// exceeds the L2, 5.7 times from DRAM (ranges that start anywhere made that
+// kernel 5 % slower).  The remaining rest < grid blocks form one line of rest * n_tiles
 // tiles of which every CTA takes an equal contiguous range, so small problems
 // neither leave the last wave empty nor pay for many short units (equal
 // splits of every query block gave the score kernel 5 units of 9 tiles per
